@@ -41,7 +41,7 @@ def build(ref: bool = True) -> None:
     reference libraries (make -C oracle [ref]) and, when libgf.a exists, the
     reference linked with libgf (make -C oracle linked)."""
     subprocess.run(["make", "-s", "-C", str(HERE)], check=True)
-    if ref and REF_SOURCE.exists():
+    if ref and (REF_SOURCE / "NewGalFinder").is_dir():  # a mount point without the tree is no tree
         subprocess.run(["make", "-s", "-C", str(HERE), f"REF={REF_SOURCE}", "ref"], check=True)
         if (HERE.parent / "galaxyfinder_b200" / "libgf.a").exists():
             subprocess.run(["make", "-s", "-C", str(HERE), f"REF={REF_SOURCE}", "linked"], check=True)
