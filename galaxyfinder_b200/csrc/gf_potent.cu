@@ -12,21 +12,43 @@
 // 1000 targets (external), then scale by potentfact and add the NFW
 // background term of the halo mass (GetBGpotent, :1093-1101).
 //
-// One thread per target.  The 32 targets of a warp are neighbours in tree
-// order and walk the preorder node array in lockstep: every iteration the warp
-// takes the smallest next-node index among its lanes, and the lanes waiting
-// at that node apply their own opening decision (open: sum the node's loose
-// particles and continue at i + 1; accept: add the cell term and continue at
-// skip[i]).  Opening decisions use the same FP64 |p - com|^2 as the
-// reference, so they are identical to an FP64 walk of the same tree; the
-// terms are FP32 evaluated from exact FP64 position differences and summed
-// with Kahan compensation.
+// A warp serves 32 targets, neighbours in tree order, one per lane.  The tree
+// is expanded for all of them together and every accepted cell and opened
+// leaf particle is evaluated by all lanes at once, so that no lane walks:
+//   * nodes to visit, each with the mask of the lanes that opened its parent,
+//     wait on a per-warp stack in shared memory; a step pops up to 32 and
+//     tests one per lane against the bounding box of the targets.  Four out
+//     of five are accepted (or opened) by every possible target in the box;
+//     the others are tested target by target, all lanes on one node.
+//     Opening decisions are those of an FP64 walk of the same tree: FP32
+//     distances decide only outside a margin above their rounding error, and
+//     what falls inside it is decided by the reference's FP64 test;
+//   * accepted cells and the loose particles of opened nodes are gathered, one
+//     per lane, into shared-memory tiles of 32 with one array per field, each
+//     entry with its lane mask, and a full tile is evaluated: lane = target,
+//     two entries per instruction (packed FP32 pairs, whose 16-byte loads
+//     serve four entries), inactive lanes by a zero 1/r.
+// The terms are FP32 evaluated from position differences with two roundings
+// (the node centre is held as the sum of two floats) and summed with Kahan
+// compensation in two interleaved sums.
+//
+// What bounds it: the FP32 pipe.  A cell costs 24 FP32 operations per lane
+// and a particle 10; a 131072-particle NFW halo at theta2 = 0.5 has, per
+// warp, 937 cells (23 of 32 lanes) and 1268 particles (12 of 32), about 35 k
+// of its cycles.  The lockstep walk that this replaces (every lane at its own
+// next node, the warp at the smallest) spent about 60 issue slots on a cell
+// and 17 on a particle, most of them on the walk and on FP64 differences.
+// Measured, lockstep -> tiled: 4096 halos (7.0 M particles) 13.3 -> 9.2 ms,
+// 300,007 particles at theta2 = 0.25 1.93 -> 1.26 ms, 131,072 at 0.5 0.46 ->
+// 0.30 ms, 64 small halos 0.31 -> 0.09 ms.  The FP32 pipe is then 46 % busy and
+// 61 % of the issue slots are used; the rest is the latency of the expansion
+// (its loads and shuffles).  A stack of 320 entries lets fewer nodes be popped
+// at once (9.4 ms), one of 768 costs resident warps (9.9 ms).
 #include <float.h>
 #include <limits.h>
 #include <math.h>
 
 #include <algorithm>
-#include <type_traits>
 
 #include "gf_tree.cuh"
 
@@ -45,16 +67,6 @@ struct Kahan {
     __device__ __forceinline__ float value() const { return s + (-c); }
 };
 
-// The sum of a target's FP32 terms: GF_BH_ACC=1 adds them in FP64 (two
-// instructions per term, one dependent add), 0 with FP32 Kahan compensation
-// (four dependent adds); both round once at the end.
-struct Fp64Acc {
-    double s = 0.0;
-    __device__ __forceinline__ void add(float v) { s += (double)v; }
-    __device__ __forceinline__ float value() const { return (float)s; }
-};
-using BhAcc = std::conditional<GF_BH_ACC == 1, Fp64Acc, Kahan>::type;
-
 // GetBGpotent, subhaloden.mod6.c:1059-1101
 __device__ double bg_potent_dev(double mvir, const PotentialParams &pp) {
     const double G = 6.672E-8, RHOC = 2.7755E11;
@@ -68,53 +80,116 @@ __device__ double bg_potent_dev(double mvir, const PotentialParams &pp) {
     return vc2 * (1 - gc * log(1 + c));
 }
 
-// ---- leaf tiles staged by the bulk-copy (TMA) engine, GF_BH_TMA=1
-// When lanes open a node whose loose particles fit a slot (at most
-// kLeafSlotP float4), one lane has the tensor-memory-access unit copy them
-// (cp.async.bulk, global -> this CTA's shared memory, completion counted on
-// an mbarrier; no multicast) into the next slot of a per-warp ring, and the
-// warp walks on; the opened leaf is summed from shared memory later, when the
-// ring is full or the walk ends.  Every wait is bounded: a copy that does not
-// complete in time sets GF_ERRBIT_WAIT and the warp falls back to global
-// loads for the rest of the launch.
-constexpr int kLeafSlots = 4;   // ring slots per warp
-constexpr int kLeafSlotP = 32;  // float4 (particles) per slot
-constexpr int kWaitTries = 1 << 20;
+// ---- packed pairs of floats (two FP32 operations per instruction, each
+// rounded as the scalar one)
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 f2_pack(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_unpack(f2 v, float &a, float &b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
+// Two Kahan sums side by side; nc is the negated compensation.  The terms
+// arrive as t * inv, folded into the first addition.
+struct Kahan2 {
+    f2 s, nc;
+    __device__ __forceinline__ void add(f2 t, f2 inv, f2 minus1) {
+        const f2 y = f2_fma(t, inv, nc);
+        const f2 n = f2_add(s, y);
+        nc = f2_add(y, f2_fma(n, minus1, s));  // y - (n - s)
+        s = n;
+    }
+};
+
+// ---- per-warp shared memory of bh_kernel
+constexpr int kCellFields = 13;  // -centre high and low parts, mass, six moments
+constexpr int kStack = 416;      // (node, lanes) still to visit
+constexpr int kDeal = 4;         // nodes per part before they are dealt out
+struct __align__(16) BhWarp {
+    float cell[kCellFields][32];
+    float leaf[4][64];   // -x, -y, -z, mass of a particle; a tile of 32 and what waits for the next
+    unsigned leaf_mask[64];
+    uint2 cells[64];     // accepted (node, lanes) waiting for a tile
+    uint2 stack[kStack];
+};
+
+// Bit l of row e (lane e's v) becomes bit e of row l: each lane receives, for
+// every tile entry, whether it takes part (five butterfly steps).
+__device__ __forceinline__ unsigned transpose_bits(unsigned v) {
+    const int lane = threadIdx.x & 31;
+    unsigned low = 0x0000ffffu;
+#pragma unroll
+    for (int j = 16; j; j >>= 1) {
+        const unsigned o = __shfl_xor_sync(0xffffffffu, v, j);
+        v = (lane & j) ? (v & ~low) | ((o & ~low) >> j) : (v & low) | ((o & low) << j);
+        low ^= low << (j >> 1);
+    }
+    return v;
 }
-__device__ __forceinline__ void mbar_init(uint64_t *bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(smem_addr(bar)), "r"(parity)
-        : "memory");
-    return done != 0;
-}
-// bytes: a multiple of 16; src and dst 16-byte aligned
-__device__ __forceinline__ void bulk_copy_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-    uint64_t g;
-    asm("cvta.to.global.u64 %0, %1;" : "=l"(g) : "l"(src));
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_addr(dst)),
-        "l"(g), "r"(bytes), "r"(smem_addr(bar))
-        : "memory");
-}
-// the generic-proxy reads of a slot precede the async-proxy write that reuses it
-__device__ __forceinline__ void fence_proxy_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+
+// The walk one node at a time over the preorder nodes [i, end): every lane at
+// its own next node, the warp at the smallest of them (taking part: lanes
+// with `on`).  Serves what the tiles do not: subtrees that no longer fit the
+// stack, and targets whose tiled sum is not finite (a squared distance below
+// the normal floats, where this walk's rsqrtf is still exact to its 2 ulp).
+__device__ __noinline__ float lockstep_walk(int i, int end, bool on, bool always_open, float4 P,
+                                            const float4 *__restrict__ spos, const BhNode *__restrict__ nodes) {
+    const double px = P.x, py = P.y, pz = P.z;
+    Kahan acc;
+    int my = on ? i : INT_MAX;
+    while (i < end) {
+        bool open = false;
+        const int4 links = __ldg(reinterpret_cast<const int4 *>(nodes + i) + 4);  // skip, lstart, lcount, count
+        if (my <= i) {
+            const BhNode &nd = nodes[i];
+            const double dx = px - nd.com[0], dy = py - nd.com[1], dz = pz - nd.com[2];
+            // separately rounded, as the reference's treeopen (ost.c:79)
+            const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+            open = always_open || d2 < nd.open_r2;
+            if (open) {
+                for (int j = links.y; j < links.y + links.z; j++) {
+                    const float4 S = spos[j];
+                    const float fx = P.x - S.x, fy = P.y - S.y, fz = P.z - S.z;
+                    const float r2 = fx * fx + fy * fy + fz * fz;
+                    if (r2 > 0.f) acc.add(-S.w * rsqrtf(r2));
+                }
+            } else {
+                const float fx = (float)dx, fy = (float)dy, fz = (float)dz;
+                const float r2 = fx * fx + fy * fy + fz * fz;
+                const float inv = rsqrtf(r2), inv2 = inv * inv, inv3 = inv * inv2;
+                const float qxy = nd.q[0] * fx * fx + nd.q[1] * fy * fy + nd.q[2] * fz * fz +
+                                  2.f * (nd.q[3] * fx * fy + nd.q[4] * fx * fz + nd.q[5] * fy * fz);
+                acc.add(-nd.mass * inv + 0.5f * nd.trq * inv3 - 1.5f * qxy * inv3 * inv2);
+                my = links.x;
+            }
+        }
+        // a lane that accepted an ancestor waits at or past this node's skip
+        i = __any_sync(0xffffffffu, open) ? i + 1 : links.x;
+    }
+    return acc.value();
 }
 
 // COUNT: interaction counters (bench and tests); off in the stage's walk.
@@ -123,29 +198,21 @@ __global__ void __launch_bounds__(GF_BH_BLOCK, GF_BH_MINB)
 bh_kernel(int64_t ntarget, const float4 *__restrict__ tpos, const int32_t *__restrict__ thalo,
           const int32_t *__restrict__ tout, const float4 *__restrict__ spos,
           const int32_t *__restrict__ root, const int32_t *__restrict__ rend,
-          const BhNode *__restrict__ nodes, const int32_t *__restrict__ direct,
-          const double *__restrict__ bg, PotentialParams pp, float *__restrict__ out,
-          float *__restrict__ raw, unsigned long long *__restrict__ counters,
-          unsigned long long *__restrict__ work, int *__restrict__ err) {
+          const BhNode *__restrict__ nodes, const WalkNode *__restrict__ wnodes,
+          const int32_t *__restrict__ direct, const double *__restrict__ bg, PotentialParams pp,
+          float *__restrict__ out, float *__restrict__ raw, unsigned long long *__restrict__ counters,
+          unsigned long long *__restrict__ work, bool together) {
+    extern __shared__ __align__(16) unsigned char bh_smem[];
     const int lane = threadIdx.x & 31;
-#if GF_BH_TMA
-    __shared__ __align__(16) float4 leaf_ring[GF_BH_BLOCK / 32][kLeafSlots][kLeafSlotP];
-    __shared__ __align__(8) uint64_t leaf_bar[GF_BH_BLOCK / 32][kLeafSlots];
-    float4(*ring)[kLeafSlotP] = leaf_ring[threadIdx.x >> 5];
-    uint64_t *bars = leaf_bar[threadIdx.x >> 5];
-    if (lane < kLeafSlots) mbar_init(bars + lane);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    __syncwarp();
-    uint32_t phases = 0;        // parity each slot's barrier completes next (warp-uniform)
-    int head = 0, pending = 0;  // oldest staged slot, staged slots (warp-uniform)
-    unsigned qmask = 0;         // in lane s < kLeafSlots: the lanes that opened slot s's leaf
-    int qcnt = 0;               // in lane s: the particles in slot s
-    bool tma_ok = true;         // cleared by a wait that ran out
-#else
-    (void)err;
-#endif
-    const int64_t warp0 = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32;
-    const int64_t wstride = (int64_t)gridDim.x * blockDim.x;
+    const unsigned lt = (1u << lane) - 1u;
+    BhWarp &W = reinterpret_cast<BhWarp *>(bh_smem)[threadIdx.x >> 5];
+    // `together`: the warps of a block share 32 targets and divide the nodes
+    // among them; warp 0 adds up and writes (one pass per launch)
+    const int split = together ? (int)blockDim.x >> 5 : 1;
+    const int part = together ? threadIdx.x >> 5 : 0;
+    const int64_t warp0 = (((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) / split) * 32;
+    const int64_t wstride = (int64_t)gridDim.x * blockDim.x / split;
+    const f2 minus1 = f2_pack(-1.f, -1.f);
     unsigned long long npp = 0, npc = 0;
     // the warp's next 32 targets: from the work counter, or grid-stride
     auto next = [&](int64_t stride_base) -> int64_t {
@@ -157,143 +224,298 @@ bh_kernel(int64_t ntarget, const float4 *__restrict__ tpos, const int32_t *__res
     for (int64_t base = next(warp0); base < ntarget; base = next(base + wstride)) {
         const int64_t t = base + lane;
         const bool valid = t < ntarget;
-        int h = 0, my = INT_MAX, my_end = 0, always_open = 0;
+        int h = -1;
         float4 P = make_float4(0.f, 0.f, 0.f, 0.f);
         if (valid) {
             h = thalo[t];
-            my = root[h];
-            my_end = rend[h];
-            if (my >= my_end) my = INT_MAX;
-            always_open = direct ? direct[h] : 0;
             P = tpos[t];
         }
-        const double px = P.x, py = P.y, pz = P.z;
-        BhAcc acc;
-        // ost.c:186-191: float offsets of the two positions.  For float
-        // inputs the FP32 difference is the correctly rounded exact
-        // difference, i.e. the same bits as rounding the FP64 difference.
-        auto particle_term = [&](const float4 &S) {
-            const float fx = P.x - S.x;
-            const float fy = P.y - S.y;
-            const float fz = P.z - S.z;
-            const float r2 = fx * fx + fy * fy + fz * fz;
-            if (r2 > 0.f) acc.add(-S.w * rsqrtf(r2));
-        };
-#if GF_BH_TMA
-        // sums the oldest staged leaf once its copy has landed
-        auto consume = [&]() {
-            const int slot = head;
-            const uint32_t par = (phases >> slot) & 1u;
-            bool ok = false;
-            for (int it = 0; it < kWaitTries && !ok; it++) ok = mbar_try_wait(bars + slot, par);
-            if (!__all_sync(0xffffffffu, ok)) {
-                if (lane == 0) atomicOr(err, GF_ERRBIT_WAIT);
-                // the copy may still land in this slot: wait for it once
-                // more, then stage no further leaves in this launch
-                ok = false;
-                for (int it = 0; it < kWaitTries && !ok; it++) ok = mbar_try_wait(bars + slot, par);
-                tma_ok = false;
+        const f2 px = f2_pack(P.x, P.x), py = f2_pack(P.y, P.y), pz = f2_pack(P.z, P.z);
+        Kahan2 acc{0ull, 0ull};
+        float aside = 0.f;  // subtrees walked one node at a time
+        int cn = 0, ln = 0;  // waiting cells and particles (warp-uniform)
+
+        // a tile of up to 32 cells, taken from the end of the waiting list
+        auto eval_cells = [&](int n) {
+            cn -= n;
+            const bool have = lane < n;
+            const uint2 c = have ? W.cells[cn + lane] : make_uint2(0u, 0u);
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a, m = a, q = a;
+            if (have) {
+                const float4 *w = reinterpret_cast<const float4 *>(wnodes + c.x);
+                a = __ldg(w);
+                b = __ldg(w + 2);
+                m = __ldg(w + 3);
+                q = __ldg(w + 4);
             }
-            phases ^= 1u << slot;
-            const unsigned m = __shfl_sync(0xffffffffu, qmask, slot);
-            const int c = __shfl_sync(0xffffffffu, qcnt, slot);
-            if ((m >> lane) & 1u)
-                for (int j = 0; j < c; j++) particle_term(ring[slot][j]);
-            __syncwarp();  // every lane's reads of the slot precede its next copy
-            head = (head + 1) % kLeafSlots;
-            pending--;
+            W.cell[0][lane] = -a.x;
+            W.cell[1][lane] = -a.y;
+            W.cell[2][lane] = -a.z;
+            W.cell[3][lane] = -b.x;
+            W.cell[4][lane] = -b.y;
+            W.cell[5][lane] = -b.z;
+            W.cell[6][lane] = b.w;
+            W.cell[7][lane] = m.x;
+            W.cell[8][lane] = m.y;
+            W.cell[9][lane] = m.z;
+            W.cell[10][lane] = m.w;
+            W.cell[11][lane] = q.x;
+            W.cell[12][lane] = q.y;
+            unsigned on = transpose_bits(c.y);
+            __syncwarp();
+#pragma unroll 1
+            for (int e = 0; e < n; e += 4, on >>= 4) {
+                ulonglong2 f[kCellFields];
+#pragma unroll
+                for (int i = 0; i < kCellFields; i++)
+                    f[i] = *reinterpret_cast<const ulonglong2 *>(&W.cell[i][e]);
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    auto F = [&](int i) { return u ? f[i].y : f[i].x; };
+                    const f2 dx = f2_add(f2_add(px, F(0)), F(3));
+                    const f2 dy = f2_add(f2_add(py, F(1)), F(4));
+                    const f2 dz = f2_add(f2_add(pz, F(2)), F(5));
+                    const f2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
+                    float ra, rb;
+                    f2_unpack(r2, ra, rb);
+                    ra = (on & (1u << (2 * u))) ? rsqrt_ftz(ra) : 0.f;
+                    rb = (on & (2u << (2 * u))) ? rsqrt_ftz(rb) : 0.f;
+                    const f2 inv = f2_pack(ra, rb), inv2 = f2_mul(inv, inv), inv4 = f2_mul(inv2, inv2);
+                    // d.Q.d over the upper triangle (off-diagonals doubled)
+                    const f2 q1 = f2_fma(F(7), dx, f2_fma(F(10), dy, f2_mul(F(11), dz)));
+                    const f2 q2 = f2_fma(F(8), dy, f2_mul(F(12), dz));
+                    const f2 qd = f2_fma(dx, q1, f2_fma(dy, q2, f2_mul(f2_mul(F(9), dz), dz)));
+                    acc.add(f2_fma(qd, inv4, F(6)), inv, minus1);
+                }
+            }
+            __syncwarp();
         };
-#endif
-        while (true) {
-            const int i = (int)__reduce_min_sync(0xffffffffu, (unsigned)my);
-            if (i == INT_MAX) break;
-            bool stage = false;  // this lane opened a leaf that is staged
-            int stage_l0 = 0, stage_n = 0;
-            if (my == i) {
-                // the node in 16-byte words: (com x, com y), (com z, open_r2),
-                // (mass, trq, qxx, qyy), (qzz, qxy, qxz, qyz), (skip, lstart, lcount, count)
-                // All five are loaded before the opening test (one broadcast
-                // line for the lanes at the node), so the moment loads of an
-                // accepted cell overlap the FP64 test instead of following it.
-                const double2 *nd2 = reinterpret_cast<const double2 *>(nodes + i);
-                const float4 *nf = reinterpret_cast<const float4 *>(nodes + i);
-                const double2 c01 = __ldg(nd2), c2r = __ldg(nd2 + 1);
-                const float4 mq = __ldg(nf + 2), q = __ldg(nf + 3);  // (mass, trq, q0, q1), (q2..q5)
-                const int4 links = __ldg(reinterpret_cast<const int4 *>(nodes + i) + 4);
-                const double dx = px - c01.x;
-                const double dy = py - c01.y;
-                const double dz = pz - c2r.x;
-                // separately rounded, as the reference's treeopen (ost.c:79)
-                const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
-                                            __dmul_rn(dz, dz));
-                if (always_open || d2 < c2r.y) {
-#if GF_BH_TMA
-                    if (tma_ok && links.z > 0 && links.z <= kLeafSlotP) {
-                        stage = true;
-                        stage_l0 = links.y;
-                        stage_n = links.z;
-                    } else
-#endif
-                    {
-                        const int l1 = links.y + links.z;
-                        int j = links.y;
-#if GF_BH_LEAF4
-                        // four loads in flight before the terms, which are
-                        // still added in particle order
-                        for (; j + 4 <= l1; j += 4) {
-                            const float4 s0 = __ldg(spos + j), s1 = __ldg(spos + j + 1);
-                            const float4 s2 = __ldg(spos + j + 2), s3 = __ldg(spos + j + 3);
-                            particle_term(s0);
-                            particle_term(s1);
-                            particle_term(s2);
-                            particle_term(s3);
-                        }
-#endif
-                        for (; j < l1; j++) particle_term(spos[j]);
+        // the first n (up to 32) waiting particles
+        auto eval_leaf = [&](int n) {
+            if (lane >= n && lane < ((n + 3) & ~3)) {  // pad to a multiple of four
+                W.leaf[3][lane] = 0.f;
+                W.leaf_mask[lane] = 0u;
+            }
+            unsigned on = transpose_bits(W.leaf_mask[lane]);
+            __syncwarp();
+#pragma unroll 2
+            for (int e = 0; e < n; e += 4, on >>= 4) {
+                const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(&W.leaf[0][e]);
+                const ulonglong2 Y = *reinterpret_cast<const ulonglong2 *>(&W.leaf[1][e]);
+                const ulonglong2 Z = *reinterpret_cast<const ulonglong2 *>(&W.leaf[2][e]);
+                const ulonglong2 M = *reinterpret_cast<const ulonglong2 *>(&W.leaf[3][e]);
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const f2 dx = f2_add(px, u ? X.y : X.x), dy = f2_add(py, u ? Y.y : Y.x);
+                    const f2 dz = f2_add(pz, u ? Z.y : Z.x);
+                    const f2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
+                    float ra, rb;
+                    f2_unpack(r2, ra, rb);
+                    // ost.c:186-191: particle terms with r > 0
+                    ra = (on & (1u << (2 * u))) && ra > 0.f ? rsqrt_ftz(ra) : 0.f;
+                    rb = (on & (2u << (2 * u))) && rb > 0.f ? rsqrt_ftz(rb) : 0.f;
+                    acc.add(u ? M.y : M.x, f2_pack(ra, rb), minus1);
+                }
+            }
+            __syncwarp();
+            ln -= n;
+            if (lane < ln) {  // the rest (at most 31) move to the front
+#pragma unroll
+                for (int i = 0; i < 4; i++) W.leaf[i][lane] = W.leaf[i][n + lane];
+                W.leaf_mask[lane] = W.leaf_mask[n + lane];
+            }
+            __syncwarp();
+        };
+
+        // ---- one halo of the warp's targets at a time (nearly always one)
+        for (unsigned todo = __ballot_sync(0xffffffffu, valid); todo;) {
+            const int hl = __shfl_sync(0xffffffffu, h, __ffs(todo) - 1);
+            const unsigned grp = __ballot_sync(0xffffffffu, valid && h == hl);
+            todo &= ~grp;
+            if (root[hl] >= rend[hl]) continue;
+            const bool all_open = direct && direct[hl];
+            float blo[3], bhi[3];  // the box of this halo's targets
+            {
+                const bool in = (grp >> lane) & 1u;
+                const float c[3] = {P.x, P.y, P.z};
+#pragma unroll
+                for (int a = 0; a < 3; a++) {
+                    float lo = in ? c[a] : FLT_MAX, hi = in ? c[a] : -FLT_MAX;
+#pragma unroll
+                    for (int o = 16; o; o >>= 1) {
+                        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+                        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
                     }
-                    if (COUNT) npp += links.z;
-                    my = i + 1;
-                } else {
-                    const float fx = (float)dx, fy = (float)dy, fz = (float)dz;
-                    const float r2 = fx * fx + fy * fy + fz * fz;
-                    const float inv = rsqrtf(r2);
-                    const float inv2 = inv * inv;
-                    const float inv3 = inv * inv2;
-                    const float qxy = mq.z * fx * fx + mq.w * fy * fy + q.x * fz * fz +
-                                      2.f * (q.y * fx * fy + q.z * fx * fz + q.w * fy * fz);
-                    acc.add(-mq.x * inv + 0.5f * mq.y * inv3 - 1.5f * qxy * inv3 * inv2);
-                    if (COUNT) npc++;
-                    my = links.x;
+                    blo[a] = lo;
+                    bhi[a] = hi;
                 }
-                if (my >= my_end) my = INT_MAX;
             }
-#if GF_BH_TMA
-            const unsigned om = __ballot_sync(0xffffffffu, stage);
-            if (om) {  // the lanes at node i that opened it share its loose particles
-                const int src = __ffs(om) - 1;
-                const int l0 = __shfl_sync(0xffffffffu, stage_l0, src);
-                const int nl = __shfl_sync(0xffffffffu, stage_n, src);
-                if (pending == kLeafSlots) consume();
-                const int slot = (head + pending) % kLeafSlots;
-                if (lane == 0) {
-                    fence_proxy_async_smem();
-                    mbar_expect_tx(bars + slot, (uint32_t)nl * 16u);
-                    bulk_copy_g2s(ring[slot], spos + l0, (uint32_t)nl * 16u, bars + slot);
+            if (lane == 0) W.stack[0] = make_uint2((unsigned)hl, grp);  // the root of halo h is walk node h
+            __syncwarp();
+            int top = 1;
+            // every part expands the first nodes, part 0 keeps their cells
+            // and particles; once there are a few nodes for each part, they
+            // are dealt out
+            bool shared = together;
+            while (top > 0) {
+                if (shared && top >= kDeal * split) {
+                    shared = false;
+                    const int mine = (top - part + split - 1) / split;
+                    for (int i = 0; i < mine; i += 32) {
+                        uint2 v = make_uint2(0u, 0u);
+                        if (i + lane < mine) v = W.stack[part + split * (i + lane)];
+                        __syncwarp();
+                        if (i + lane < mine) W.stack[i + lane] = v;
+                        __syncwarp();
+                    }
+                    top = mine;
+                    continue;
                 }
-                if (lane == slot) {
-                    qmask = om;
-                    qcnt = nl;
+                // as many as leave room for eight children each
+                int take = min(min(32, top), (kStack - top) / 7);
+                const bool full = take < 1;
+                take = max(take, 1);
+                top -= take;
+                int node = 0;
+                unsigned m = 0u;
+                if (lane < take) {
+                    const uint2 v = W.stack[top + lane];
+                    node = (int)v.x;
+                    m = v.y;
                 }
-                pending++;
+                __syncwarp();
+                if (full) {  // no room for this node's children
+                    const int nd = __shfl_sync(0xffffffffu, node, 0);
+                    const unsigned mm = __shfl_sync(0xffffffffu, m, 0);
+                    const int pre = wnodes[nd].pre;
+                    const float v = lockstep_walk(pre, nodes[pre].skip, (mm >> lane) & 1u, all_open, P, spos, nodes);
+                    if (!(shared && part)) aside += v;
+                    continue;
+                }
+                const WalkNode *w = wnodes + node;
+                int4 lk = make_int4(0, 0, 0, 0);  // first, nchild, lstart, lcount
+                unsigned am = 0u, om = m;         // lanes that accept, that open
+                bool mixed = false;
+                if (lane < take) {
+                    const float4 a = __ldg(reinterpret_cast<const float4 *>(w));
+                    lk = __ldg(reinterpret_cast<const int4 *>(w) + 1);
+                    // nearest and farthest distance from the node's centre to
+                    // the box, widened by the rounding of a coordinate
+                    const float c[3] = {a.x, a.y, a.z};
+                    float mn = 0.f, mx = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 3; i++) {
+                        const float g0 = blo[i] - c[i], g1 = c[i] - bhi[i];
+                        const float e = fabsf(c[i]) * 1.2e-7f;
+                        const float g = fmaxf(fmaxf(g0, g1) - e, 0.f), f = fmaxf(fabsf(g0), fabsf(g1)) + e;
+                        mn += g * g;
+                        mx += f * f;
+                    }
+                    if (!all_open) {
+                        if (mn > walk_open_hi(a.w) * (1.f + 2e-6f)) {
+                            am = m;
+                            om = 0u;
+                        } else {
+                            mixed = !(mx * (1.f + 2e-6f) < a.w);
+                        }
+                    }
+                }
+                // nodes that the box does not settle, target by target
+                for (unsigned mb = __ballot_sync(0xffffffffu, mixed); mb; mb &= mb - 1) {
+                    const int src = __ffs(mb) - 1;
+                    const int nd = __shfl_sync(0xffffffffu, node, src);
+                    const unsigned ms = __shfl_sync(0xffffffffu, m, src);
+                    const float4 a = __ldg(reinterpret_cast<const float4 *>(wnodes + nd));
+                    const float4 b = __ldg(reinterpret_cast<const float4 *>(wnodes + nd) + 2);
+                    const float dx = (P.x - a.x) - b.x, dy = (P.y - a.y) - b.y, dz = (P.z - a.z) - b.z;
+                    const float r2 = dx * dx + dy * dy + dz * dz;
+                    bool open = r2 < a.w;
+                    if (!open && !(r2 > walk_open_hi(a.w)) && ((ms >> lane) & 1u)) {
+                        // within the margin: the reference's treeopen in FP64,
+                        // separately rounded (ost.c:79)
+                        const BhNode &n = nodes[wnodes[nd].pre];
+                        const double ex = (double)P.x - n.com[0], ey = (double)P.y - n.com[1], ez = (double)P.z - n.com[2];
+                        open = __dadd_rn(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)), __dmul_rn(ez, ez)) < n.open_r2;
+                    }
+                    const unsigned ob = __ballot_sync(0xffffffffu, open);
+                    if (lane == src) {
+                        am = m & ~ob;
+                        om = m & ob;
+                    }
+                }
+                // ---- children of the opened nodes onto the stack
+                const int nch = om ? lk.y : 0;
+                int at = nch;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, at, o);
+                    if (lane >= o) at += v;
+                }
+                const int nall = __shfl_sync(0xffffffffu, at, 31);
+                for (int c = 0, s0 = top + at - nch; c < nch; c++) W.stack[s0 + c] = make_uint2((unsigned)(lk.x + c), om);
+                top += nall;
+                if (shared && part) {  // part 0 has these
+                    am = 0u;
+                    lk.w = 0;
+                }
+                if (COUNT) {
+                    npc += __popc(am);
+                    npp += (unsigned long long)lk.w * __popc(om);
+                }
+                // ---- accepted cells
+                const unsigned ab = __ballot_sync(0xffffffffu, am != 0u);
+                if (am) W.cells[cn + __popc(ab & lt)] = make_uint2((unsigned)node, am);
+                cn += __popc(ab);
+                __syncwarp();
+                if (cn >= 32) eval_cells(32);
+                // ---- loose particles of the opened nodes
+                for (unsigned lb = __ballot_sync(0xffffffffu, om != 0u && lk.w > 0); lb; lb &= lb - 1) {
+                    const int src = __ffs(lb) - 1;
+                    const int l0 = __shfl_sync(0xffffffffu, lk.z, src), lc = __shfl_sync(0xffffffffu, lk.w, src);
+                    const unsigned lm = __shfl_sync(0xffffffffu, om, src);
+                    for (int o = 0; o < lc; o += 32) {
+                        const int k = min(32, lc - o);
+                        if (lane < k) {
+                            const float4 S = __ldg(spos + l0 + o + lane);
+                            W.leaf[0][ln + lane] = -S.x;
+                            W.leaf[1][ln + lane] = -S.y;
+                            W.leaf[2][ln + lane] = -S.z;
+                            W.leaf[3][ln + lane] = S.w;
+                            W.leaf_mask[ln + lane] = lm;
+                        }
+                        ln += k;
+                        __syncwarp();
+                        if (ln >= 32) eval_leaf(32);
+                    }
+                }
             }
-#endif
         }
-#if GF_BH_TMA
-        while (pending) consume();  // the walk's staged leaves, before the outputs
-#endif
+        if (cn > 0) eval_cells(cn);
+        if (ln > 0) eval_leaf(ln);
+        // the two sums and their compensations
+        float s0, s1, c0, c1;
+        f2_unpack(acc.s, s0, s1);
+        f2_unpack(acc.nc, c0, c1);
+        double sum = (double)aside - (((double)s0 + (double)s1) + ((double)c0 + (double)c1));
+        if (together) {
+            double *red = reinterpret_cast<double *>(W.stack);  // 32 of each part, done with its stack
+            __syncwarp();
+            red[lane] = sum;
+            __syncthreads();
+            if (part) continue;
+            for (int q = 1; q < split; q++) sum += reinterpret_cast<const double *>((&W + q)->stack)[lane];
+        }
+        float phi = (float)(0.0 + sum);
+        bool redo = valid && !(fabsf(phi) <= FLT_MAX);
+        for (unsigned rb = __ballot_sync(0xffffffffu, redo); rb;) {
+            const int hl = __shfl_sync(0xffffffffu, h, __ffs(rb) - 1);
+            const bool on = redo && h == hl;
+            const float v = lockstep_walk(root[hl], rend[hl], on, direct && direct[hl], P, spos, nodes);
+            if (on) phi = v;
+            rb &= ~__ballot_sync(0xffffffffu, on);
+        }
         if (valid) {
             const int64_t o = tout ? tout[t] : t;
-            const float phi = acc.value();
             if (raw) raw[o] = phi;
             if (out) {
                 double e = pp.potentfact != 0.0 ? (double)phi * pp.potentfact : (double)phi;
@@ -319,25 +541,36 @@ bh_kernel(int64_t ntarget, const float4 *__restrict__ tpos, const int32_t *__res
 // memory, so warps that drew cheap targets keep drawing and the launch ends
 // when the work does (with a static grid-stride split, the warps holding the
 // costliest targets finish last, alone).
-int launch_bh(gf_ctx *ctx, int64_t grid, int64_t ntarget, const float4 *tpos, const int32_t *thalo,
-              const int32_t *tout, const float4 *spos, const int32_t *root, const int32_t *rend,
-              const BhNode *nodes, const int32_t *direct, const double *bg, const PotentialParams &pp,
-              float *out, float *raw, unsigned long long *counters) {
+int launch_bh(gf_ctx *ctx, int64_t ntarget, const float4 *tpos, const int32_t *thalo,
+              const int32_t *tout, const TreeView &t, const int32_t *direct, const double *bg,
+              const PotentialParams &pp, float *out, float *raw, unsigned long long *counters) {
     const int block = GF_BH_BLOCK;
+    const size_t shmem = (size_t)(block / 32) * sizeof(BhWarp);
     unsigned long long *work = nullptr;
-    // a grid of 1.6 waves (16 blocks per SM requested, 10 resident) would
-    // leave 40 % of the SMs' block slots empty in its second wave
     auto kern = counters ? bh_kernel<true> : bh_kernel<false>;
     int per_sm = 0;
-    GF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0));
-    grid = std::max<int64_t>(1, std::min<int64_t>(grid, (int64_t)sm_count() * std::max(per_sm, 1)));
-    if (GF_BH_DYN) {
-        GF_TRY(ctx->work.reserve(256));
-        work = ctx->work.as<unsigned long long>();  // slot 0: this walk
-        GF_CUDA_TRY(cudaMemsetAsync(work, 0, sizeof(unsigned long long), ctx->stream));
+    GF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem));
+    GF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, shmem));
+    const int64_t wave = (int64_t)sm_count() * std::max(per_sm, 1);  // resident blocks
+    const int64_t groups = (ntarget + 31) / 32, warps = block / 32;
+    // few targets: a block's warps divide the nodes of 32 targets among them
+    // instead of leaving most of the SMs' warps without work.  Above half of
+    // the resident warps the dealing costs more than it fills (more steps
+    // with less than 32 nodes each): 36,001 targets 165 -> 131 us, a batch of
+    // 64 small halos 150 -> 90, but 131,072 targets 305 -> 345.
+    const bool together = 2 * groups <= wave * warps;
+    int64_t grid = together ? groups : (groups + warps - 1) / warps;
+    if (!together) {
+        // a grid of 1.6 waves would leave 40 % of the SMs' block slots empty in its second wave
+        grid = std::min(grid, wave);
+        if (GF_BH_DYN) {
+            GF_TRY(ctx->work.reserve(256));
+            work = ctx->work.as<unsigned long long>();  // slot 0: this walk
+            GF_CUDA_TRY(cudaMemsetAsync(work, 0, sizeof(unsigned long long), ctx->stream));
+        }
     }
-    kern<<<(int)grid, block, 0, ctx->stream>>>(ntarget, tpos, thalo, tout, spos, root, rend, nodes, direct, bg, pp,
-                                               out, raw, counters, work, ctx->d_err);
+    kern<<<(int)grid, block, shmem, ctx->stream>>>(ntarget, tpos, thalo, tout, t.pos, t.root, t.rend, t.bh, t.walk,
+                                                   direct, bg, pp, out, raw, counters, work, together);
     GF_LAUNCH_CHECK();
     return GF_OK;
 }
@@ -423,11 +656,7 @@ int launch_self_potential(gf_ctx *ctx, const TreeView &t, const int64_t *pstart,
     double *bg;
     int32_t *direct;
     GF_TRY(launch_halo_bg(ctx, t, pstart, pp, nullptr, &bg, &direct));
-    const int block = GF_BH_BLOCK;
-    int64_t grid = (t.n + block - 1) / block;
-    grid = std::min<int64_t>(grid, (int64_t)sm_count() * (2048 / block));
-    GF_TRY(launch_bh(ctx, grid, t.n, t.pos, t.phalo, t.perm, t.pos, t.root, t.rend, t.bh, direct, bg, pp,
-                     penergy, raw, counters));
+    GF_TRY(launch_bh(ctx, t.n, t.pos, t.phalo, t.perm, t, direct, bg, pp, penergy, raw, counters));
     return GF_OK;
 }
 
@@ -440,10 +669,7 @@ int launch_external_potential(gf_ctx *ctx, const TreeView &t, const int64_t *pst
     double *bg;
     int32_t *direct;
     GF_TRY(launch_halo_bg(ctx, t, pstart_src, pp, ntarget_halo, &bg, &direct));
-    const int block = GF_BH_BLOCK;
-    int64_t grid = std::min<int64_t>((ntarget + block - 1) / block, (int64_t)sm_count() * (2048 / block));
-    GF_TRY(launch_bh(ctx, grid, ntarget, tpos, thalo, nullptr, t.pos, t.root, t.rend, t.bh, direct, bg, pp,
-                     penergy, raw, nullptr));
+    GF_TRY(launch_bh(ctx, ntarget, tpos, thalo, nullptr, t, direct, bg, pp, penergy, raw, nullptr));
     return GF_OK;
 }
 

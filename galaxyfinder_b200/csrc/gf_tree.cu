@@ -505,7 +505,8 @@ __global__ void preorder(int L, Build b) {
 }
 
 __global__ void emit_nodes(int nlev, float theta2, Build b, KnnNode *__restrict__ knn,
-                           BhNode *__restrict__ bh, int32_t *__restrict__ owner) {
+                           BhNode *__restrict__ bh, WalkNode *__restrict__ walk,
+                           int32_t *__restrict__ owner) {
     for (int node = blockIdx.x * blockDim.x + threadIdx.x; node < b.lev[nlev]; node += gridDim.x * blockDim.x) {
     const int i = b.pre[node];
     KnnNode k;
@@ -537,6 +538,30 @@ __global__ void emit_nodes(int nlev, float theta2, Build b, KnnNode *__restrict_
     h.lcount = k.lcount;
     h.count = k.count;
     bh[i] = h;
+    WalkNode w;
+    w.hx = (float)h.com[0];
+    w.hy = (float)h.com[1];
+    w.hz = (float)h.com[2];
+    w.open_lo = __double2float_rd(h.open_r2 * (1.0 - 2e-6));
+    if (w.open_lo < kWalkMinR2) w.open_lo = 0.f;
+    w.first = b.first[node];
+    w.nchild = b.nchild[node];
+    w.lstart = h.lstart;
+    w.lcount = h.lcount;
+    w.lx = (float)(h.com[0] - (double)w.hx);
+    w.ly = (float)(h.com[1] - (double)w.hy);
+    w.lz = (float)(h.com[2] - (double)w.hz);
+    w.mass = h.mass;
+    w.pre = i;
+    const double half_tr = 0.5 * ((double)q[0] + (double)q[1] + (double)q[2]);
+    w.txx = (float)(1.5 * (double)q[0] - half_tr);
+    w.tyy = (float)(1.5 * (double)q[1] - half_tr);
+    w.tzz = (float)(1.5 * (double)q[2] - half_tr);
+    w.txy = 3.f * q[3];
+    w.txz = 3.f * q[4];
+    w.tyz = 3.f * q[5];
+    w.pad = 0;
+    walk[node] = w;
     }
 }
 
@@ -714,19 +739,21 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
         // ---- output buffers
         const int64_t nout = fixed ? ncap : std::max(nnode, 1);  // node slots written
         const size_t obytes = al((size_t)nout * sizeof(KnnNode)) + al((size_t)nout * sizeof(BhNode)) +
+                              al((size_t)nout * sizeof(WalkNode)) +
                               2 * al((size_t)std::max(nhalo, 1) * 4) +
                               2 * al((size_t)std::max<int64_t>(n, 1) * 4);
         GF_TRY(ctx->tree[2].reserve(obytes + 256));
         char *op = ctx->tree[2].as<char>();
         KnnNode *knn = carve<KnnNode>(op, (size_t)nout);
         BhNode *bh = carve<BhNode>(op, (size_t)nout);
+        WalkNode *walk = carve<WalkNode>(op, (size_t)nout);
         int32_t *root = carve<int32_t>(op, std::max(nhalo, 1));
         int32_t *rend = carve<int32_t>(op, std::max(nhalo, 1));
         int32_t *phalo = carve<int32_t>(op, std::max<int64_t>(n, 1));
         int32_t *owner = carve<int32_t>(op, std::max<int64_t>(n, 1));
         if (fixed || nnode > 0) {
             emit_nodes<<<fixed ? fixed_grid : grid_exact(nnode, 256), 256, 0, s>>>(nlev, theta2, b, knn, bh,
-                                                                                  owner);
+                                                                                  walk, owner);
             GF_LAUNCH_CHECK();
             emit_roots<<<grid_exact(nhalo, 256), 256, 0, s>>>(nhalo, b, root, rend);
             GF_LAUNCH_CHECK();
@@ -742,6 +769,7 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
         out->rend = rend;
         out->knn = knn;
         out->bh = bh;
+        out->walk = walk;
         out->phalo = phalo;
         out->owner = owner;
         return GF_OK;

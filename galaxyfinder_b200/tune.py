@@ -17,8 +17,7 @@ the GPU and the workload), which build.py turns into -D flags.
           GF_KNNB_FILT x GF_KNNB_HEAPF (tile filter, heap order) for the
           float-key kernel; for the warp-per-query
           kernel GF_KNN_CHUNK, then GF_KNN_BLOCK x register cap   knn
-  bh      GF_BH_DYN, GF_BH_ACC, GF_BH_TMA (leaf staging), GF_BH_LEAF4, GF_BH_BLOCK,
-          then the register cap                        potential
+  bh      GF_BH_DYN, GF_BH_BLOCK, then the register cap   potential
   fft     GF_FFT_PENCILS                               smooth
   tsc     GF_TSC_TILE (0: direct global atomics)       tsc
   tree    GF_TREE_BLOCK                                tree
@@ -72,9 +71,6 @@ def stages(group: str):
                 [{"GF_KNN_BLOCK": b, "GF_KNN_MINB": minb(b, r)} for b in (128, 256) for r in REGCAPS]]
     if group == "bh":
         return [lambda base: [{"GF_BH_DYN": d} for d in (0, 1)],
-                lambda base: [{"GF_BH_ACC": a} for a in (0, 1)],
-                lambda base: [{"GF_BH_TMA": t} for t in (0, 1)],
-                lambda base: [{"GF_BH_LEAF4": v} for v in (0, 1)],
                 lambda base: [{"GF_BH_BLOCK": b, "GF_BH_MINB": 1} for b in (64, 128, 256)],
                 lambda base: [{"GF_BH_MINB": minb(base["GF_BH_BLOCK"], r)} for r in REGCAPS]]
     if group == "fft":
