@@ -2,12 +2,13 @@
 //
 // The reference (NewGalFinder/nnost.c:375-422 Find_Near, :560-630
 // findsphdensity) walks a COM octree per particle and keeps a sorted list of
-// the k closest particles, self included.  Three kernels compute the same
-// lists (GF_KNN_ALGO selects; the autotuner keeps the fastest):
-// knn_bucket_kernel and knn_fbucket_kernel (below) walk once per 32
-// tree-order queries with one query per lane (the second with float keys and
-// an exact certification); knn_kernel serves one query per warp, walking a
-// chunk of consecutive tree-order queries:
+// the k closest particles, self included.  Four kernels compute the same
+// lists (GF_KNN_ALGO selects one at build time): knn_net_kernel, the default
+// (3), and its predecessors knn_fbucket_kernel (2) and knn_bucket_kernel (1),
+// all below, walk once per 32 tree-order queries with one query per lane (the
+// first two with float keys and an exact certification); knn_kernel (0, and
+// the kernel of query subsets) serves one query per warp, walking a chunk of
+// consecutive tree-order queries:
 //   * the sorted list (k <= 32) lives in registers, entry j in lane j;
 //   * the list starts as the k closest of the previous query's list (or,
 //     for the first query of a chunk, of the 32 tree-order neighbours), with
@@ -1217,6 +1218,623 @@ knn_fbucket_kernel(int64_t n, int k, const float4 *__restrict__ pos, const int32
     }
 }
 
+// ------------------------------------------------- bucket kNN, sorted lists
+// As the float-key bucket kernel above (a warp walks the tree once for 32
+// tree-order queries, lane = query, certification in FP64), with the lists
+// kept by sorting networks instead of heaps.  A lane's k nearest so far are 32
+// sorted 32-bit keys in registers, float distance^2 bits with the low six
+// replaced by a slot number; the slot holds the particle's tree position in
+// shared memory.  Candidates that pass the lane's bound are appended to 16
+// waiting keys in shared memory; when some lane's are full (or a level of the
+// walk ends) all lanes sort theirs (63 compare-exchanges) and merge them into
+// their lists (16 + 80), two instructions per compare-exchange and no
+// divergence, and the 16 keys that fall out of the merge name the slots that
+// the next 16 waiting ones use.
+// Dropping six bits of the distance makes an order within 7.6e-6 uncertain:
+//   * the bound is the largest key's upper end plus one more such step, so
+//     that whatever the filter or a node's box rejects lies clear of the list;
+//   * the least key ever dropped by a merge is kept, and the list is certified
+//     as above against min(that key's lower end, the bound, the distance to
+//     the outside of the processed box); a query that fails goes to knn_kernel;
+//   * the certified list is ordered by its exact distances.
+// Lists shorter than 32 (k < 32, small halos) start with 32 - k keys below
+// every distance, so that the bound is always the last key.
+//
+// Small batches give a query two or four lanes, each with its own list of every
+// second or fourth group of four candidates; the bound is then the largest of
+// the lanes' 16th or 8th keys, and the lists are merged by shuffles at the end.
+//
+// What bounds it: issue slots (64 % used, 40 k warp instructions per 32
+// queries of a clumpy halo: about 8 k append, 7 k test 1100 candidates, 6 k
+// merge 15 times, 5 k visit 160 nodes, 4 k write the lists) and, below a wave
+// of warps, the latency of one warp's chain of node visits and tiles.
+// Heaps (knn_fbucket_kernel) -> networks: 4096 halos (7.0 M particles) 14.5 ->
+// 8.7 ms, 1,000,003 particles 3.71 -> 2.29 ms, 131,072 0.62 -> 0.39 ms, 120
+// 65 -> 16 us.  16 waiting keys, because 32 need 12.7 KB of shared memory per
+// warp instead of 8.6 (16 resident warps instead of 24) and sort twice the
+// keys at half the number of merges.  Tiles of 64 candidates over several
+// nodes (9.4 ms), tiles filled to 32 over several nodes (8.8) and L1 prefetches
+// of the next nodes (8.8 to 9.1) gained nothing over one node's particles at
+// a time.
+constexpr int kWait = 16;                 // waiting keys per lane
+constexpr int kSlotRows = 32 + kWait;     // slots: every listed or waiting key has its own
+constexpr int kNetWindow = 96;            // tree-order neighbours tested before the walk
+constexpr int kInfKey = 0x7fffffc0;       // above every distance (slot in the low bits)
+constexpr int kZeroKey = 64;              // keys below: distance zero
+struct __align__(16) NetWarp {
+    int row[kSlotRows + kWait][32];  // slots, then the waiting keys; a column per lane
+    float x[32], y[32], z[32];       // candidates of the current tile
+};
+static_assert(kSlotRows <= 64, "the slot number has six bits");
+
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 f2_pack(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_unpack(f2 v, float &a, float &b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// Batcher's odd-even merge sort of N keys, ascending.
+template <int N>
+__device__ __forceinline__ void net_sort(int (&v)[N]) {
+#pragma unroll
+    for (int p = 1; p < N; p <<= 1) {
+#pragma unroll
+        for (int k = p; k >= 1; k >>= 1) {
+#pragma unroll
+            for (int a = 0; a < N; a++) {
+                // a pairs with a + k when it starts a block of 2k (offset k mod p)
+                // and both lie in the same run of 2p
+                const int r = a - k % p;
+                if (r >= 0 && r % (2 * k) < k && a + k < N && a / (2 * p) == (a + k) / (2 * p)) {
+                    const int lo = min(v[a], v[a + k]), hi = max(v[a], v[a + k]);
+                    v[a] = lo;
+                    v[a + k] = hi;
+                }
+            }
+        }
+    }
+}
+
+// A bitonic sequence of 32 keys in ascending order.
+__device__ __forceinline__ void net_clean(int (&v)[32]) {
+#pragma unroll
+    for (int st = 16; st > 0; st >>= 1) {
+#pragma unroll
+        for (int a = 0; a < 32; a++) {
+            if (a & st) continue;
+            const int lo = min(v[a], v[a + st]), hi = max(v[a], v[a + st]);
+            v[a] = lo;
+            v[a + st] = hi;
+        }
+    }
+}
+
+template <int S, bool COUNT>
+__global__ void __launch_bounds__(GF_KNNB_BLOCK, GF_KNNB_MINB)
+knn_net_kernel(int64_t n, int k, const float4 *__restrict__ pos, const int32_t *__restrict__ perm,
+               const float4 *__restrict__ pos_batch, const int32_t *__restrict__ phalo,
+               const int64_t *__restrict__ pstart, const int32_t *__restrict__ owner,
+               const KnnNode *__restrict__ nodes, int32_t *__restrict__ nearindex,
+               float *__restrict__ dens, int2 *__restrict__ redo, unsigned *__restrict__ nredo,
+               unsigned long long *__restrict__ counters, unsigned long long *__restrict__ work) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x & 31;
+    NetWarp &W = reinterpret_cast<NetWarp *>(smem)[threadIdx.x >> 5];
+    // S consecutive lanes share a query: each takes every S-th group of four
+    // candidates into a list of its own
+    constexpr int kOwn = 32 / S;  // a lane's part of the 32 nearest; queries per warp
+    const int sub = lane % S;
+    int *const col = &W.row[0][lane];         // row r of this lane: col[32 * r]
+    int *const qcol = &W.row[0][lane - sub];  // the query's column at the end
+    // work counters: node tests, particle tests, keys appended (per lane),
+    // warp-wide append steps, queries sent to the exact kernel
+    unsigned long long ctr[5] = {0, 0, 0, 0, 0};
+    const float kInfF = __int_as_float(0x7f800000);
+    const bool vec_out = k % 4 == 0 && ((uintptr_t)nearindex & 15) == 0;
+    const int64_t wid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t nbucket = (n + kOwn - 1) / kOwn;
+    // the warp's next bucket: from the work counter, or grid-stride
+    auto next = [&](int64_t stride_bucket) -> int64_t {
+        if (!GF_KNNB_DYN || !work) return stride_bucket;
+        unsigned long long b = 0;
+        if (lane == 0) b = atomicAdd(work, 1ull);
+        return (int64_t)__shfl_sync(0xffffffffu, b, 0);
+    };
+    for (int64_t bucket = next(wid); bucket < nbucket; bucket = next(bucket + nwarps)) {
+        const int64_t b = bucket * kOwn;
+        const int64_t q = b + lane / S;
+        const bool valid = q < n;
+        const int h = valid ? phalo[q] : -1;
+        const float4 Q = valid ? pos[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const f2 nqx = f2_pack(-Q.x, -Q.x), nqy = f2_pack(-Q.y, -Q.y), nqz = f2_pack(-Q.z, -Q.z);
+        unsigned remaining = __ballot_sync(0xffffffffu, valid);
+        while (remaining) {
+            const int leader = __ffs(remaining) - 1;
+            const int hl = __shfl_sync(0xffffffffu, h, leader);
+            const unsigned act = __ballot_sync(0xffffffffu, valid && h == hl);
+            remaining &= ~act;
+            const bool me = (act >> lane) & 1;
+            const int qa = (int)(b + leader / S);
+            const int qb = (int)(b + (31 - __clz(act)) / S);
+            const int hs = (int)pstart[hl], he = (int)pstart[hl + 1];
+            const int kk = min(k, he - hs);
+            const int nph = 32 - kk;  // keys below every distance, of all S lists
+            // ---- the lists start as kk particles about the bucket
+            const int f0 = min(qa, he - kk);
+            int K[32];
+            {
+                const int own = (kk - sub + S - 1) / S;  // of the kk, this lane's
+                int first[kOwn];
+#pragma unroll
+                for (int t = 0; t < kOwn; t++) {
+                    const int c = f0 + (t - (kOwn - own)) * S + sub;
+                    first[t] = (int)0x80000000 | t;
+                    if (t >= kOwn - own) {
+                        first[t] = (__float_as_int(f_d2_fma(Q, pos[c])) & ~63) | t;
+                        col[32 * t] = c;
+                    }
+                }
+                net_sort(first);
+#pragma unroll
+                for (int t = 0; t < 32; t++) K[t] = t < kOwn ? first[t < kOwn ? t : 0] : kInfKey | t;
+            }
+            int cnt = 0;              // waiting keys
+            int dropped = 0x7fffffff; // least key dropped by a merge
+#pragma unroll
+            for (int j = 0; j < kWait; j++) col[32 * (kSlotRows + j)] = kInfKey | (32 + j);
+            // the largest of the lanes' kOwn-th keys (together 32 keys lie at
+            // or below it): its upper end and one step more (at most the
+            // largest finite float: a distance that overflows is never taken)
+            auto bound = [&]() {
+                int top = K[kOwn - 1];
+#pragma unroll
+                for (int o = 1; o < S; o <<= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+                return me ? __int_as_float((min(top, 0x7f800000 - 128) | 63) + 64) : -1.f;
+            };
+            float bf = bound();
+            // ---- the tree-order window about the bucket, then the walk from
+            // the smallest subtree holding [qa, qb]
+            int win0 = qa - (kNetWindow - 32) / 2;
+            win0 = max(hs, min(win0, he - kNetWindow));
+            const int win1 = min(he, max(win0 + kNetWindow, f0 + kk));
+            win0 = min(win0, f0);
+            int c = owner[qa];
+            KnnNode C = nodes[c];
+            while (!(C.lstart <= qa && qb < C.lstart + C.count) && C.parent >= 0) {
+                c = C.parent;
+                C = nodes[c];
+            }
+            int i = c, iend = C.skip, parent = C.parent, x0 = -1, x1 = -1;
+            // candidate ranges to test: r0..r1, then s0..s1 (the part of a
+            // node's loose particles before and after the window)
+            int r0 = win0, r1 = f0, s0 = f0 + kk, s1 = win1;
+            double tbox = 0.0;  // squared distance from the query to the outside of the processed box
+            while (true) {
+                // ---- the next tile of up to 32 candidates, or the end of a level
+                bool level_end = false;
+                if (r0 >= r1) {
+                    r0 = s0;
+                    r1 = s1;
+                    s0 = s1 = 0;
+                }
+                while (r0 >= r1) {
+                    if (i == x0) i = x1;
+                    if (i >= iend) {
+                        level_end = true;
+                        break;
+                    }
+                    const float4 *nv = reinterpret_cast<const float4 *>(nodes + i);  // one broadcast line
+                    const float4 n0 = __ldg(nv), n1 = __ldg(nv + 1);
+                    const float gx = fmaxf(fmaxf(n0.x - Q.x, Q.x - n0.w), 0.f);
+                    const float gy = fmaxf(fmaxf(n0.y - Q.y, Q.y - n1.x), 0.f);
+                    const float gz = fmaxf(fmaxf(n0.z - Q.z, Q.z - n1.y), 0.f);
+                    const float lb = __fmaf_rn(gx, gx, __fmaf_rn(gy, gy, __fmul_rn(gz, gz)));
+                    if (COUNT) ctr[0]++;
+                    if (!__any_sync(0xffffffffu, lb <= bf)) {
+                        i = __float_as_int(n1.z);  // the whole subtree lies beyond every bound
+                        continue;
+                    }
+                    i++;
+                    const int l0 = __float_as_int(n1.w);
+                    const int l1 = l0 + __float_as_int(__ldg(reinterpret_cast<const float *>(nv + 2)));
+                    r0 = l0;
+                    r1 = l1;
+                    if (l0 < win1 && l1 > win0) {  // without the window
+                        r1 = min(l1, win0);
+                        s0 = max(l0, win1);
+                        s1 = l1;
+                        if (r0 >= r1) {
+                            r0 = s0;
+                            r1 = s1;
+                            s0 = s1 = 0;
+                        }
+                    }
+                }
+                unsigned pass = 0;
+                int base = 0;
+                if (!level_end) {
+                    base = r0;
+                    const int m = min(32, r1 - r0);
+                    r0 += m;
+                    float4 cand = make_float4(kInfF, kInfF, kInfF, 0.f);  // padding: at no finite distance
+                    if (lane < m) cand = pos[base + lane];
+                    W.x[lane] = cand.x;
+                    W.y[lane] = cand.y;
+                    W.z[lane] = cand.z;
+                    __syncwarp();
+                    if (COUNT) ctr[1] += m;
+                    // filter: a branch-free pass over the tile against the
+                    // bound at its start (the bound only tightens)
+#pragma unroll 2
+                    for (int t0 = 0; t0 < m; t0 += 4 * S) {
+                        const int t = t0 + 4 * sub;
+                        const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(&W.x[t]);
+                        const ulonglong2 Y = *reinterpret_cast<const ulonglong2 *>(&W.y[t]);
+                        const ulonglong2 Z = *reinterpret_cast<const ulonglong2 *>(&W.z[t]);
+                        unsigned four = 0;
+#pragma unroll
+                        for (int u = 0; u < 2; u++) {
+                            const f2 dx = f2_add(u ? X.y : X.x, nqx), dy = f2_add(u ? Y.y : Y.x, nqy);
+                            const f2 dz = f2_add(u ? Z.y : Z.x, nqz);
+                            float fa, fb;
+                            f2_unpack(f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz))), fa, fb);
+                            if (fa <= bf) four |= 1u << (2 * u);
+                            if (fb <= bf) four |= 2u << (2 * u);
+                        }
+                        pass |= four << t;
+                    }
+                    if (COUNT) {
+                        ctr[2] += __popc(pass);
+                        ctr[3] += __reduce_max_sync(0xffffffffu, (unsigned)__popc(pass));
+                    }
+                }
+                // ---- append the survivors, each lane its own; merge when a
+                // lane has no room left or a level ends with keys waiting
+                bool merge;
+                do {
+                    while (pass && cnt < kWait) {
+                        const int t = __ffs(pass) - 1;
+                        pass &= pass - 1;
+                        const float f = f_d2_fma(Q, make_float4(W.x[t], W.y[t], W.z[t], 0.f));
+                        int *w = col + 32 * (kSlotRows + cnt);
+                        const int slot = *w & 63;
+                        *w = (__float_as_int(f) & ~63) | slot;
+                        col[32 * slot] = base + t;
+                        cnt++;
+                    }
+                    const bool more = __any_sync(0xffffffffu, pass != 0u);
+                    merge = more || (level_end && __any_sync(0xffffffffu, cnt > 0));
+                    if (merge) {
+                        int P[kWait];
+#pragma unroll
+                        for (int j = 0; j < kWait; j++) P[j] = col[32 * (kSlotRows + j)];
+                        net_sort(P);
+                        // the 32 smallest of both, a bitonic sequence; the
+                        // other 16 are dropped and free their slots
+#pragma unroll
+                        for (int j = 0; j < kWait; j++) {
+                            const int a = K[32 - kWait + j], d = P[kWait - 1 - j];
+                            const int out = max(a, d);
+                            K[32 - kWait + j] = min(a, d);
+                            dropped = min(dropped, out);
+                            col[32 * (kSlotRows + j)] = kInfKey | (out & 63);
+                        }
+                        net_clean(K);
+                        cnt = 0;
+                        bf = bound();
+                        // a dropped particle at distance zero: more than 32 lie
+                        // on the query, which only the exact kernel can order
+                        if (dropped < kZeroKey) bf = -1.f;
+                        merge = more;
+                    }
+                } while (merge);
+                __syncwarp();  // the tile is read; the next one may be written
+                if (!level_end) continue;
+                // distance from the query to the outside of the processed box
+                // (exact differences of floats, squared in double)
+                const float4 *cv = reinterpret_cast<const float4 *>(nodes + c);
+                const float4 c0 = __ldg(cv), c1 = __ldg(cv + 1);
+                const double dbx = fmin((double)Q.x - (double)c0.x, (double)c0.w - (double)Q.x);
+                const double dby = fmin((double)Q.y - (double)c0.y, (double)c1.x - (double)Q.y);
+                const double dbz = fmin((double)Q.z - (double)c0.z, (double)c1.y - (double)Q.z);
+                const double db = fmin(fmin(dbx, dby), dbz);
+                tbox = parent < 0 ? kInf : (db > 0.0 ? db * db : 0.0);
+                const bool done = !me || tbox > (double)bf * (1.0 + 4e-6);
+                if (parent < 0 || __all_sync(0xffffffffu, done)) break;
+                x0 = c;
+                x1 = __float_as_int(c1.z);
+                c = parent;
+                const KnnNode *A = nodes + c;
+                i = c;
+                iend = A->skip;
+                parent = A->parent;
+            }
+            // ---- the lists become one, in key order; row 32 + e of the
+            // query's column its tree positions
+            {
+                int I[32];
+#pragma unroll
+                for (int e = 0; e < 32; e++) I[e] = col[32 * (K[e] & 63)];
+#pragma unroll
+                for (int e = 0; e < 32; e++) col[32 * (32 + e)] = I[e];
+            }
+            if (S > 1) {
+                // keys now name (list, place); one step of the distance is
+                // kCode + 1 units in the last place
+                constexpr int kCode = S > 2 ? 127 : 63;
+#pragma unroll
+                for (int e = 0; e < 32; e++) K[e] = (K[e] & ~kCode) | (sub << 5) | e;
+#pragma unroll
+                for (int o = 1; o < S; o <<= 1) {
+#pragma unroll
+                    for (int e = 0; e < 16; e++) {
+                        const int pa = __shfl_xor_sync(0xffffffffu, K[31 - e], o);
+                        const int pb = __shfl_xor_sync(0xffffffffu, K[e], o);
+                        dropped = min(dropped, min(max(K[e], pa), max(K[31 - e], pb)));
+                        K[e] = min(K[e], pa);
+                        K[31 - e] = min(K[31 - e], pb);
+                    }
+                    net_clean(K);
+                    dropped = min(dropped, __shfl_xor_sync(0xffffffffu, dropped, o));
+                }
+                dropped &= ~kCode;
+                int T[kOwn];  // entries sub, sub + S, ... of the query's list
+#pragma unroll
+                for (int j = 0; j < kOwn; j++) {
+                    int code = K[j * S];
+#pragma unroll
+                    for (int u = 1; u < S; u++) code = sub == u ? K[j * S + u] : code;
+                    code &= kCode;
+                    T[j] = W.row[32 + (code & 31)][lane - sub + (code >> 5)];
+                }
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < kOwn; j++) qcol[32 * (32 + j * S + sub)] = T[j];
+            }
+            __syncwarp();
+            // exact FP64 distances in that order: row e their float (the
+            // density needs nothing else), row 32 + e the batch index
+            bool sorted = true;
+            double dprev = -1.0;
+            int iprev = -1;
+#pragma unroll 4
+            for (int e0 = 0; e0 < 32; e0 += S) {
+                const int e = e0 + sub;
+                double d = -1.0;
+                int id = -1;
+                if (me && e >= nph) {
+                    const int tp = qcol[32 * (32 + e)];
+                    id = perm[tp];
+                    d = exact_d2(Q, pos[tp]);
+                    qcol[32 * e] = __float_as_int((float)d);
+                    qcol[32 * (32 + e)] = id;
+                }
+                if (S == 1) {
+                    sorted = sorted && !key_lt(d, id, dprev, iprev);
+                    dprev = d;
+                    iprev = id;
+                } else {
+                    // against the entry before: the lane before, or the last
+                    // lane's of the step before
+                    double dl = __shfl_up_sync(0xffffffffu, d, 1, S);
+                    int il = __shfl_up_sync(0xffffffffu, id, 1, S);
+                    if (sub == 0) {
+                        dl = dprev;
+                        il = iprev;
+                    }
+                    sorted = sorted && !key_lt(d, id, dl, il);
+                    dprev = __shfl_sync(0xffffffffu, d, S - 1, S);
+                    iprev = __shfl_sync(0xffffffffu, id, S - 1, S);
+                }
+            }
+#pragma unroll
+            for (int o = 1; o < S; o <<= 1) sorted = __shfl_xor_sync(0xffffffffu, sorted, o) && sorted;
+            __syncwarp();
+            if (me && !sorted && sub == 0) {
+                // near-ties ordered differently by the keys: insertion sort by
+                // the exact distance (recomputed) and index
+                for (int e = nph + 1; e < 32; e++) {
+                    const int vid = qcol[32 * (32 + e)], vf = qcol[32 * e];
+                    const double vd = exact_d2(Q, pos_batch[vid]);
+                    int f = e;
+                    for (; f > nph; f--) {
+                        const int uid = qcol[32 * (32 + f - 1)];
+                        if (!key_lt(vd, vid, exact_d2(Q, pos_batch[uid]), uid)) break;
+                        qcol[32 * f] = qcol[32 * (f - 1)];
+                        qcol[32 * (32 + f)] = uid;
+                    }
+                    qcol[32 * f] = vf;
+                    qcol[32 * (32 + f)] = vid;
+                }
+            }
+            __syncwarp();
+            if (me && !sorted) dprev = exact_d2(Q, pos_batch[qcol[32 * 63]]);
+            // a lower bound of the exact distance^2 of every particle not kept
+            const float fd = dropped < 0x7f800000 ? __int_as_float(dropped & ~63) : kInfF;
+            const bool ok = dprev < fmin((double)fminf(fd, bf) * (1.0 - 2e-6), tbox * (1.0 - 1e-12));
+            const int myid = me ? perm[q] : 0;
+            if (me && ok) {
+                int32_t *row = nearindex + (int64_t)myid * k;
+                const int *ids = qcol + 32 * (32 + nph);
+                if (vec_out) {
+                    for (int j = 4 * sub; j < k; j += 4 * S) {
+                        int4 v;
+                        v.x = j < kk ? ids[32 * j] - hs : -1;
+                        v.y = j + 1 < kk ? ids[32 * (j + 1)] - hs : -1;
+                        v.z = j + 2 < kk ? ids[32 * (j + 2)] - hs : -1;
+                        v.w = j + 3 < kk ? ids[32 * (j + 3)] - hs : -1;
+                        *reinterpret_cast<int4 *>(row + j) = v;
+                    }
+                } else {
+                    for (int j = sub; j < k; j += S) row[j] = j < kk ? ids[32 * j] - hs : -1;
+                }
+            }
+            if (me && !ok && sub == 0) {
+                redo[atomicAdd(nredo, 1u)] = make_int2((int)q, dropped < kZeroKey ? 2 * kZeroKey - 1 : __float_as_int(bf));
+                if (COUNT) ctr[4]++;
+            }
+            if (dens) {
+                // nnost.c:292,415: maxr = sqrtf(maxdist2); W4(sqrtf(d2_j), maxr/2.),
+                // summed in list order
+                const float neardist = sqrtf((float)dprev);
+                const float hh = (float)(neardist / 2.);
+                float rho = 0.f;
+                for (int e0 = 0; e0 < 32; e0 += S) {
+                    const int e = e0 + sub;
+                    const float w = me && ok && e >= nph ? w4(sqrtf(__int_as_float(qcol[32 * e])), hh) : 0.f;
+                    if (S == 1) {
+                        rho += w;
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < S; u++) rho += __shfl_sync(0xffffffffu, w, u, S);
+                    }
+                }
+                if (me && ok && sub == 0) dens[myid] = rho;
+            }
+            __syncwarp();
+        }
+    }
+    if (COUNT && counters) {
+        for (int off = 16; off; off >>= 1) {
+            ctr[2] += __shfl_xor_sync(0xffffffffu, ctr[2], off);
+            ctr[4] += __shfl_xor_sync(0xffffffffu, ctr[4], off);
+        }
+        if (lane == 0)
+            for (int e = 0; e < 5; e++) atomicAdd(counters + e, ctr[e]);
+    }
+}
+
+// The queries that knn_net_kernel could not certify, exactly, a warp each.
+// The list's bound bf covers every particle that can be among the k nearest
+// (it lies at least 64 units in the last place above the k-th float
+// distance), so one pruned expansion of the tree from the root finds them:
+// nodes wait on a stack, 32 are tested at once (lane = node; children are
+// consecutive in the walk numbering, their boxes are read through the
+// preorder index), and the loose particles within bf are merged by exact
+// distance and index.  A handful of dependent steps per query: the bottom-up
+// walk of knn_kernel took 25 to 130 us for the few queries of a launch, most
+// of it latency that nothing else covers.
+constexpr int kRedoStack = 416;
+__global__ void __launch_bounds__(128) knn_redo_kernel(
+    int k, const float4 *__restrict__ pos, const int32_t *__restrict__ perm, const int32_t *__restrict__ phalo,
+    const int64_t *__restrict__ pstart, const KnnNode *__restrict__ nodes, const WalkNode *__restrict__ walk,
+    int32_t *__restrict__ nearindex, float *__restrict__ dens, int *err, const int2 *__restrict__ redo,
+    const unsigned *__restrict__ nredo) {
+    __shared__ int stacks[4][kRedoStack];
+    const int lane = threadIdx.x & 31;
+    int *stack = stacks[threadIdx.x >> 5];
+    const unsigned n = *nredo;
+    for (unsigned e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < n; e += (gridDim.x * blockDim.x) >> 5) {
+        const int q = redo[e].x;
+        float bf = __int_as_float(redo[e].y);
+        if (bf >= FLT_MAX) bf = __int_as_float(0x7f800000);  // no bound was found
+        const int h = phalo[q];
+        const int hs = (int)pstart[h], he = (int)pstart[h + 1];
+        const float4 Q = pos[q];
+        ListState L;
+        L.Ld = L.bd = kInf;
+        L.Li = L.bi = INT_MAX;
+        L.cnt = 0;
+        L.kk = min(k, he - hs);
+        unsigned long long none = 0;
+        auto scan = [&](int l0, int l1) {
+            for (int base = l0; base < l1; base += 32) {
+                const int j = base + lane;
+                double d = kInf;
+                int id = INT_MAX;
+                bool in = false;
+                if (j < l1) {
+                    const float4 P = pos[j];
+                    if (f_d2(Q, P) <= bf) {
+                        d = exact_d2(Q, P);
+                        id = perm[j];
+                        in = !key_lt(L.bd, L.bi, d, id);
+                    }
+                }
+                const unsigned mask = __ballot_sync(0xffffffffu, in);
+                if (mask) merge_batch(mask, d, id, L.Ld, L.Li, L.cnt, L.kk, L.bd, L.bi, none, none);
+            }
+        };
+        __syncwarp();
+        if (lane == 0) stack[0] = h;
+        __syncwarp();
+        int top = 1;
+        while (top > 0) {
+            int take = min(min(32, top), (kRedoStack - top) / 7);
+            const bool full = take < 1;
+            take = max(take, 1);
+            top -= take;
+            const int node = lane < take ? stack[top + lane] : 0;
+            __syncwarp();
+            int4 lk = make_int4(0, 0, 0, 0);  // first, nchild, lstart, lcount
+            int pre = 0;
+            if (lane < take) {
+                lk = __ldg(reinterpret_cast<const int4 *>(walk + node) + 1);
+                pre = __ldg(&walk[node].pre);
+            }
+            if (full) {  // no room for this node's children: its preorder range in turn
+                const int p0 = __shfl_sync(0xffffffffu, pre, 0), p1 = nodes[p0].skip;
+                for (int i = p0; i < p1;) {
+                    const KnnNode nd = nodes[i];
+                    const bool in = f_box_lb2(Q, nd) <= bf;
+                    if (in) scan(nd.lstart, nd.lstart + nd.lcount);
+                    i = in ? i + 1 : nd.skip;
+                }
+                continue;
+            }
+            const bool in = lane < take && f_box_lb2(Q, nodes[pre]) <= bf;
+            const int nch = in ? lk.y : 0;
+            int at = nch;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, at, o);
+                if (lane >= o) at += v;
+            }
+            for (int c = 0, s0 = top + at - nch; c < nch; c++) stack[s0 + c] = lk.x + c;
+            top += __shfl_sync(0xffffffffu, at, 31);
+            __syncwarp();
+            for (unsigned lb = __ballot_sync(0xffffffffu, in && lk.w > 0); lb; lb &= lb - 1) {
+                const int src = __ffs(lb) - 1;
+                const int l0 = __shfl_sync(0xffffffffu, lk.z, src);
+                scan(l0, l0 + __shfl_sync(0xffffffffu, lk.w, src));
+            }
+        }
+        if (L.cnt < L.kk) {
+            if (lane == 0) atomicOr(err, GF_ERRBIT_KNN);
+            continue;
+        }
+        const int64_t qo = perm[q];
+        if (lane < k) nearindex[qo * k + lane] = lane < L.kk ? L.Li - hs : -1;
+        // nnost.c:292,415: maxr = sqrtf(maxdist2); W4(sqrtf(d2_j), maxr/2.)
+        const float neardist = sqrtf((float)__shfl_sync(0xffffffffu, L.Ld, L.kk - 1));
+        const float hh = (float)(neardist / 2.);
+        const float wj = lane < L.kk ? w4(sqrtf((float)L.Ld), hh) : 0.f;
+        float rho = 0.f;
+        for (int j = 0; j < L.kk; j++) rho += __shfl_sync(0xffffffffu, wj, j);
+        if (lane == 0 && dens) dens[qo] = rho;
+    }
+}
+
 }  // namespace
 
 int launch_knn(gf_ctx *ctx, const TreeView &t, const int64_t *pstart, const float4 *pos_batch, int k,
@@ -1228,21 +1846,46 @@ int launch_knn(gf_ctx *ctx, const TreeView &t, const int64_t *pstart, const floa
     }
     const int64_t nquery = qlist ? nq : t.n;
     if (t.n <= 0 || nquery <= 0) return GF_OK;
-    if (GF_KNN_ALGO == 2 && !qlist) {
-        // scratch: the list of queries the float-key kernel could not certify
-        GF_TRY(ctx->tmp[7].reserve((size_t)t.n * sizeof(int32_t) + 256));
-        unsigned *nredo = ctx->tmp[7].as<unsigned>();
-        int32_t *redo = reinterpret_cast<int32_t *>(ctx->tmp[7].as<char>() + 256);
-        GF_CUDA_TRY(cudaMemsetAsync(nredo, 0, sizeof(unsigned), ctx->stream));
+#if GF_KNN_ALGO >= 2
+    if (!qlist) {
         const int block = GF_KNNB_BLOCK;
-        const size_t shmem = (size_t)(block / 32) * kFBucketWarpBytes;
         int per_sm = 0;
+#if GF_KNN_ALGO == 3
+        using Redo = int2;
+        const size_t shmem = (size_t)(block / 32) * sizeof(NetWarp);
+        auto kern = counters ? knn_net_kernel<1, true> : knn_net_kernel<1, false>;
+#else
+        using Redo = int32_t;
+        const size_t shmem = (size_t)(block / 32) * kFBucketWarpBytes;
         auto kern = counters ? knn_fbucket_kernel<true> : knn_fbucket_kernel<false>;
+#endif
+        // scratch: the list of queries the float-key kernel could not certify
+        GF_TRY(ctx->tmp[7].reserve((size_t)t.n * sizeof(Redo) + 256));
+        unsigned *nredo = ctx->tmp[7].as<unsigned>();
+        Redo *redo = reinterpret_cast<Redo *>(ctx->tmp[7].as<char>() + 256);
+        GF_CUDA_TRY(cudaMemsetAsync(nredo, 0, sizeof(unsigned), ctx->stream));
         GF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem));
         GF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, shmem));
-        const int64_t nbucket = (t.n + 31) / 32;
-        int64_t grid = (nbucket * 32 + block - 1) / block;
-        grid = std::max<int64_t>(1, std::min<int64_t>(grid, (int64_t)sm_count() * std::max(per_sm, 1)));
+        const int64_t wave = (int64_t)sm_count() * std::max(per_sm, 1);  // resident blocks
+        int lanes = 1;  // per query
+#if GF_KNN_ALGO == 3
+        // Fewer queries per warp where 32 would leave warps idle: a warp's own
+        // time falls (a smaller part of the tree, shorter lists) while the
+        // work of all of them grows.  us with 1 / 2 / 4 lanes: 120 particles
+        // 30 / 21 / 16, 36,001 267 / 212 / 211, 131,072 425 / 395 / 489,
+        // 1,000,003 2300 / 2660 / 3440.
+        const int64_t warps = wave * (block / 32);
+        if (t.n <= 8 * warps) {
+            lanes = 4;
+            kern = counters ? knn_net_kernel<4, true> : knn_net_kernel<4, false>;
+        } else if (2 * t.n <= 5 * 16 * warps) {
+            lanes = 2;
+            kern = counters ? knn_net_kernel<2, true> : knn_net_kernel<2, false>;
+        }
+        if (lanes > 1) GF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem));
+#endif
+        const int64_t nbucket = (t.n * lanes + 31) / 32;
+        const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((nbucket * 32 + block - 1) / block, wave));
         unsigned long long *work = nullptr;
         if (GF_KNNB_DYN) {  // one resident wave; each warp takes its next bucket from a counter
             GF_TRY(ctx->work.reserve(256));
@@ -1254,12 +1897,18 @@ int launch_knn(gf_ctx *ctx, const TreeView &t, const int64_t *pstart, const floa
         GF_LAUNCH_CHECK();
         // the uncertified queries, exactly, into their own rows (the count
         // stays on the device; the grid strides over whatever it is)
+#if GF_KNN_ALGO == 3
+        knn_redo_kernel<<<(int)std::min<int64_t>((t.n + 3) / 4, sm_count() * 8), 128, 0, ctx->stream>>>(
+            k, t.pos, t.perm, t.phalo, pstart, t.knn, t.walk, nearindex, dens, ctx->d_err, redo, nredo);
+#else
         knn_kernel<false><<<sm_count() * (2048 / GF_KNN_BLOCK), GF_KNN_BLOCK, 0, ctx->stream>>>(
             t.n, k, t.pos, t.perm, pos_batch, t.phalo, pstart, t.owner, t.knn, nearindex, dens, ctx->d_err,
             nullptr, redo, nredo, true, 1);  // scattered queries: one per warp task
+#endif
         GF_LAUNCH_CHECK();
         return GF_OK;
     }
+#endif
     if (GF_KNN_ALGO == 1 && !qlist) {
         const int block = GF_KNNB_BLOCK;
         const size_t shmem = (size_t)(block / 32) * kBucketWarpBytes;
@@ -1276,17 +1925,17 @@ int launch_knn(gf_ctx *ctx, const TreeView &t, const int64_t *pstart, const floa
         return GF_OK;
     }
     const int block = GF_KNN_BLOCK;
-    const int64_t warps_needed = (nquery + kChunk - 1) / kChunk;
+    // consecutive queries of a task start from each other's lists, but few
+    // queries are spread over the SMs' warps first (4096 probes of 1e6
+    // particles: 32 per warp kept 128 warps busy for 1.07 ms)
+    const int64_t all_warps = (int64_t)sm_count() * (2048 / 32);
+    const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(kChunk, nquery / all_warps));
+    const int64_t warps_needed = (nquery + chunk - 1) / chunk;
     int64_t grid = (warps_needed * 32 + block - 1) / block;
     grid = std::max<int64_t>(1, std::min<int64_t>(grid, (int64_t)sm_count() * (2048 / block)));
-    if (counters)
-        knn_kernel<true><<<(int)grid, block, 0, ctx->stream>>>(nquery, k, t.pos, t.perm, pos_batch, t.phalo,
-                                                               pstart, t.owner, t.knn, nearindex, dens,
-                                                               ctx->d_err, counters, qlist);
-    else
-        knn_kernel<false><<<(int)grid, block, 0, ctx->stream>>>(nquery, k, t.pos, t.perm, pos_batch, t.phalo,
-                                                                pstart, t.owner, t.knn, nearindex, dens,
-                                                                ctx->d_err, nullptr, qlist);
+    auto kern = counters ? knn_kernel<true> : knn_kernel<false>;
+    kern<<<(int)grid, block, 0, ctx->stream>>>(nquery, k, t.pos, t.perm, pos_batch, t.phalo, pstart, t.owner, t.knn,
+                                               nearindex, dens, ctx->d_err, counters, qlist, nullptr, false, chunk);
     GF_LAUNCH_CHECK();
     return GF_OK;
 }
