@@ -43,10 +43,12 @@ __device__ __forceinline__ float fkey_inv(unsigned k) {
 // BFS-numbered node arrays used while building.
 struct Build {
     int32_t *start, *count, *halo;
+    // accumulators, zeroed when their node is allocated (a memset of the node
+    // capacity touched ten times the nodes that a tree has)
     double *m, *mx, *my, *mz;       // mass and first moments, then COM in mx..mz
     unsigned *r2;                   // float bits of max |x - com|^2
     float *q;                       // 6 second moments
-    unsigned *box;                  // 6 fkeys: min xyz, max xyz
+    unsigned *box;                  // 6 fkeys as maxima: ~min xyz, max xyz
     int32_t *oct;                   // 8 octant counts
     int32_t *cur;                   // 8 octant cursors
     int32_t *ochild;                // 8 child ids or -1
@@ -56,6 +58,20 @@ struct Build {
     int32_t *counter;               // [0] nodes allocated, [1] overflow flag, [2] blocks done
     int32_t *lev;                   // level L holds BFS nodes [lev[L], lev[L+1])
 };
+
+__device__ __forceinline__ void zero_node(const Build &b, int node) {
+    b.m[node] = b.mx[node] = b.my[node] = b.mz[node] = 0.0;
+    b.r2[node] = 0u;
+    float2 *q = reinterpret_cast<float2 *>(b.q + 6 * (int64_t)node);
+    uint2 *box = reinterpret_cast<uint2 *>(b.box + 6 * (int64_t)node);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        q[i] = make_float2(0.f, 0.f);
+        box[i] = make_uint2(0u, 0u);
+    }
+    int4 *oct = reinterpret_cast<int4 *>(b.oct + 8 * (int64_t)node);
+    oct[0] = oct[1] = make_int4(0, 0, 0, 0);
+}
 
 constexpr int kMaxLevels = 4096;
 
@@ -81,6 +97,7 @@ __global__ void init_roots(int32_t nhalo, const int64_t *__restrict__ pstart, Bu
     b.count[h] = (int32_t)(pstart[h + 1] - pstart[h]);
     b.halo[h] = h;
     b.par[h] = -1;
+    zero_node(b, h);
 }
 
 __global__ void init_particles(int64_t n, const int64_t *__restrict__ pstart, int32_t nhalo,
@@ -137,9 +154,6 @@ __device__ __forceinline__ T run_scan(T v, const WarpRuns &r, Op op) {
 }
 struct AddOp {
     template <class T> __device__ __forceinline__ T operator()(T a, T b) const { return a + b; }
-};
-struct MinOp {
-    template <class T> __device__ __forceinline__ T operator()(T a, T b) const { return min(a, b); }
 };
 struct MaxOp {
     template <class T> __device__ __forceinline__ T operator()(T a, T b) const { return max(a, b); }
@@ -249,7 +263,7 @@ accum_moments(int64_t n, const float4 *__restrict__ pos, const int32_t *__restri
         const int64_t p = base + threadIdx.x;
         const int node = p < n ? pnode[p] : -1;
         float v[7] = {0, 0, 0, 0, 0, 0, 0};  // max |x - com|^2, then q0..q5
-        unsigned bx[6] = {~0u, ~0u, ~0u, 0u, 0u, 0u};
+        unsigned bx[6] = {0u, 0u, 0u, 0u, 0u, 0u};  // ~min xyz, max xyz: all maxima
         int key = 0;
         if (node >= 0) {
             const float4 P = pos[p];
@@ -266,9 +280,12 @@ accum_moments(int64_t n, const float4 *__restrict__ pos, const int32_t *__restri
             v[4] = m * tx * ty;
             v[5] = m * tx * tz;
             v[6] = q5_asbuilt ? m * ty * tx : m * ty * tz;
-            bx[0] = bx[3] = fkey(P.x);
-            bx[1] = bx[4] = fkey(P.y);
-            bx[2] = bx[5] = fkey(P.z);
+            bx[3] = fkey(P.x);
+            bx[4] = fkey(P.y);
+            bx[5] = fkey(P.z);
+            bx[0] = ~bx[3];
+            bx[1] = ~bx[4];
+            bx[2] = ~bx[5];
             // ost.c:589-592: SubCellDicision(x, monox) = x > monox
             key = ((double)P.x > cx ? 1 : 0) | ((double)P.y > cy ? 2 : 0) | ((double)P.z > cz ? 4 : 0);
             pkey[p] = (uint8_t)key;
@@ -281,26 +298,18 @@ accum_moments(int64_t n, const float4 *__restrict__ pos, const int32_t *__restri
             for (int off = 16; node >= 0 && off; off >>= 1) {
                 v[0] = fmaxf(v[0], __shfl_xor_sync(0xffffffffu, v[0], off));
                 for (int i = 1; i < 7; i++) v[i] += __shfl_xor_sync(0xffffffffu, v[i], off);
-                for (int i = 0; i < 3; i++) {
-                    bx[i] = min(bx[i], __shfl_xor_sync(0xffffffffu, bx[i], off));
-                    bx[3 + i] = max(bx[3 + i], __shfl_xor_sync(0xffffffffu, bx[3 + i], off));
-                }
             }
+            if (node >= 0)
+                for (int i = 0; i < 6; i++) bx[i] = __reduce_max_sync(0xffffffffu, bx[i]);
         } else {  // several nodes: segmented over the warp's runs
             const WarpRuns r = warp_runs(node);
             v[0] = run_scan(v[0], r, FMaxOp());
             for (int i = 1; i < 7; i++) v[i] = run_scan(v[i], r, AddOp());
-            for (int i = 0; i < 3; i++) {
-                bx[i] = run_scan(bx[i], r, MinOp());
-                bx[3 + i] = run_scan(bx[3 + i], r, MaxOp());
-            }
+            for (int i = 0; i < 6; i++) bx[i] = run_scan(bx[i], r, MaxOp());
             if (r.tail && node >= 0) {
                 atomicMax(b.r2 + node, __float_as_uint(v[0]));  // non-negative floats
                 for (int i = 0; i < 6; i++) atomicAdd(b.q + 6 * (int64_t)node + i, v[1 + i]);
-                for (int i = 0; i < 3; i++) {
-                    atomicMin(b.box + 6 * (int64_t)node + i, bx[i]);
-                    atomicMax(b.box + 6 * (int64_t)node + 3 + i, bx[3 + i]);
-                }
+                for (int i = 0; i < 6; i++) atomicMax(b.box + 6 * (int64_t)node + i, bx[i]);
             }
         }
         if (block_uniform) {  // then over the block: one atomic per value
@@ -320,9 +329,8 @@ accum_moments(int64_t n, const float4 *__restrict__ pos, const int32_t *__restri
             } else if (threadIdx.x < 13) {
                 const int i = threadIdx.x - 7;
                 unsigned a = s_k[i][0];
-                for (int w2 = 1; w2 < kWarps; w2++) a = i < 3 ? min(a, s_k[i][w2]) : max(a, s_k[i][w2]);
-                if (i < 3) atomicMin(b.box + 6 * (int64_t)s_node + i, a);
-                else atomicMax(b.box + 6 * (int64_t)s_node + i, a);
+                for (int w2 = 1; w2 < kWarps; w2++) a = max(a, s_k[i][w2]);
+                atomicMax(b.box + 6 * (int64_t)s_node + i, a);
             } else if (threadIdx.x >= 32 && threadIdx.x < 40) {
                 const int c = threadIdx.x - 32;
                 if (s_oct[c]) atomicAdd(b.oct + 8 * (int64_t)s_node + c, s_oct[c]);
@@ -332,10 +340,7 @@ accum_moments(int64_t n, const float4 *__restrict__ pos, const int32_t *__restri
             if (warp_uniform && node >= 0 && lane == 0) {
                 atomicMax(b.r2 + node, __float_as_uint(v[0]));
                 for (int i = 0; i < 6; i++) atomicAdd(b.q + 6 * (int64_t)node + i, v[1 + i]);
-                for (int i = 0; i < 3; i++) {
-                    atomicMin(b.box + 6 * (int64_t)node + i, bx[i]);
-                    atomicMax(b.box + 6 * (int64_t)node + 3 + i, bx[3 + i]);
-                }
+                for (int i = 0; i < 6; i++) atomicMax(b.box + 6 * (int64_t)node + i, bx[i]);
             }
             // octant counts: lanes sharing (node, key)
             const unsigned g2 = __match_any_sync(0xffffffffu, node * 8 + key);
@@ -354,11 +359,16 @@ __global__ void split_nodes(int L, int32_t ncap, int last, Build b) {
     const float r2 = __uint_as_float(b.r2[node]);
     const double nodesize = sqrt((double)r2);           // ost.c:574
     const bool divide = nodesize > 0.5 * kMinWidth;     // divideThisNode, tree.h:36
-    int cnt[8], nch = 0;
-    for (int c = 0; c < 8; c++) {
-        cnt[c] = b.oct[8 * (int64_t)node + c];
-        if (divide && cnt[c] >= kMinCell) nch++;
+    int cnt[8], cur[8], child_of[8], nch = 0;
+    {
+        const int4 *o = reinterpret_cast<const int4 *>(b.oct + 8 * (int64_t)node);
+        const int4 o0 = o[0], o1 = o[1];
+        cnt[0] = o0.x; cnt[1] = o0.y; cnt[2] = o0.z; cnt[3] = o0.w;
+        cnt[4] = o1.x; cnt[5] = o1.y; cnt[6] = o1.z; cnt[7] = o1.w;
     }
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+        if (divide && cnt[c] >= kMinCell) nch++;
     if (last && nch > 0) {
         atomicOr(b.counter + 1, 2);
         nch = 0;
@@ -372,30 +382,42 @@ __global__ void split_nodes(int L, int32_t ncap, int last, Build b) {
             first = -1;
         }
     }
-    int off = b.start[node];
+    const int start = b.start[node], halo = b.halo[node];
+    int off = start;
+#pragma unroll
     for (int c = 0; c < 8; c++) {
         const bool child = nch > 0 && divide && cnt[c] >= kMinCell;
+        child_of[c] = -1;
         if (!child) {
-            b.cur[8 * (int64_t)node + c] = off;
-            b.ochild[8 * (int64_t)node + c] = -1;
+            cur[c] = off;
             off += cnt[c];
         }
     }
-    b.lstart[node] = b.start[node];
-    b.lcount[node] = off - b.start[node];
+    b.lstart[node] = start;
+    b.lcount[node] = off - start;
     int k = 0;
+#pragma unroll
     for (int c = 0; c < 8; c++) {
         const bool child = nch > 0 && divide && cnt[c] >= kMinCell;
         if (child) {
             const int id = first + k++;
-            b.cur[8 * (int64_t)node + c] = off;
-            b.ochild[8 * (int64_t)node + c] = id;
+            cur[c] = off;
+            child_of[c] = id;
             b.start[id] = off;
             b.count[id] = cnt[c];
-            b.halo[id] = b.halo[node];
+            b.halo[id] = halo;
             b.par[id] = node;
+            zero_node(b, id);
             off += cnt[c];
         }
+    }
+    {
+        int4 *u = reinterpret_cast<int4 *>(b.cur + 8 * (int64_t)node);
+        int4 *v = reinterpret_cast<int4 *>(b.ochild + 8 * (int64_t)node);
+        u[0] = make_int4(cur[0], cur[1], cur[2], cur[3]);
+        u[1] = make_int4(cur[4], cur[5], cur[6], cur[7]);
+        v[0] = make_int4(child_of[0], child_of[1], child_of[2], child_of[3]);
+        v[1] = make_int4(child_of[4], child_of[5], child_of[6], child_of[7]);
     }
     b.first[node] = first;
     b.nchild[node] = nch;
@@ -511,7 +533,7 @@ __global__ void emit_nodes(int nlev, float theta2, Build b, KnnNode *__restrict_
     const int i = b.pre[node];
     KnnNode k;
     for (int a = 0; a < 3; a++) {
-        k.lo[a] = fkey_inv(b.box[6 * (int64_t)node + a]);
+        k.lo[a] = fkey_inv(~b.box[6 * (int64_t)node + a]);
         k.hi[a] = fkey_inv(b.box[6 * (int64_t)node + 3 + a]);
     }
     k.skip = i + b.sub[node];
@@ -633,7 +655,6 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
         GF_TRY(ctx->tree[1].reserve(nbytes + 256));
         char *np_ = ctx->tree[1].as<char>();
         Build b;
-        char *zero_begin = np_;
         b.start = carve<int32_t>(np_, nc);
         b.count = carve<int32_t>(np_, nc);
         b.halo = carve<int32_t>(np_, nc);
@@ -643,10 +664,8 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
         b.mz = carve<double>(np_, nc);
         b.r2 = carve<unsigned>(np_, nc);
         b.q = carve<float>(np_, nc * 6);
-        char *zero_end = np_;
         b.box = carve<unsigned>(np_, nc * 6);
         b.oct = carve<int32_t>(np_, nc * 8);
-        char *zero2_end = np_;
         b.cur = carve<int32_t>(np_, nc * 8);
         b.ochild = carve<int32_t>(np_, nc * 8);
         b.first = carve<int32_t>(np_, nc);
@@ -659,14 +678,6 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
         b.counter = carve<int32_t>(np_, 16);
         b.lev = carve<int32_t>(np_, kMaxLevels + 2);
         cudaStream_t s = ctx->stream;
-        GF_CUDA_TRY(cudaMemsetAsync(zero_begin, 0, zero_end - zero_begin, s));
-        // box: minima start at all-ones, maxima at zero (per node: 3 min then 3 max)
-        GF_CUDA_TRY(cudaMemsetAsync(b.box, 0, nc * 6 * 4, s));
-        GF_CUDA_TRY(cudaMemsetAsync(b.oct, 0, zero2_end - (char *)b.oct, s));
-        {
-            // min slots set to 0xff..: strided pattern, do it with a 2D memset
-            GF_CUDA_TRY(cudaMemset2DAsync(b.box, 6 * 4, 0xff, 3 * 4, nc, s));
-        }
         init_build<<<1, 32, 0, s>>>(nhalo, b);
         GF_LAUNCH_CHECK();
         if (nhalo > 0) {
