@@ -239,10 +239,11 @@ struct SmoothGroup {
     int64_t ntiles;
 };
 struct SmoothPlan {
-    // [axes | tables | on-chip halos | per group: halos, starts | zeroed-plane prefix]
+    // [axes | tables | table jobs | on-chip halos | per group: halos, starts | zeroed-plane prefix]
     std::vector<char> blob;
-    size_t off_tab = 0, off_chip = 0, off_zero = 0;
+    size_t off_tab = 0, off_jobs = 0, off_chip = 0, off_zero = 0;
     int32_t nchip = 0, nhalo = 0;
+    int32_t njobs = 0, job_max = 0;  // tables filled on the device, the longest of them
     bool box_ok = false;  // every group an FFT axis: the box-restricted passes apply
     std::vector<SmoothGroup> groups;
 };
@@ -252,6 +253,8 @@ int smooth_launch(gf_ctx *ctx, const SmoothPlan &plan, const char *dbuf, const g
 // Copies the plan's blob into ctx->smooth_tables (through pinned staging);
 // *dbuf receives its device address.
 int smooth_upload(gf_ctx *ctx, const SmoothPlan &plan, char **dbuf);
+// Fills the tables that the plan leaves to the device, once its blob is at dbuf.
+int smooth_fill_tables(gf_ctx *ctx, const SmoothPlan &plan, char *dbuf);
 // The box-restricted mesh stage, for meshes that only findDen reads (the
 // stage): launch_mesh_boxes fills the occupied boxes from the particles
 // before any deposit; smooth_box_prepare counts the passes' tiles from the

@@ -10,12 +10,12 @@
 //   * for power-of-two lengths runs a Stockham radix-2 FFT, multiplies the
 //     spectrum by G_n/n, and runs the inverse FFT, all in shared memory;
 //   * for any other length applies the full n-tap circular convolution with
-//     the exact h_n (computed in FP64 on the host), so arbitrary sizes such
-//     as the reference's extent/cellsize + 10 meshes are exact too.
+//     the exact h_n (computed in FP64), so arbitrary sizes such as the
+//     reference's extent/cellsize + 10 meshes are exact too.
 // Two real pencils are packed into one complex pencil (real and imaginary
 // parts): because G_n is real and even, filtering preserves that split.
 // Every pass reads and writes each mesh element once (8 B per element per
-// axis); twiddles and filters are generated in FP64 on the host.
+// axis); twiddles and filters are generated in FP64.
 #include <math.h>
 
 #include <algorithm>
@@ -215,6 +215,186 @@ smooth_axis_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mes
         else { s = e / (2 * npair); p = e - s * (2 * npair); }
         if (p < t.npen) den[elem_addr<AXIS>(m, mx, t, p, s)] = fs[2 * ((p >> 1) * n + s) + (p & 1)];
     }
+}
+
+// ------------------------------------------------------------- direct path
+// The full n-tap circular convolution for the lengths that are no power of
+// two (the reference's own meshes, extent/cellsize + 10), as
+// smooth_axis_kernel's direct branch with the same sums in the same order
+// (ascending taps, one fused multiply-add each, so the values are the same),
+// register blocked: a thread computes kOut = 8 consecutive outputs of a pencil
+// pair, and eight taps need only eight new elements for 64 packed complex
+// multiply-adds.  Each pair is held twice over (index i <-> element
+// (i - n8) mod n, n8 = n rounded up to 8), so no index wraps; taps past n are
+// zero.  Lanes run over the pairs, whose stride is an odd number of 16-byte
+// words: conflict-free 16-byte loads.
+// What bounds it: the FP32 pipe (n multiply-adds per cell and axis).  One
+// output per thread spent seven instructions per complex multiply-add; 48
+// stellar meshes of 36 to 160 cells per axis: three passes 551 -> 264 us.
+constexpr int kOut = 8;
+constexpr int kDirectThreads = 128;
+constexpr int kDirectMaxAxis = 2048;  // longer axes keep the one-output branch (shared memory)
+
+__host__ __device__ inline int direct_n8(int n) { return (n + kOut - 1) & ~(kOut - 1); }
+// float2 stride of a pencil pair: an odd number of 16-byte words
+__host__ __device__ inline int direct_stride(int n) { return 2 * direct_n8(n) + 2; }
+
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+template <int AXIS>
+__global__ void __launch_bounds__(kDirectThreads)
+smooth_direct_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh, GroupLaunch g,
+                     const AxisTable *__restrict__ axes, const float *__restrict__ tables, int pmax,
+                     const int32_t *__restrict__ boxes, int trim) {
+    extern __shared__ __align__(16) float2 smem[];
+    const SmoothTile t = decode_group_tile<AXIS>(blockIdx.x, g, mesh, pmax);
+    const gf_mesh_desc m = mesh[t.halo];
+    // the whole block leaves together (before any barrier)
+    if (boxes && !tile_needed<AXIS>(t, m, boxes + (int64_t)kMeshBoxInts * t.halo, trim)) return;
+    const AxisTable at = axes[3 * t.halo + AXIS];
+    const int n = at.n, n8 = direct_n8(n), stride = direct_stride(n);
+    const int64_t mx = 2 * (m.nx / 2 + 1);
+    // mx and every tile's first pencil are even: pairs of cells are 8-byte
+    // aligned when the mesh is
+    const bool pairs_ok = ((uintptr_t)(den + m.off) & 7) == 0;
+    const int npair = (t.npen + 1) >> 1;
+    float2 *hh = smem;           // the taps, each twice: (h, h)
+    float2 *xs = smem + n8;      // npair pencil pairs
+    float *xf = reinterpret_cast<float *>(xs);
+    const float *h = tables + at.tab_off;
+    for (int i = threadIdx.x; i < n8; i += kDirectThreads) {
+        const float v = i < n ? h[i] : 0.f;
+        hh[i] = make_float2(v, v);
+    }
+    // ---- load: pencil p -> component (p & 1) of pair p >> 1
+    const int total = 2 * npair * n;
+    for (int e = threadIdx.x; e < total; e += kDirectThreads) {
+        int p, s;
+        if (AXIS == 0) { p = e / n; s = e - p * n; }
+        else { s = e / (2 * npair); p = e - s * (2 * npair); }
+        float v = 0.f;
+        if (p < t.npen) v = den[elem_addr<AXIS>(m, mx, t, p, s)];
+        float *x = xf + 2 * (p >> 1) * stride + (p & 1);
+        // every i in [0, 2 n8) with (i - n8) mod n == s
+        for (int i = (s + n8) % n; i < 2 * n8; i += n) x[2 * i] = v;
+    }
+    __syncthreads();
+    const int chunks = n8 / kOut, items = npair * chunks;
+    for (int e0 = 0; e0 < items; e0 += kDirectThreads) {
+        const int e = e0 + threadIdx.x;
+        const int ch = e / npair, c = e - ch * npair;
+        f2 acc[kOut];
+#pragma unroll
+        for (int j = 0; j < kOut; j++) acc[j] = 0ull;
+        if (e < items) {
+            // x[k]: element s0 + 7 - m - k of the pair, k = 0..14
+            const float2 *base = xs + c * stride + n8 + ch * kOut;
+            f2 x[2 * kOut - 1];
+            {
+                const ulonglong2 *v = reinterpret_cast<const ulonglong2 *>(base);
+#pragma unroll
+                for (int i = 0; i < kOut / 2; i++) {  // elements s0 .. s0 + 7
+                    const ulonglong2 w = v[i];
+                    x[7 - 2 * i] = w.x;
+                    x[6 - 2 * i] = w.y;
+                }
+            }
+            for (int mm = 0; mm < n8; mm += kOut) {
+                const ulonglong2 *v = reinterpret_cast<const ulonglong2 *>(base - mm - kOut);
+                const ulonglong2 *hv = reinterpret_cast<const ulonglong2 *>(hh + mm);
+                f2 tap[kOut], below;
+#pragma unroll
+                for (int i = 0; i < kOut / 2; i++) {  // elements s0 - mm - 8 .. s0 - mm - 1
+                    const ulonglong2 w = v[i];
+                    const ulonglong2 u = hv[i];
+                    if (i == 0) below = w.x;
+                    else x[15 - 2 * i] = w.x;
+                    x[14 - 2 * i] = w.y;
+                    tap[2 * i] = u.x;
+                    tap[2 * i + 1] = u.y;
+                }
+#pragma unroll
+                for (int u = 0; u < kOut; u++) {
+#pragma unroll
+                    for (int j = 0; j < kOut; j++) acc[j] = f2_fma(tap[u], x[7 - j + u], acc[j]);
+                }
+                // the window moves down by eight elements
+#pragma unroll
+                for (int i = 0; i < kOut - 1; i++) x[i] = x[i + kOut];
+                x[kOut - 1] = below;
+            }
+        }
+        if (e >= items) continue;
+        if (AXIS == 0) {  // a row of eight cells per pencil
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                if (2 * c + q >= t.npen) break;
+                float *d = den + elem_addr<AXIS>(m, mx, t, 2 * c + q, ch * kOut);
+#pragma unroll
+                for (int j = 0; j < kOut; j += 2) {
+                    const float2 a0 = *reinterpret_cast<float2 *>(&acc[j]), a1 = *reinterpret_cast<float2 *>(&acc[j + 1]);
+                    const float2 v = q ? make_float2(a0.y, a1.y) : make_float2(a0.x, a1.x);
+                    if (pairs_ok && ch * kOut + j + 1 < n) {
+                        *reinterpret_cast<float2 *>(d + j) = v;
+                    } else {
+                        if (ch * kOut + j < n) d[j] = v.x;
+                        if (ch * kOut + j + 1 < n) d[j + 1] = v.y;
+                    }
+                }
+            }
+        } else {  // neighbouring pairs are neighbouring cells: 16 lanes store 128 bytes
+#pragma unroll
+            for (int j = 0; j < kOut; j++) {
+                if (ch * kOut + j >= n) break;
+                const float2 v = *reinterpret_cast<float2 *>(&acc[j]);
+                float *d = den + elem_addr<AXIS>(m, mx, t, 2 * c, ch * kOut + j);
+                if (pairs_ok && 2 * c + 1 < t.npen) {
+                    *reinterpret_cast<float2 *>(d) = v;
+                } else {
+                    d[0] = v.x;
+                    if (2 * c + 1 < t.npen) d[1] = v.y;
+                }
+            }
+        }
+    }
+}
+
+// The taps of the direct path: h_m = (1/n) sum_i G_i cos(2 pi (i m mod n) / n) in
+// FP64, rounded once; a block per 128 taps of a table.  On the host these
+// O(n^2) sums were most of a call on the reference's own meshes (48 meshes,
+// 144 tables: 0.8 of 1.41 ms; 5 us here).
+struct TableJob {
+    int32_t n, pad;
+    int64_t tab_off;  // float offset of the table
+    double rg_cells;
+};
+
+__device__ __host__ inline double axis_factor(int k, int n, double rg_cells);
+
+__global__ void __launch_bounds__(128) axis_taps_kernel(const TableJob *__restrict__ jobs, float *__restrict__ tables) {
+    __shared__ double g[kDirectMaxAxis], c[kDirectMaxAxis];
+    const TableJob job = jobs[blockIdx.x];
+    const int n = job.n;
+    if ((int)blockIdx.y * 128 >= n) return;
+    for (int i = threadIdx.x; i < n; i += 128) {
+        g[i] = axis_factor(i, n, job.rg_cells);
+        c[i] = cos(2.0 * M_PI * (double)i / (double)n);
+    }
+    __syncthreads();
+    const int mm = blockIdx.y * 128 + threadIdx.x;
+    if (mm >= n) return;
+    double acc = 0.0;
+    for (int i = 0, r = 0; i < n; i++) {
+        acc += g[i] * c[r];
+        r += mm;
+        if (r >= n) r -= n;
+    }
+    tables[job.tab_off + mm] = (float)(acc / n);
 }
 
 // ---------------------------------------------------------------- FFT path
@@ -909,7 +1089,7 @@ int ilog2_exact(int n) {
 
 // Spectral factor of one axis (gsmooth.c:67-86): G(k) = exp(k_s^2 expfac / n^2)
 // with k_s the signed frequency, expfac = -(pi RG/cellsize)^2.
-double axis_factor(int k, int n, double rg_cells) {
+__device__ __host__ inline double axis_factor(int k, int n, double rg_cells) {
     const double expfac = -(M_PI * rg_cells) * (M_PI * rg_cells);
     long ks = k;
     if (k > n / 2) ks = k - n;
@@ -934,6 +1114,18 @@ int64_t axis_table_floats(int n) {
     const PathKind pk = path_of(n);
     if (pk == PATH_DIRECT) return n;
     return 2 * (int64_t)(pk == PATH_FFT8 ? n : n / 2) + n;
+}
+
+// Whether smooth_direct_kernel serves an axis of n cells, and its pencils per
+// tile: a tile of at most 72 KB leaves three blocks per SM.
+bool direct_blocked(int n) { return path_of(n) == PATH_DIRECT && n <= kDirectMaxAxis; }
+size_t direct_smem(int n, int pmax) {
+    return ((size_t)direct_n8(n) + (size_t)((pmax + 1) / 2) * direct_stride(n)) * sizeof(float2);
+}
+int direct_tile_pencils(int n) {
+    int pmax = 32;
+    while (pmax > 2 && direct_smem(n, pmax) > 72 * 1024) pmax -= 2;
+    return pmax;
 }
 
 // Writes the table of one axis into out[0 .. axis_table_floats(n)).  The
@@ -966,7 +1158,7 @@ void write_axis_tables(int n, double rg_cells, float *out, double *g, double *c)
     }
 }
 
-void append_tables(std::vector<float> &tab, int n, double rg_cells, AxisTable &at) {
+void append_tables(std::vector<float> &tab, int n, double rg_cells, AxisTable &at, std::vector<TableJob> &jobs) {
     // every table starts on a 16-byte boundary: the FFT paths read float2
     // twiddles, and a preceding table may hold an odd number of floats
     while (tab.size() % 4) tab.push_back(0.f);
@@ -975,6 +1167,10 @@ void append_tables(std::vector<float> &tab, int n, double rg_cells, AxisTable &a
     at.tab_off = (int64_t)tab.size();
     const size_t base = tab.size();
     tab.resize(base + (size_t)axis_table_floats(n));
+    if (direct_blocked(n)) {  // filled on the device (smooth_fill_tables)
+        jobs.push_back(TableJob{n, 0, at.tab_off, rg_cells});
+        return;
+    }
     std::vector<double> work(path_of(n) == PATH_DIRECT ? 2 * (size_t)n : 0);
     write_axis_tables(n, rg_cells, tab.data() + base, work.data(), work.data() + (work.empty() ? 0 : n));
 }
@@ -1016,6 +1212,15 @@ int launch_group(gf_ctx *ctx, float *den, const gf_mesh_desc *mesh_dev, GroupLau
         case 9: return launch_fft<AXIS, 9>(ctx, den, mesh_dev, g, ntiles, axes, tables, boxes, trim);
         default: break;
     }
+    if (direct_blocked(n)) {
+        const size_t bytes = direct_smem(n, pmax);
+        GF_CUDA_TRY(cudaFuncSetAttribute(smooth_direct_kernel<AXIS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)bytes));
+        smooth_direct_kernel<AXIS><<<(unsigned)ntiles, kDirectThreads, bytes, ctx->stream>>>(den, mesh_dev, g, axes,
+                                                                                            tables, pmax, boxes, trim);
+        GF_LAUNCH_CHECK();
+        return GF_OK;
+    }
     const size_t smem = (size_t)2 * ((pmax + 1) / 2) * n * sizeof(float2);
     GF_CUDA_TRY(cudaFuncSetAttribute(smooth_axis_kernel<AXIS>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1033,6 +1238,7 @@ int smooth_plan(int32_t nhalo, const gf_mesh_desc *mesh_host, const OnChipMeshes
     const int32_t non_chip = onchip ? onchip->nmesh : 0;  // meshes on chip
     std::vector<AxisTable> axes(3 * (size_t)nhalo);
     std::vector<float> tables;
+    std::vector<TableJob> jobs;
     std::map<std::pair<int, double>, AxisTable> cache;
     for (int h = 0; h < nhalo; h++) {
         const gf_mesh_desc &m = mesh_host[h];
@@ -1048,13 +1254,14 @@ int smooth_plan(int32_t nhalo, const gf_mesh_desc *mesh_host, const OnChipMeshes
             auto it = cache.find(key);
             if (it == cache.end()) {
                 AxisTable at;
-                append_tables(tables, dims[a], rg_cells, at);
+                append_tables(tables, dims[a], rg_cells, at, jobs);
                 it = cache.emplace(key, at).first;
             }
             axes[3 * (size_t)h + a] = it->second;
         }
     }
-    // groups: (axis, n) for the FFT path; one group per axis for the rest
+    // groups: (axis, n) for the FFT path; per axis, one group for the blocked
+    // direct path and one for the rest
     struct Group {
         int axis, n, pmax;
         std::vector<int32_t> halos;
@@ -1068,7 +1275,7 @@ int smooth_plan(int32_t nhalo, const gf_mesh_desc *mesh_host, const OnChipMeshes
             if (m.ptype == kMeshOnChip) continue;  // smoothed on chip
             const int dims[3] = {m.nx, m.ny, m.nz};
             const int n = dims[a];
-            const int key_n = path_of(n) == PATH_FFT8 ? n : -1;
+            const int key_n = path_of(n) == PATH_FFT8 ? n : direct_blocked(n) ? -2 : -1;
             auto k = std::make_pair(a, key_n);
             auto it = gidx.find(k);
             if (it == gidx.end()) {
@@ -1083,6 +1290,8 @@ int smooth_plan(int32_t nhalo, const gf_mesh_desc *mesh_host, const OnChipMeshes
     for (Group &g : groups) {
         if (path_of(g.n) == PATH_FFT8 && g.n == (1 << ilog2_exact(g.n))) {
             g.pmax = fft_tile_pencils(g.n);
+        } else if (direct_blocked(g.n)) {
+            g.pmax = direct_tile_pencils(g.n);
         } else {
             int pmax = 32;
             while (pmax > 2 && (size_t)2 * (pmax / 2) * g.n * sizeof(float2) > 200 * 1024) pmax -= 2;
@@ -1110,6 +1319,10 @@ int smooth_plan(int32_t nhalo, const gf_mesh_desc *mesh_host, const OnChipMeshes
     size_t off = align(axes.size() * sizeof(AxisTable));
     plan->off_tab = off;
     off = align(off + tables.size() * sizeof(float));
+    plan->off_jobs = off;
+    plan->njobs = (int32_t)jobs.size();
+    for (const TableJob &j : jobs) plan->job_max = std::max(plan->job_max, j.n);
+    off = align(off + jobs.size() * sizeof(TableJob));
     plan->off_chip = off;
     plan->nchip = non_chip;
     off = align(off + (size_t)non_chip * sizeof(int32_t));
@@ -1126,6 +1339,7 @@ int smooth_plan(int32_t nhalo, const gf_mesh_desc *mesh_host, const OnChipMeshes
     char *hbuf = plan->blob.data();
     memcpy(hbuf, axes.data(), axes.size() * sizeof(AxisTable));
     memcpy(hbuf + plan->off_tab, tables.data(), tables.size() * sizeof(float));
+    memcpy(hbuf + plan->off_jobs, jobs.data(), jobs.size() * sizeof(TableJob));
     if (non_chip) memcpy(hbuf + plan->off_chip, onchip->halos_host, (size_t)non_chip * sizeof(int32_t));
     for (size_t i = 0; i < groups.size(); i++) {
         memcpy(hbuf + off_h[i], groups[i].halos.data(), groups[i].halos.size() * sizeof(int32_t));
@@ -1192,6 +1406,14 @@ int smooth_upload(gf_ctx *ctx, const SmoothPlan &plan, char **dbuf) {
     memcpy(ctx->pin[3].ptr, plan.blob.data(), total);
     *dbuf = ctx->smooth_tables.as<char>();
     GF_CUDA_TRY(cudaMemcpyAsync(*dbuf, ctx->pin[3].ptr, total, cudaMemcpyHostToDevice, ctx->stream));
+    return smooth_fill_tables(ctx, plan, *dbuf);
+}
+
+int smooth_fill_tables(gf_ctx *ctx, const SmoothPlan &plan, char *dbuf) {
+    if (plan.njobs == 0) return GF_OK;
+    axis_taps_kernel<<<dim3((unsigned)plan.njobs, (unsigned)((plan.job_max + 127) / 128)), 128, 0, ctx->stream>>>(
+        reinterpret_cast<const TableJob *>(dbuf + plan.off_jobs), reinterpret_cast<float *>(dbuf + plan.off_tab));
+    GF_LAUNCH_CHECK();
     return GF_OK;
 }
 
@@ -1358,7 +1580,9 @@ int smooth_single_build(const gf_mesh_desc &m, unsigned char *blob, size_t cap, 
         // tiles as smooth_meshes cuts them: the FFT kernel's tile width on the
         // FFT path, else as many as fit in shared memory
         int pmax = fft_tile_pencils(n);
-        if (path_of(n) != PATH_FFT8) {
+        if (direct_blocked(n)) {
+            pmax = direct_tile_pencils(n);
+        } else if (path_of(n) != PATH_FFT8) {
             pmax = 32;
             while (pmax > 2 && (size_t)2 * (pmax / 2) * n * sizeof(float2) > 200 * 1024) pmax -= 2;
         }

@@ -547,6 +547,7 @@ int capture_graph(StageGraph &g) {
         if (!g.smooth.blob.empty())
             GF_CUDA_TRY(cudaMemcpy(g.smooth_blob.ptr, g.smooth.blob.data(), g.smooth.blob.size(),
                                    cudaMemcpyHostToDevice));
+        GF_TRY(smooth_fill_tables(ctx, g.smooth, g.smooth_blob.as<char>()));
     }
     GF_TRY(stage_pass_graph(g));
     GF_TRY(check_device_errors(ctx));
