@@ -84,20 +84,8 @@ __global__ void tsc_deposit_kernel(int64_t n, const double *__restrict__ x,
                     c[4] = (int)s.k[0] - 1; c[5] = (int)s.k[0] + 1;
                     if (dep) {
                         tsc_deposit_weights(s, xd1, yd1, zd1, mass[p]);
-                        const int64_t mx = 2 * (m.nx / 2 + 1);
-                        float *mesh_h = den + m.off;
-#pragma unroll
-                        for (int cc = 0; cc < 3; cc++) {
-#pragma unroll
-                            for (int b = 0; b < 3; b++) {
-#pragma unroll
-                                for (int a = 0; a < 3; a++) {
-                                    // volfold is 1 or an exact power of two (see launch_tsc_deposit)
-                                    atomicAdd(mesh_h + s.i[a] + mx * (s.j[b] + (int64_t)m.ny * s.k[cc]),
-                                              tsc_deposit_value(s, a, b, cc, volfold));
-                                }
-                            }
-                        }
+                        // volfold is 1 or an exact power of two (see launch_tsc_deposit)
+                        tsc_deposit_global(den + m.off, s, m, volfold, mesh_wide(den + m.off));
                     }
                 }
             }
@@ -266,21 +254,20 @@ tsc_tile_deposit_kernel(int64_t n, const double *__restrict__ x, const double *_
                     tsc_cells(x[p], y[p], z[p], m, s, xd1, yd1, zd1);
                     if (!tsc_in_mesh(s, m)) continue;
                     tsc_deposit_weights(s, xd1, yd1, zd1, mass[p]);
+                    // volfold is 1 or an exact power of two (see launch_tsc_deposit)
+                    if (!use_tile) {
+                        tsc_deposit_global(mesh_h, s, m, volfold, mesh_wide(mesh_h));
+                        continue;
+                    }
 #pragma unroll
                     for (int cc = 0; cc < 3; cc++) {
 #pragma unroll
                         for (int b = 0; b < 3; b++) {
 #pragma unroll
-                            for (int a = 0; a < 3; a++) {
-                                // volfold is 1 or an exact power of two (see launch_tsc_deposit)
-                                const float v = tsc_deposit_value(s, a, b, cc, volfold);
-                                if (use_tile)
-                                    atomicAdd(tile + ((int)s.i[a] - bb.v[0]) +
-                                                  wx * (((int)s.j[b] - bb.v[2]) + wy * ((int)s.k[cc] - bb.v[4])),
-                                              v);
-                                else
-                                    atomicAdd(mesh_h + s.i[a] + mx * (s.j[b] + (int64_t)m.ny * s.k[cc]), v);
-                            }
+                            for (int a = 0; a < 3; a++)
+                                atomicAdd(tile + ((int)s.i[a] - bb.v[0]) +
+                                              wx * (((int)s.j[b] - bb.v[2]) + wy * ((int)s.k[cc] - bb.v[4])),
+                                          tsc_deposit_value(s, a, b, cc, volfold));
                         }
                     }
                 }
