@@ -428,6 +428,36 @@ __device__ __forceinline__ void dft(float2 (&a)[R]) {
         a[1] = csub(t, a[1]);
     } else if (R == 4) {
         dft4<INV>(a[0], a[1], a[2], a[3]);
+    } else if (R == 16) {  // 4 x 4: columns, W16 twiddles, rows
+        // cos and sin of pi/8, and of pi/4
+        const float c1 = 0.92387953251128676f, s1 = 0.38268343236508977f, h = 0.70710678118654752f;
+        auto tw = [](float2 v, float c, float s) {  // v * (c - i s), conjugated for the inverse
+            return INV ? make_float2(v.x * c - v.y * s, v.y * c + v.x * s)
+                       : make_float2(v.x * c + v.y * s, v.y * c - v.x * s);
+        };
+#pragma unroll
+        for (int i = 0; i < 4; i++) dft4<INV>(a[i], a[4 + i], a[8 + i], a[12 + i]);
+        a[5] = tw(a[5], c1, s1);     // W16^1
+        a[9] = tw(a[9], h, h);       // W16^2
+        a[13] = tw(a[13], s1, c1);   // W16^3
+        a[6] = tw(a[6], h, h);       // W16^2
+        a[10] = mul_mi<INV>(a[10]);  // W16^4
+        a[14] = tw(a[14], -h, h);    // W16^6
+        a[7] = tw(a[7], s1, c1);     // W16^3
+        a[11] = tw(a[11], -h, h);    // W16^6
+        a[15] = tw(a[15], -c1, -s1); // W16^9
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) dft4<INV>(a[i], a[i + 1], a[i + 2], a[i + 3]);
+        // entry 4 k + j holds output k + 4 j
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+#pragma unroll
+            for (int j = k + 1; j < 4; j++) {
+                const float2 t = a[4 * k + j];
+                a[4 * k + j] = a[4 * j + k];
+                a[4 * j + k] = t;
+            }
+        }
     } else {  // R == 8: two 4-point DFTs (even, odd) and the W8 butterflies
         float2 e0 = a[0], e1 = a[2], e2 = a[4], e3 = a[6];
         float2 o0 = a[1], o1 = a[3], o2 = a[5], o3 = a[7];
@@ -741,17 +771,150 @@ int launch_onchip(gf_ctx *ctx, const OnChipArgs &a) {
 
 constexpr int kPencils = GF_FFT_PENCILS;  // real pencils per FFT tile (2 per complex pencil)
 
-// Real pencils per tile of an FFT axis of 2^LOGN cells: wider tiles for the
-// short axes, whose tiles are otherwise small (8 KB at 64 cells).
+// Axes of 512 cells: Stockham passes over a tile of P real pencils.
 template <int LOGN>
 struct FftTile {
-    static constexpr int P = LOGN == 6 ? GF_FFT_PENCILS_64 : LOGN == 7 ? GF_FFT_PENCILS_128 : kPencils;
+    static constexpr int P = kPencils;
     static constexpr int NT = (P / 2) * (1 << LOGN) / 8;  // threads per tile
 };
-static_assert(FftTile<9>::NT <= 1024 && FftTile<6>::NT <= 1024 && FftTile<7>::NT <= 1024, "FFT tile threads");
+static_assert(FftTile<9>::NT <= 1024, "FFT tile threads");
+
+// ---- axes of 64, 128 and 256 cells: the transform of a pencil pair in two
+// register passes, N = R1 x R2 (8 x 8, 16 x 8, 16 x 16), T = R2 threads per pair.
+// A thread loads the R1 elements n0 + r T of its pair from the mesh straight
+// into registers, transforms them, applies w^(n0 j) and leaves output j at
+// place j T + n0 of the shared tile; block j (R2 consecutive places) is then a
+// transform of its own, whose outputs are the frequencies j + R1 k: one thread
+// reads it, multiplies by the filter and transforms it back in place; the
+// mirrored first pass ends in registers again and stores to the mesh.  Two
+// exchanges through shared memory and three barriers per tile, where separate
+// load, Stockham passes and store took five (64) or seven.
+// Rows (x) keep a pair's threads in one warp, so they need no block barrier;
+// columns (y, z) have neighbouring pairs in neighbouring lanes, for the
+// mesh accesses and for conflict-free rows of the tile.
+// What bounds it: the latency of the mesh loads (16 to 32 in flight per thread;
+// whole 256^3 passes move 134 MB in 38 us, 54 % of the measured copy rate).
+// Stockham tiles -> register passes: the box passes of 4096 halos 4.93 -> 2.50
+// ms (64 cells 1.59 -> 0.87, 128 1.30 -> 0.62, 256 2.02 -> 1.02), nine whole
+// passes of a 256^3 mesh 661 -> 350 us.  Resident threads per SM (registers
+// against warps), 512 / 768 / 1024: box passes of 64 cells 942 / 921 / 866 us,
+// of 128 625 / 670 / 730, of 256 1022 / 1062 / 1106; whole passes 374 / 350 / 386.
+template <int LOGN>
+struct RegFft {
+    static constexpr int N = 1 << LOGN;
+    static constexpr int R1 = LOGN == 6 ? 8 : 16;
+    static constexpr int R2 = N / R1;
+    static constexpr int T = R2;       // threads per pair
+    static constexpr int B = R1 / T;   // blocks per thread in the second pass
+    static constexpr int P = LOGN == 6 ? GF_FFT_PENCILS_64 : LOGN == 7 ? GF_FFT_PENCILS_128 : 32;  // real pencils per tile
+    static constexpr int PAIRS = P / 2;
+    static constexpr int NT = PAIRS * T;
+    // float2 stride of a pair of rows: a padding slot per block, and pairs of
+    // one half-warp in different banks
+    static constexpr int SN = N + R1 + (LOGN == 7 ? 8 : 0);
+    static_assert(LOGN >= 6 && LOGN <= 8 && NT <= 1024, "register FFT lengths 64..256");
+    template <int AXIS>
+    static constexpr size_t smem() { return (size_t)(AXIS == 0 ? PAIRS * SN : N * PAIRS) * sizeof(float2); }
+    template <int AXIS>
+    __device__ static __forceinline__ int at(int c, int pos) {
+        return AXIS == 0 ? c * SN + pos + pos / R2 : pos * PAIRS + c;
+    }
+};
+
+template <int AXIS>
+__device__ __forceinline__ void tile_sync() {
+    if (AXIS == 0) __syncwarp(); else __syncthreads();
+}
+
+// Pair c of a tile (on: it holds a pencil), thread n0 of T: load(s) gives both
+// pencils' element s, store(s, v) takes the filtered one.
+template <int AXIS, int LOGN, class Load, class Store>
+__device__ __forceinline__ void reg_fft_pair(float2 *sm, int c, int n0, bool on, const float2 *__restrict__ tw,
+                                             const float *__restrict__ filt, Load load, Store store) {
+    using F = RegFft<LOGN>;
+    float2 a[F::R1];
+    if (on) {
+#pragma unroll
+        for (int r = 0; r < F::R1; r++) a[r] = load(n0 + r * F::T);
+        dft<F::R1, false>(a);
+#pragma unroll
+        for (int j = 1; j < F::R1; j++) a[j] = cmul(a[j], __ldg(tw + n0 * j));
+#pragma unroll
+        for (int j = 0; j < F::R1; j++) sm[F::template at<AXIS>(c, j * F::T + n0)] = a[j];
+    }
+    tile_sync<AXIS>();
+    if (on) {
+#pragma unroll
+        for (int b = 0; b < F::B; b++) {
+            const int u = n0 + b * F::T;
+            float2 d[F::R2];
+#pragma unroll
+            for (int i = 0; i < F::R2; i++) d[i] = sm[F::template at<AXIS>(c, u * F::R2 + i)];
+            dft<F::R2, false>(d);
+#pragma unroll
+            for (int i = 0; i < F::R2; i++) {
+                const float g = __ldg(filt + u + F::R1 * i);
+                d[i].x *= g;
+                d[i].y *= g;
+            }
+            dft<F::R2, true>(d);
+#pragma unroll
+            for (int i = 0; i < F::R2; i++) sm[F::template at<AXIS>(c, u * F::R2 + i)] = d[i];
+        }
+    }
+    tile_sync<AXIS>();
+    if (on) {
+#pragma unroll
+        for (int j = 0; j < F::R1; j++) a[j] = sm[F::template at<AXIS>(c, j * F::T + n0)];
+#pragma unroll
+        for (int j = 1; j < F::R1; j++) {
+            float2 w = __ldg(tw + n0 * j);
+            w.y = -w.y;
+            a[j] = cmul(a[j], w);
+        }
+        dft<F::R1, true>(a);
+#pragma unroll
+        for (int r = 0; r < F::R1; r++) store(n0 + r * F::T, a[r]);
+    }
+}
+
+template <int AXIS, int LOGN>
+__global__ void __launch_bounds__(RegFft<LOGN>::NT, 768 / RegFft<LOGN>::NT)
+smooth_reg_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh, GroupLaunch g,
+                  const AxisTable *__restrict__ axes, const float *__restrict__ tables,
+                  const int32_t *__restrict__ boxes, int trim) {
+    using F = RegFft<LOGN>;
+    extern __shared__ float2 smem[];
+    const SmoothTile t = decode_group_tile<AXIS>(blockIdx.x, g, mesh, F::P);
+    const gf_mesh_desc m = mesh[t.halo];
+    // the whole block leaves together (before any barrier)
+    if (boxes && !tile_needed<AXIS>(t, m, boxes + (int64_t)kMeshBoxInts * t.halo, trim)) return;
+    const AxisTable at = axes[3 * t.halo + AXIS];
+    const int64_t mx = 2 * (m.nx / 2 + 1);
+    const int c = AXIS == 0 ? threadIdx.x / F::T : threadIdx.x % F::PAIRS;
+    const int n0 = AXIS == 0 ? threadIdx.x % F::T : threadIdx.x / F::PAIRS;
+    const int half = (t.npen + 1) >> 1;  // pair c: pencils c and c + half
+    const bool two = c + half < t.npen;
+    // element (pencil p, position s) lives at base + p*pstride + s*sstride;
+    // within one tile the offsets fit in 32 bits (axes <= 512, mx*ny < 2^21)
+    int64_t base;
+    int pstride, sstride;
+    if (AXIS == 0) { base = m.off + mx * t.base; pstride = (int)mx; sstride = 1; }
+    else if (AXIS == 1) { base = m.off + t.base + mx * (int64_t)m.ny * t.other; pstride = 1; sstride = (int)mx; }
+    else { base = m.off + t.base + mx * (int64_t)t.other; pstride = 1; sstride = (int)(mx * m.ny); }
+    float *p0 = den + base + c * pstride, *p1 = p0 + half * pstride;
+    const float2 *tw = reinterpret_cast<const float2 *>(tables + at.tab_off);
+    reg_fft_pair<AXIS, LOGN>(
+        smem, c, n0, c < half, tw, tables + at.tab_off + 2 * F::N,
+        [&](int s) { return make_float2(p0[s * sstride], two ? p1[s * sstride] : 0.f); },
+        [&](int s, float2 v) {
+            p0[s * sstride] = v.x;
+            if (two) p1[s * sstride] = v.y;
+        });
+}
 
 int fft_tile_pencils(int n) {
-    return n == 64 ? FftTile<6>::P : n == 128 ? FftTile<7>::P : kPencils;
+    return n == 64 ? RegFft<6>::P : n == 128 ? RegFft<7>::P : n == 256 ? RegFft<8>::P : kPencils;
 }
 
 template <int AXIS, int LOGN>
@@ -1080,6 +1243,52 @@ smooth_box_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh
     }
 }
 
+// The same passes of the axes that the register transform serves.
+template <int AXIS, int LOGN>
+__global__ void __launch_bounds__(RegFft<LOGN>::NT, (LOGN == 6 ? 1024 : 512) / RegFft<LOGN>::NT)
+smooth_reg_box_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh, GroupLaunch g,
+                      const AxisTable *__restrict__ axes, const float *__restrict__ tables,
+                      const int32_t *__restrict__ boxes) {
+    using F = RegFft<LOGN>;
+    extern __shared__ float2 smem[];
+    const int c = AXIS == 0 ? threadIdx.x / F::T : threadIdx.x % F::PAIRS;
+    const int n0 = AXIS == 0 ? threadIdx.x % F::T : threadIdx.x / F::PAIRS;
+    int64_t t0, t1;
+    block_share(g.tile_start[g.ngroup], t0, t1);
+    int gi = -1;
+    for (int64_t tb = t0; tb < t1; tb++) {
+        gi = (gi < 0 || __ldg(g.tile_start + gi + 1) <= tb) ? prefix_find(g.tile_start, max(gi, 0), g.ngroup, tb)
+                                                           : gi;
+        const int h = g.halos[gi];
+        const gf_mesh_desc m = mesh[h];
+        const BoxGeom q = box_geom<AXIS>(m, boxes + (int64_t)kMeshBoxInts * h);
+        const int64_t f0 = (tb - g.tile_start[gi]) * F::P;
+        const int npen = (int)min((int64_t)F::P, (int64_t)q.nu * q.nv - f0);
+        const int half = (npen + 1) >> 1;  // pair c: pencils f0 + c and f0 + c + half
+        const bool two = c + half < npen;
+        auto pencil = [&](int64_t f) {
+            const int v = (int)((unsigned)f / (unsigned)q.nu), u = (int)f - v * q.nu;  // nu nv < 2^31
+            return den + m.off + (int64_t)((q.u0 + u) * q.ustride + (q.v0 + v) * q.vstride);
+        };
+        float *p0 = pencil(f0 + (c < half ? c : 0));
+        float *p1 = pencil(f0 + (two ? c + half : 0));
+        const AxisTable at = axes[3 * h + AXIS];
+        const float2 *tw = reinterpret_cast<const float2 *>(tables + at.tab_off);
+        reg_fft_pair<AXIS, LOGN>(
+            smem, c, n0, c < half, tw, tables + at.tab_off + 2 * F::N,
+            [&](int s) {
+                const bool in = s >= q.l0 && s <= q.l1;
+                return make_float2(in ? p0[s * q.sstride] : 0.f, in && two ? p1[s * q.sstride] : 0.f);
+            },
+            [&](int s, float2 v) {
+                if (s < q.s0 || s > q.s1) return;
+                p0[s * q.sstride] = v.x;
+                if (two) p1[s * q.sstride] = v.y;
+            });
+        tile_sync<AXIS>();  // the tile is reused by the next one
+    }
+}
+
 int ilog2_exact(int n) {
     if (n <= 0 || (n & (n - 1))) return -1;
     int l = 0;
@@ -1178,13 +1387,21 @@ void append_tables(std::vector<float> &tab, int n, double rg_cells, AxisTable &a
 template <int AXIS, int LOGN>
 int launch_fft(gf_ctx *ctx, float *den, const gf_mesh_desc *mesh_dev, GroupLaunch g, int64_t ntiles,
                const AxisTable *axes, const float *tables, const int32_t *boxes, int trim) {
-    constexpr int N = 1 << LOGN;
-    const int threads = FftTile<LOGN>::NT;
-    const size_t smem = (size_t)2 * (FftTile<LOGN>::P / 2) * FftLayout<N>::SN * sizeof(float2);
-    GF_CUDA_TRY(cudaFuncSetAttribute(smooth_fft_kernel<AXIS, LOGN>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    smooth_fft_kernel<AXIS, LOGN><<<(unsigned)ntiles, threads, smem, ctx->stream>>>(den, mesh_dev, g,
-                                                                                   axes, tables, boxes, trim);
+    if constexpr (LOGN <= 8) {
+        using F = RegFft<LOGN>;
+        auto kern = smooth_reg_kernel<AXIS, LOGN>;
+        const size_t smem = F::template smem<AXIS>();
+        GF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kern<<<(unsigned)ntiles, F::NT, smem, ctx->stream>>>(den, mesh_dev, g, axes, tables, boxes, trim);
+    } else {
+        constexpr int N = 1 << LOGN;
+        const int threads = FftTile<LOGN>::NT;
+        const size_t smem = (size_t)2 * (FftTile<LOGN>::P / 2) * FftLayout<N>::SN * sizeof(float2);
+        GF_CUDA_TRY(cudaFuncSetAttribute(smooth_fft_kernel<AXIS, LOGN>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        smooth_fft_kernel<AXIS, LOGN><<<(unsigned)ntiles, threads, smem, ctx->stream>>>(den, mesh_dev, g,
+                                                                                       axes, tables, boxes, trim);
+    }
     GF_LAUNCH_CHECK();
     return GF_OK;
 }
@@ -1433,10 +1650,18 @@ namespace {
 template <int AXIS, int LOGN>
 int launch_box_fft(gf_ctx *ctx, float *den, const gf_mesh_desc *mesh_dev, GroupLaunch g, int64_t max_tiles,
                    const AxisTable *axes, const float *tables, const int32_t *boxes) {
-    constexpr int N = 1 << LOGN;
-    const int threads = FftTile<LOGN>::NT;
-    const size_t smem = (size_t)2 * (FftTile<LOGN>::P / 2) * FftLayout<N>::SN * sizeof(float2);
-    auto kern = smooth_box_kernel<AXIS, LOGN>;
+    void (*kern)(float *, const gf_mesh_desc *, GroupLaunch, const AxisTable *, const float *, const int32_t *);
+    int threads;
+    size_t smem;
+    if constexpr (LOGN <= 8) {
+        kern = smooth_reg_box_kernel<AXIS, LOGN>;
+        threads = RegFft<LOGN>::NT;
+        smem = RegFft<LOGN>::template smem<AXIS>();
+    } else {
+        kern = smooth_box_kernel<AXIS, LOGN>;
+        threads = FftTile<LOGN>::NT;
+        smem = (size_t)2 * (FftTile<LOGN>::P / 2) * FftLayout<(1 << LOGN)>::SN * sizeof(float2);
+    }
     GF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     GF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
