@@ -8,13 +8,16 @@
 //     exceeds 0.5e-6 (MINCELLWIDTH/2); smaller octants stay as loose
 //     particles of the node;
 //   * monopole, second moments and dist2 = max |x - com|^2 are per node.
-// Each level processes every still-active particle at once (all halos, all
-// nodes of the level): accumulate mass and first moments, finalise the COM,
-// accumulate extents/second moments/octant counts, allocate children, and
-// scatter the particles into [loose | child 0 | child 1 | ...] order.  After
-// the last level the nodes are renumbered in depth-first preorder so the walks
-// are stackless: opening node i continues at i + 1, skipping it continues at
-// skip[i].
+// Nodes of more than kSmall particles are built level by level, every active
+// particle of all halos at once: accumulate mass and first moments, finalise
+// the COM, accumulate extents/second moments/octant counts, allocate children,
+// and scatter the particles into [loose | child 0 | child 1 | ...] order.  A
+// node of at most kSmall particles is left to one warp, which builds its whole
+// subtree in shared memory (small_subtrees).  The nodes are then numbered in
+// depth-first preorder so the walks are stackless: opening node i continues at
+// i + 1, skipping it continues at skip[i].  A node's preorder number is the
+// number of nodes that start before its first particle (a scan over the
+// particles of the nodes starting at each), plus the ancestors starting with it.
 #include <math.h>
 
 #include <algorithm>
@@ -53,11 +56,25 @@ struct Build {
     int32_t *cur;                   // 8 octant cursors
     int32_t *ochild;                // 8 child ids or -1
     int32_t *first, *nchild, *lstart, *lcount;
-    int32_t *sub, *pre;             // subtree size, preorder index
-    int32_t *par;                   // BFS id of the parent, -1 for roots
-    int32_t *counter;               // [0] nodes allocated, [1] overflow flag, [2] blocks done
-    int32_t *lev;                   // level L holds BFS nodes [lev[L], lev[L+1])
+    int32_t *par;                   // id of the parent, -1 for roots
+    int32_t *small;                 // nodes left to small_subtrees (their level stands in first until then)
+    int32_t *counter;               // [0] nodes allocated, [1] overflow flags, [2] blocks done, [3] small nodes,
+                                    // [4] depth of the trees (small_subtrees)
+    int32_t *lev;                   // level L holds the nodes [lev[L], lev[L+1]) (while the levels run)
+    int32_t *nact;                  // nodes of level L that the level passes process
 };
+
+// A node of at most kSmall particles is built with its subtree by one warp.  The
+// level passes cost five launches a level (and, eagerly, a host wait) however
+// few particles are left, and read every one of those from memory, so the
+// lower levels, most of a small batch's, go to shared memory: the stage on a
+// halo of 120 took 0.32 ms, now 0.24; on one of 131,072 1.59, now 1.40; a
+// replayed graph of 64 halos 0.70, now 0.59; four gradients of one million
+// particles, whose tree was their largest part, 1.35, now 1.16.  256 particles
+// (two buffers, 10 KB) leave 20 warps per SM; the pass is bound by the chain
+// of shuffles of a node (log2 32 steps for 17 values), 0.42 ms for 6 M
+// particles.
+constexpr int kSmall = 256;
 
 __device__ __forceinline__ void zero_node(const Build &b, int node) {
     b.m[node] = b.mx[node] = b.my[node] = b.mz[node] = 0.0;
@@ -80,29 +97,35 @@ constexpr int kMaxLevels = 4096;
     for (int node = (b).lev[L] + blockIdx.x * blockDim.x + threadIdx.x; node < (b).lev[(L) + 1]; \
          node += gridDim.x * blockDim.x)
 
-__global__ void init_build(int32_t nhalo, Build b) {
-    if (threadIdx.x == 0) {
-        b.counter[0] = nhalo;  // the roots are nodes 0 .. nhalo-1
-        b.counter[1] = 0;
-        b.counter[2] = 0;
+// The roots are nodes 0 .. nhalo-1 (counter and nact start zeroed).
+__global__ void init_roots(int32_t nhalo, const int64_t *__restrict__ pstart, Build b) {
+    int h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h == 0) {
+        b.counter[0] = nhalo;
         b.lev[0] = 0;
         b.lev[1] = nhalo;
     }
-}
-
-__global__ void init_roots(int32_t nhalo, const int64_t *__restrict__ pstart, Build b) {
-    int h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= nhalo) return;
+    const int c = (int32_t)(pstart[h + 1] - pstart[h]);
     b.start[h] = (int32_t)pstart[h];
-    b.count[h] = (int32_t)(pstart[h + 1] - pstart[h]);
+    b.count[h] = c;
     b.halo[h] = h;
     b.par[h] = -1;
-    zero_node(b, h);
+    if (c > kSmall) {
+        zero_node(b, h);
+        atomicAdd(b.nact, 1);
+    } else {
+        b.first[h] = 0;
+        b.small[atomicAdd(b.counter + 3, 1)] = h;
+    }
 }
 
+// Particles of small halos go straight to the final arrays, where
+// small_subtrees orders them.
 __global__ void init_particles(int64_t n, const int64_t *__restrict__ pstart, int32_t nhalo,
                                const float4 *__restrict__ pos_in, float4 *__restrict__ pos,
-                               int32_t *__restrict__ perm, int32_t *__restrict__ pnode) {
+                               int32_t *__restrict__ perm, int32_t *__restrict__ pnode, float4 *__restrict__ fpos,
+                               int32_t *__restrict__ fperm, int32_t *__restrict__ phalo) {
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
          p += (int64_t)gridDim.x * blockDim.x) {
         int lo = 0, hi = nhalo;
@@ -110,19 +133,12 @@ __global__ void init_particles(int64_t n, const int64_t *__restrict__ pstart, in
             int mid = (lo + hi) >> 1;
             if (pstart[mid] <= p) lo = mid; else hi = mid;
         }
-        pos[p] = pos_in[p];
-        perm[p] = (int32_t)p;
-        pnode[p] = lo;  // the root of halo h is node h
+        phalo[p] = lo;
+        const bool active = pstart[lo + 1] - pstart[lo] > kSmall;
+        (active ? pos : fpos)[p] = pos_in[p];
+        (active ? perm : fperm)[p] = (int32_t)p;
+        pnode[p] = active ? lo : -1;  // the root of halo h is node h
     }
-}
-
-// Sum of v over the lanes of `mask` that share this lane's key group.
-template <class T>
-__device__ __forceinline__ T group_sum(unsigned mask, T v) {
-    // mask: lanes with the same node; reduce by walking set bits (<= 32 adds)
-    T acc = 0;
-    for (unsigned m = mask; m; m &= m - 1) acc += __shfl_sync(mask, v, __ffs(m) - 1);
-    return acc;
 }
 
 // Runs of a warp: lanes with equal node ids are consecutive (a node's active
@@ -164,7 +180,8 @@ struct FMaxOp {
 
 // Pass 1: mass and mass-weighted position per node (FP64 accumulation).
 __global__ void __launch_bounds__(kBlock)
-accum_mass(int64_t n, const float4 *__restrict__ pos, const int32_t *__restrict__ pnode, Build b) {
+accum_mass(int L, int64_t n, const float4 *__restrict__ pos, const int32_t *__restrict__ pnode, Build b) {
+    if (b.nact[L] == 0) return;  // a level past the last one (fixed shapes, levels run ahead of the host)
     __shared__ double s[4][kBlock / 32];
     __shared__ int s_node;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -234,7 +251,9 @@ accum_mass(int64_t n, const float4 *__restrict__ pos, const int32_t *__restrict_
 }
 
 __global__ void finalize_com(int L, Build b) {
+    if (b.nact[L] == 0) return;
     FOR_LEVEL_NODES(node, L, b) {
+        if (b.count[node] <= kSmall) continue;
         const double m = b.m[node];
         if (m > 0) {  // ost.c:553-555
             b.mx[node] /= m;
@@ -250,8 +269,9 @@ __global__ void finalize_com(int L, Build b) {
 // (one atomic per value and block: the top levels of large halos), over the
 // warp when it does, else over the warp's runs.
 __global__ void __launch_bounds__(kBlock)
-accum_moments(int64_t n, const float4 *__restrict__ pos, const int32_t *__restrict__ pnode,
+accum_moments(int L, int64_t n, const float4 *__restrict__ pos, const int32_t *__restrict__ pnode,
               uint8_t *__restrict__ pkey, int q5_asbuilt, Build b) {
+    if (b.nact[L] == 0) return;
     constexpr int kWarps = kBlock / 32;
     __shared__ float s_f[7][kWarps];
     __shared__ unsigned s_k[6][kWarps];
@@ -350,12 +370,27 @@ accum_moments(int64_t n, const float4 *__restrict__ pos, const int32_t *__restri
     }
 }
 
+// Takes nch node ids, or -1 when they do not fit (the build is flagged, and
+// the ids up to the capacity become nodes that nothing refers to).
+__device__ __forceinline__ int take_nodes(const Build &b, int nch, int32_t ncap) {
+    const int first = atomicAdd(b.counter, nch);
+    if (first + nch <= ncap) return first;
+    atomicOr(b.counter + 1, 1);
+    for (int id = first; id < ncap && id < first + nch; id++) {
+        b.start[id] = b.count[id] = 0;
+        b.halo[id] = -1;
+    }
+    return -1;
+}
+
 // Decides children, allocates them, and lays out [loose | children] ranges.
-// last: the final level of a fixed-depth build, whose nodes keep all their
-// particles loose (children there would never be processed); a node that
-// would have split flags the build (counter[1]) instead.
+// last: the final level of a fixed-depth build: a node with a child that a
+// further level would have to process keeps all its particles loose and flags
+// the build (counter[1]).
 __global__ void split_nodes(int L, int32_t ncap, int last, Build b) {
+    if (b.nact[L] == 0) return;
     FOR_LEVEL_NODES(node, L, b) {
+    if (b.count[node] <= kSmall) continue;
     const float r2 = __uint_as_float(b.r2[node]);
     const double nodesize = sqrt((double)r2);           // ost.c:574
     const bool divide = nodesize > 0.5 * kMinWidth;     // divideThisNode, tree.h:36
@@ -369,19 +404,20 @@ __global__ void split_nodes(int L, int32_t ncap, int last, Build b) {
 #pragma unroll
     for (int c = 0; c < 8; c++)
         if (divide && cnt[c] >= kMinCell) nch++;
-    if (last && nch > 0) {
+    int nbig = 0;
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+        if (divide && cnt[c] > kSmall) nbig++;
+    if (last && nbig > 0) {
         atomicOr(b.counter + 1, 2);
-        nch = 0;
+        nch = nbig = 0;
     }
     int first = -1;
     if (nch > 0) {
-        first = atomicAdd(b.counter, nch);
-        if (first + nch > ncap) {  // out of node capacity: keep all particles loose
-            atomicOr(b.counter + 1, 1);
-            nch = 0;
-            first = -1;
-        }
+        first = take_nodes(b, nch, ncap);
+        if (first < 0) nch = nbig = 0;  // out of node capacity: keep all particles loose
     }
+    if (nbig > 0) atomicAdd(b.nact + L + 1, nbig);
     const int start = b.start[node], halo = b.halo[node];
     int off = start;
 #pragma unroll
@@ -402,12 +438,17 @@ __global__ void split_nodes(int L, int32_t ncap, int last, Build b) {
         if (child) {
             const int id = first + k++;
             cur[c] = off;
-            child_of[c] = id;
             b.start[id] = off;
             b.count[id] = cnt[c];
             b.halo[id] = halo;
             b.par[id] = node;
-            zero_node(b, id);
+            if (cnt[c] > kSmall) {
+                child_of[c] = id;
+                zero_node(b, id);
+            } else {  // its particles go to the final arrays, as loose ones
+                b.first[id] = L + 1;
+                b.small[atomicAdd(b.counter + 3, 1)] = id;
+            }
             off += cnt[c];
         }
     }
@@ -438,13 +479,14 @@ __global__ void split_nodes(int L, int32_t ncap, int last, Build b) {
 // A particle that stays loose here has its final tree-order slot: it is
 // written once into the final arrays (fpos, fperm) and never copied again;
 // its slot, like every earlier-settled one, carries node -1 into the next
-// level.
-__global__ void scatter_particles(int64_t n, const float4 *__restrict__ pos_in,
+// level.  So do the particles of small children.
+__global__ void scatter_particles(int L, int64_t n, const float4 *__restrict__ pos_in,
                                   const int32_t *__restrict__ perm_in,
                                   const int32_t *__restrict__ pnode_in,
                                   const uint8_t *__restrict__ pkey, float4 *__restrict__ pos_out,
                                   int32_t *__restrict__ perm_out, int32_t *__restrict__ pnode_out,
                                   float4 *__restrict__ fpos, int32_t *__restrict__ fperm, Build b) {
+    if (b.nact[L] == 0) return;
     const int lane = threadIdx.x & 31;
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p - lane < n;
          p += (int64_t)gridDim.x * blockDim.x) {
@@ -473,74 +515,331 @@ __global__ void scatter_particles(int64_t n, const float4 *__restrict__ pos_in,
     }
 }
 
-// subtree sizes, deepest level first
-__global__ void subtree_sizes(int L, Build b) {
-    FOR_LEVEL_NODES(node, L, b) {
-        int s = 1;
-        const int f = b.first[node];
-        for (int c = 0; c < b.nchild[node]; c++) s += b.sub[f + c];
-        b.sub[node] = s;
-    }
+// ---- subtrees of small nodes
+struct SmallWarp {
+    float4 pos[2][kSmall];
+    int32_t perm[2][kSmall];
+    int4 stack[kSmall / kMinCell + 1];  // (node, first place, particles, levels below the root); pending nodes are disjoint
+};
+constexpr int kSmallWarps = 4;
+
+// Field key of eight 16-bit fields in four words.
+__device__ __forceinline__ unsigned field16(const unsigned (&w)[4], int key) {
+    const unsigned a = key & 2 ? w[1] : w[0], c = key & 2 ? w[3] : w[2];
+    return ((key & 4 ? c : a) >> (16 * (key & 1))) & 0xffffu;
 }
 
-// Preorder numbers of the roots: consecutive blocks in halo order (an
-// exclusive scan of the roots' subtree sizes, one block).
-__global__ void __launch_bounds__(1024) root_preorder(int32_t nhalo, Build b) {
-    __shared__ int32_t part[1024];
-    const int t = threadIdx.x;
-    const int per = (nhalo + 1023) / 1024;
-    const int h0 = min(nhalo, t * per), h1 = min(nhalo, h0 + per);
-    int32_t sum = 0;
-    for (int h = h0; h < h1; h++) sum += b.sub[h];
-    part[t] = sum;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {  // inclusive Hillis-Steele scan
-        const int32_t v = t >= off ? part[t - off] : 0;
-        __syncthreads();
-        part[t] += v;
-        __syncthreads();
-    }
-    int32_t acc = part[t] - sum;
-    for (int h = h0; h < h1; h++) {
-        b.pre[h] = acc;
-        acc += b.sub[h];
-    }
-}
-
-// Flags a fixed-depth build that the batch outgrew: a node of the last level
-// that would have split, or the node capacity exceeded.  The tree built is
-// consistent either way (those particles stay loose).
-__global__ void check_build(Build b, int *err) {
-    if (blockIdx.x == 0 && threadIdx.x == 0 && b.counter[1]) atomicOr(err, GF_ERRBIT_PLAN);
-}
-
-// preorder numbers, shallowest level first (roots set beforehand)
-__global__ void preorder(int L, Build b) {
-    FOR_LEVEL_NODES(node, L, b) {
-        int p = b.pre[node] + 1;
-        const int f = b.first[node];
-        for (int c = 0; c < b.nchild[node]; c++) {
-            b.pre[f + c] = p;
-            p += b.sub[f + c];
+// One warp per node of at most kSmall particles: the node and all its
+// descendants, with the rules and formulas of the level passes (accum_mass,
+// accum_moments, split_nodes).  The particles sit in one of two shared
+// buffers; a node's lanes reduce its moments, and place every particle behind
+// its octant's lower lanes: loose ones into the final arrays, those of
+// children into the other buffer.
+__global__ void __launch_bounds__(32 * kSmallWarps)
+small_subtrees(int32_t ncap, int q5_asbuilt, float4 *__restrict__ fpos, int32_t *__restrict__ fperm, Build b) {
+    __shared__ SmallWarp warps[kSmallWarps];
+    SmallWarp &W = warps[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int nsmall = b.counter[3];
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nsmall; i += (gridDim.x * blockDim.x) >> 5) {
+        const int root = b.small[i];
+        const int start = b.start[root], halo = b.halo[root], level = b.first[root];
+        int depth = 0;
+        for (int k = lane; k < b.count[root]; k += 32) {
+            W.pos[0][k] = fpos[start + k];
+            W.perm[0][k] = fperm[start + k];
         }
+        if (lane == 0) W.stack[0] = make_int4(root, 0, b.count[root], 0);
+        __syncwarp();
+        int top = 1;
+        while (top > 0) {
+            const int4 e = W.stack[--top];
+            const int node = e.x, off = e.y, cnt = e.z, buf = e.w & 1;
+            depth = max(depth, e.w);
+            const float4 *X = W.pos[buf] + off;
+            const int32_t *id = W.perm[buf] + off;
+            // ost.c:546-555: mass, mass-weighted position, centre of mass
+            double w = 0, cx = 0, cy = 0, cz = 0;
+            for (int k = lane; k < cnt; k += 32) {
+                const float4 v = X[k];
+                w += v.w;
+                cx += (double)v.w * (double)v.x;
+                cy += (double)v.w * (double)v.y;
+                cz += (double)v.w * (double)v.z;
+            }
+#pragma unroll
+            for (int o = 16; o; o >>= 1) {
+                w += __shfl_xor_sync(0xffffffffu, w, o);
+                cx += __shfl_xor_sync(0xffffffffu, cx, o);
+                cy += __shfl_xor_sync(0xffffffffu, cy, o);
+                cz += __shfl_xor_sync(0xffffffffu, cz, o);
+            }
+            if (w > 0) {
+                cx /= w;
+                cy /= w;
+                cz /= w;
+            }
+            // ost.c:561-571, 589-592: float offsets and moments, octants
+            float r2 = 0.f, q[6] = {0, 0, 0, 0, 0, 0};
+            unsigned bx[6] = {0u, 0u, 0u, 0u, 0u, 0u};  // ~min xyz, max xyz: all maxima
+            unsigned keys = 0, oct = 0;  // octant of each own particle (3 bits), own particles per octant (4 bits)
+            for (int k = lane, u = 0; k < cnt; k += 32, u += 3) {
+                const float4 P = X[k];
+                const float tx = (float)((double)P.x - cx);
+                const float ty = (float)((double)P.y - cy);
+                const float tz = (float)((double)P.z - cz);
+                const float m = P.w;
+                r2 = fmaxf(r2, tx * tx + ty * ty + tz * tz);
+                q[0] += m * tx * tx;
+                q[1] += m * ty * ty;
+                q[2] += m * tz * tz;
+                q[3] += m * tx * ty;
+                q[4] += m * tx * tz;
+                q[5] += q5_asbuilt ? m * ty * tx : m * ty * tz;
+                const unsigned fx = fkey(P.x), fy = fkey(P.y), fz = fkey(P.z);
+                bx[0] = max(bx[0], ~fx);
+                bx[1] = max(bx[1], ~fy);
+                bx[2] = max(bx[2], ~fz);
+                bx[3] = max(bx[3], fx);
+                bx[4] = max(bx[4], fy);
+                bx[5] = max(bx[5], fz);
+                const unsigned key = ((double)P.x > cx ? 1 : 0) | ((double)P.y > cy ? 2 : 0) | ((double)P.z > cz ? 4 : 0);
+                keys |= key << u;
+                oct += 1u << (4 * key);
+            }
+            const unsigned r2b = __reduce_max_sync(0xffffffffu, __float_as_uint(r2));  // non-negative floats
+#pragma unroll
+            for (int a = 0; a < 6; a++) {
+                bx[a] = __reduce_max_sync(0xffffffffu, bx[a]);
+#pragma unroll
+                for (int o = 16; o; o >>= 1) q[a] += __shfl_xor_sync(0xffffffffu, q[a], o);
+            }
+            // particles of every octant in the lanes up to this one: two
+            // 16-bit counts per word
+            unsigned at[4], sum[4];
+#pragma unroll
+            for (int a = 0; a < 4; a++) {
+                const unsigned own = ((oct >> (8 * a)) & 15u) | (((oct >> (8 * a + 4)) & 15u) << 16);
+                unsigned v = own;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned t = __shfl_up_sync(0xffffffffu, v, o);
+                    if (lane >= o) v += t;
+                }
+                sum[a] = __shfl_sync(0xffffffffu, v, 31);
+                at[a] = v - own;  // in the lanes before
+            }
+            // ost.c:574, tree.h:36: children are octants of at least kMinCell
+            // particles of a node that is large enough
+            const bool divide = sqrt((double)__uint_as_float(r2b)) > 0.5 * kMinWidth;
+            unsigned child = 0;  // octants that become children
+#pragma unroll
+            for (int c = 0; c < 8; c++)
+                if (divide && ((sum[c >> 1] >> (16 * (c & 1))) & 0xffffu) >= (unsigned)kMinCell) child |= 1u << c;
+            int first = -1;
+            if (child && level + e.w + 2 > kMaxLevels) {  // only non-finite or degenerate particles nest like this
+                if (lane == 0) atomicOr(b.counter + 1, 4);
+                child = 0;
+            }
+            if (child) {
+                if (lane == 0) first = take_nodes(b, __popc(child), ncap);
+                first = __shfl_sync(0xffffffffu, first, 0);
+                if (first < 0) child = 0;  // out of node capacity: keep all particles loose
+            }
+            // [loose | child 0 | child 1 | ...]: places of the octants, added
+            // to the counts of the lanes before
+            int place = 0, nloose = 0;
+            __syncwarp();  // every lane has read this node's stack entry
+#pragma unroll
+            for (int pass = 0; pass < 2; pass++) {
+                int k = 0;
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    const int n = (sum[c >> 1] >> (16 * (c & 1))) & 0xffffu;
+                    const bool is_child = (child >> c) & 1u;
+                    if (is_child != (pass == 1)) continue;
+                    at[c >> 1] += (unsigned)place << (16 * (c & 1));
+                    if (is_child) {
+                        if (lane == 0) {
+                            const int kid = first + k;
+                            W.stack[top + k] = make_int4(kid, off + place, n, e.w + 1);
+                            b.start[kid] = start + off + place;
+                            b.count[kid] = n;
+                            b.halo[kid] = halo;
+                            b.par[kid] = node;
+                        }
+                        k++;
+                    }
+                    place += n;
+                }
+                if (pass == 0) nloose = place;
+            }
+            top += __popc(child);
+            unsigned seen = 0;  // own particles placed, per octant
+            for (int k = lane; k < cnt; k += 32, keys >>= 3) {
+                const int key = keys & 7;
+                const int dst = (int)field16(at, key) + (int)((seen >> (4 * key)) & 15u);
+                seen += 1u << (4 * key);
+                const float4 v = X[k];
+                const int32_t pi = id[k];
+                if ((child >> key) & 1u) {
+                    W.pos[buf ^ 1][off + dst] = v;
+                    W.perm[buf ^ 1][off + dst] = pi;
+                } else {
+                    fpos[start + off + dst] = v;
+                    fperm[start + off + dst] = pi;
+                }
+            }
+            if (lane == 0) {
+                b.m[node] = w;
+                b.mx[node] = cx;
+                b.my[node] = cy;
+                b.mz[node] = cz;
+                b.r2[node] = r2b;
+#pragma unroll
+                for (int a = 0; a < 6; a++) {
+                    b.q[6 * (int64_t)node + a] = q[a];
+                    b.box[6 * (int64_t)node + a] = bx[a];
+                }
+                b.first[node] = first;
+                b.nchild[node] = __popc(child);
+                b.lstart[node] = start + off;
+                b.lcount[node] = nloose;
+            }
+            __syncwarp();  // the stack and the other buffer are written
+        }
+        if (lane == 0) atomicMax(b.counter + 4, level + depth + 1);
     }
 }
 
-__global__ void emit_nodes(int nlev, float theta2, Build b, KnnNode *__restrict__ knn,
-                           BhNode *__restrict__ bh, WalkNode *__restrict__ walk,
-                           int32_t *__restrict__ owner) {
-    for (int node = blockIdx.x * blockDim.x + threadIdx.x; node < b.lev[nlev]; node += gridDim.x * blockDim.x) {
-    const int i = b.pre[node];
+// ---- numbering
+// hist[p]: nodes whose first particle is p (nodes without particles apart).
+__global__ void count_starts(int32_t ncap, Build b, int32_t *__restrict__ hist) {
+    const int nn = min(b.counter[0], ncap);
+    for (int node = blockIdx.x * blockDim.x + threadIdx.x; node < nn; node += gridDim.x * blockDim.x)
+        if (b.count[node] > 0) atomicAdd(hist + b.start[node], 1);
+}
+
+constexpr int kScanThreads = 256, kScanItems = 16, kScanChunk = kScanThreads * kScanItems;
+
+// Exclusive scan of `v` over the block's threads; `total` receives the sum.
+template <int THREADS>
+__device__ __forceinline__ int block_scan(int v, int &total, int *scratch) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) scratch[warp] = inc;
+    __syncthreads();
+    int before = 0;
+    total = 0;
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; w++) {
+        if (w < warp) before += scratch[w];
+        total += scratch[w];
+    }
+    __syncthreads();  // scratch is reused
+    return before + inc - v;
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+scan_sums(int64_t n, const int32_t *__restrict__ hist, int32_t *__restrict__ sums) {
+    __shared__ int scratch[kScanThreads / 32];
+    const int64_t base = blockIdx.x * (int64_t)kScanChunk;
+    int v = 0;
+#pragma unroll
+    for (int i = 0; i < kScanItems; i++) {
+        const int64_t p = base + threadIdx.x + i * kScanThreads;
+        if (p < n) v += hist[p];
+    }
+    int total;
+    block_scan<kScanThreads>(v, total, scratch);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+// The chunk sums (in place) and, per halo, the halos before it without
+// particles (their roots are nodes too), as exclusive prefixes: one block.
+__global__ void __launch_bounds__(1024)
+scan_mid(int64_t nchunk, int32_t *__restrict__ sums, int32_t nhalo, const int64_t *__restrict__ pstart,
+         int32_t *__restrict__ empty) {
+    __shared__ int scratch[32];
+    int run = 0, total;
+    for (int64_t c = 0; c < nchunk; c += 1024) {
+        const int v = c + threadIdx.x < nchunk ? sums[c + threadIdx.x] : 0;
+        const int at = run + block_scan<1024>(v, total, scratch);
+        if (c + threadIdx.x < nchunk) sums[c + threadIdx.x] = at;
+        run += total;
+    }
+    run = 0;
+    for (int32_t c = 0; c < nhalo; c += 1024) {
+        const int h = c + threadIdx.x;
+        const int v = h < nhalo && pstart[h] == pstart[h + 1];
+        const int at = run + block_scan<1024>(v, total, scratch);
+        if (h < nhalo) empty[h] = at;
+        run += total;
+    }
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+scan_chunks(int64_t n, int32_t *__restrict__ hist, const int32_t *__restrict__ sums) {
+    __shared__ int scratch[kScanThreads / 32];
+    const int64_t base = blockIdx.x * (int64_t)kScanChunk + threadIdx.x * (int64_t)kScanItems;
+    int v[kScanItems], s = 0;
+#pragma unroll
+    for (int i = 0; i < kScanItems; i++) {
+        v[i] = base + i < n ? hist[base + i] : 0;
+        s += v[i];
+    }
+    int total;
+    int at = sums[blockIdx.x] + block_scan<kScanThreads>(s, total, scratch);
+#pragma unroll
+    for (int i = 0; i < kScanItems; i++) {
+        if (base + i < n) hist[base + i] = at;
+        at += v[i];
+    }
+}
+
+// Preorder number of a node and its subtree's size.  before[p]: nodes with
+// particles that start before particle p.
+__device__ __forceinline__ int2 number_of(const Build &b, const int32_t *__restrict__ before,
+                                          const int32_t *__restrict__ empty, int node) {
+    const int s = b.start[node], c = b.count[node], h = b.halo[node];
+    if (c == 0) return make_int2(before[s] + empty[h], 1);
+    int above = 0;  // ancestors that start with the same particle
+    for (int p = b.par[node]; p >= 0 && b.start[p] == s; p = b.par[p]) above++;
+    return make_int2(before[s] + above + empty[h], before[s + c] - before[s] - above);
+}
+
+// fixed: flag a build that the batch outgrew (a node of the last level that
+// would have split into large ones, or the node capacity exceeded); the tree
+// is consistent either way (those particles stay loose).
+__global__ void emit_nodes(int32_t ncap, float theta2, Build b, const int32_t *__restrict__ before,
+                           const int32_t *__restrict__ empty, int32_t nhalo, KnnNode *__restrict__ knn,
+                           BhNode *__restrict__ bh, WalkNode *__restrict__ walk, int32_t *__restrict__ owner,
+                           int32_t *__restrict__ root, int32_t *__restrict__ rend, int fixed, int *err) {
+    if (fixed && blockIdx.x == 0 && threadIdx.x == 0 && b.counter[1]) atomicOr(err, GF_ERRBIT_PLAN);
+    const int nn = min(b.counter[0], ncap);
+    for (int node = blockIdx.x * blockDim.x + threadIdx.x; node < nn; node += gridDim.x * blockDim.x) {
+    if (b.halo[node] < 0) continue;  // an id that the capacity cut off
+    const int2 num = number_of(b, before, empty, node);
+    const int i = num.x;
+    if (node < nhalo) {
+        root[node] = i;
+        rend[node] = i + num.y;
+    }
     KnnNode k;
     for (int a = 0; a < 3; a++) {
         k.lo[a] = fkey_inv(~b.box[6 * (int64_t)node + a]);
         k.hi[a] = fkey_inv(b.box[6 * (int64_t)node + 3 + a]);
     }
-    k.skip = i + b.sub[node];
+    k.skip = i + num.y;
     k.lstart = b.lstart[node];
     k.lcount = b.lcount[node];
     k.count = b.count[node];
-    k.parent = b.par[node] >= 0 ? b.pre[b.par[node]] : -1;
+    k.parent = b.par[node] >= 0 ? number_of(b, before, empty, b.par[node]).x : -1;
     k.pad = 0;
     for (int j = 0; j < k.lcount; j++) owner[k.lstart + j] = i;
     knn[i] = k;
@@ -587,27 +886,6 @@ __global__ void emit_nodes(int nlev, float theta2, Build b, KnnNode *__restrict_
     }
 }
 
-__global__ void emit_roots(int32_t nhalo, Build b, int32_t *__restrict__ root,
-                           int32_t *__restrict__ rend) {
-    int h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= nhalo) return;
-    root[h] = b.pre[h];
-    rend[h] = b.pre[h] + b.sub[h];
-}
-
-__global__ void particle_halo(int64_t n, const int64_t *__restrict__ pstart, int32_t nhalo,
-                              int32_t *__restrict__ phalo) {
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
-         p += (int64_t)gridDim.x * blockDim.x) {
-        int lo = 0, hi = nhalo;
-        while (hi - lo > 1) {
-            int mid = (lo + hi) >> 1;
-            if (pstart[mid] <= p) lo = mid; else hi = mid;
-        }
-        phalo[p] = lo;
-    }
-}
-
 int grid_n(int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((n + kBlock - 1) / kBlock, sm_count() * 8));
 }
@@ -638,7 +916,10 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
     for (int attempt = 0; attempt < (fixed ? 1 : 4); attempt++, ncap *= 2) {
         // ---- particle buffers: pos x2, perm x2, pnode x2, key
         auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
-        const size_t pbytes = 3 * al(n * sizeof(float4)) + 5 * al(n * sizeof(int32_t)) + al(n);
+        const int64_t nscan = n + 1, nchunk = (nscan + kScanChunk - 1) / kScanChunk;
+        const size_t pbytes = 3 * al(n * sizeof(float4)) + 6 * al(n * sizeof(int32_t)) + al(n) +
+                              al(nscan * sizeof(int32_t)) + al(nchunk * sizeof(int32_t)) +
+                              al(std::max(nhalo, 1) * sizeof(int32_t));
         GF_TRY(ctx->tree[0].reserve(pbytes + 256));
         char *pp = ctx->tree[0].as<char>();
         float4 *pos[2] = {carve<float4>(pp, n), carve<float4>(pp, n)};
@@ -647,11 +928,15 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
         uint8_t *pkey = carve<uint8_t>(pp, n);
         float4 *fpos = carve<float4>(pp, n);    // final tree order, written as particles settle
         int32_t *fperm = carve<int32_t>(pp, n);
+        int32_t *phalo = carve<int32_t>(pp, n);
+        int32_t *before = carve<int32_t>(pp, nscan);  // nodes starting at, then before, each particle
+        int32_t *sums = carve<int32_t>(pp, nchunk);
+        int32_t *empty = carve<int32_t>(pp, std::max(nhalo, 1));
         // ---- node buffers (BFS numbering): exactly the carves below
         const size_t nc = (size_t)ncap;
         const size_t nbytes = 3 * al(nc * 4) + 4 * al(nc * 8) + al(nc * 4) + al(nc * 24) +
-                              al(nc * 24) + 3 * al(nc * 32) + 7 * al(nc * 4) + al(64) +
-                              al((kMaxLevels + 2) * sizeof(int32_t));
+                              al(nc * 24) + 3 * al(nc * 32) + 6 * al(nc * 4) + al(64) +
+                              2 * al((kMaxLevels + 2) * sizeof(int32_t));
         GF_TRY(ctx->tree[1].reserve(nbytes + 256));
         char *np_ = ctx->tree[1].as<char>();
         Build b;
@@ -672,78 +957,79 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
         b.nchild = carve<int32_t>(np_, nc);
         b.lstart = carve<int32_t>(np_, nc);
         b.lcount = carve<int32_t>(np_, nc);
-        b.sub = carve<int32_t>(np_, nc);
-        b.pre = carve<int32_t>(np_, nc);
         b.par = carve<int32_t>(np_, nc);
+        b.small = carve<int32_t>(np_, nc);
         b.counter = carve<int32_t>(np_, 16);
+        b.nact = carve<int32_t>(np_, kMaxLevels + 2);
+        char *const zero_end = np_;
         b.lev = carve<int32_t>(np_, kMaxLevels + 2);
         cudaStream_t s = ctx->stream;
-        init_build<<<1, 32, 0, s>>>(nhalo, b);
+        GF_CUDA_TRY(cudaMemsetAsync(b.counter, 0, zero_end - (char *)b.counter, s));
+        GF_CUDA_TRY(cudaMemsetAsync(before, 0, nscan * sizeof(int32_t), s));
+        init_roots<<<grid_exact(nhalo, 256), 256, 0, s>>>(nhalo, pstart_dev, b);
         GF_LAUNCH_CHECK();
-        if (nhalo > 0) {
-            init_roots<<<grid_exact(nhalo, 256), 256, 0, s>>>(nhalo, pstart_dev, b);
-            GF_LAUNCH_CHECK();
-        }
-        init_particles<<<grid_n(n), kBlock, 0, s>>>(n, pstart_dev, nhalo, pos_in, pos[0], perm[0],
-                                                    pnode[0]);
+        init_particles<<<grid_n(n), kBlock, 0, s>>>(n, pstart_dev, nhalo, pos_in, pos[0], perm[0], pnode[0], fpos,
+                                                    fperm, phalo);
         GF_LAUNCH_CHECK();
-        // Level by level.  Eagerly, the node count is read back after each
-        // level and the build stops at the first level that allocates no
-        // children; with a fixed shape it runs fixed->levels levels without
-        // a host round trip (the levels past the tree's depth are empty: their
-        // particle passes copy settled particles through) and check_build
-        // flags a tree that needed more levels or nodes.
+        // Level by level.  Eagerly, the host looks after every third level
+        // whether a level is left (levels past the last one return at once);
+        // with a fixed shape fixed->levels levels run without a host round
+        // trip and emit_nodes flags a tree that needed more levels or nodes.
+        // A batch of at most kSmall particles has no node for these passes.
         const int fixed_grid = sm_count() * 4;
-        std::vector<int32_t> levels = {0, nhalo};  // eager only: the host copy of b.lev
+        const int level_grid = (int)std::min<int64_t>(fixed_grid, std::max<int64_t>(n / 4096, nhalo / 256) + 1);
         int cur = 0;
-        int32_t hc[2] = {nhalo, 0};
-        int nlev = 0;
-        for (int L = 0; fixed ? L < fixed->levels : levels[L] < levels[L + 1]; L++) {
-            const int gl = fixed ? fixed_grid : grid_exact(levels[L + 1] - levels[L], 256);
-            accum_mass<<<grid_n(n), kBlock, 0, s>>>(n, pos[cur], pnode[cur], b);
+        int32_t hc[16] = {0}, act = 0;
+        bool more = fixed || n > kSmall;
+        for (int L = 0; more; L++) {
+            if (fixed ? L == fixed->levels : L >= kMaxLevels) {
+                if (fixed) break;
+                set_status(GF_EINVAL, "octree deeper than %d levels", kMaxLevels);
+                return GF_EINVAL;
+            }
+            accum_mass<<<grid_n(n), kBlock, 0, s>>>(L, n, pos[cur], pnode[cur], b);
             GF_LAUNCH_CHECK();
-            finalize_com<<<gl, 256, 0, s>>>(L, b);
+            finalize_com<<<level_grid, 256, 0, s>>>(L, b);
             GF_LAUNCH_CHECK();
-            accum_moments<<<grid_n(n), kBlock, 0, s>>>(n, pos[cur], pnode[cur], pkey, q5_asbuilt, b);
+            accum_moments<<<grid_n(n), kBlock, 0, s>>>(L, n, pos[cur], pnode[cur], pkey, q5_asbuilt, b);
             GF_LAUNCH_CHECK();
-            split_nodes<<<gl, 256, 0, s>>>(L, (int32_t)ncap, fixed && L == fixed->levels - 1, b);
+            split_nodes<<<level_grid, 256, 0, s>>>(L, (int32_t)ncap, fixed && L == fixed->levels - 1, b);
             GF_LAUNCH_CHECK();
-            scatter_particles<<<grid_n(n), kBlock, 0, s>>>(n, pos[cur], perm[cur], pnode[cur], pkey,
+            scatter_particles<<<grid_n(n), kBlock, 0, s>>>(L, n, pos[cur], perm[cur], pnode[cur], pkey,
                                                            pos[cur ^ 1], perm[cur ^ 1],
                                                            pnode[cur ^ 1], fpos, fperm, b);
             GF_LAUNCH_CHECK();
             cur ^= 1;
-            nlev = L + 1;
-            if (fixed) continue;
+            if (fixed || L % 3 != 2) continue;
+            GF_CUDA_TRY(cudaMemcpyAsync(&act, b.nact + L + 1, sizeof(act), cudaMemcpyDeviceToHost, s));
+            GF_CUDA_TRY(cudaStreamSynchronize(s));
+            more = act > 0;
+        }
+        small_subtrees<<<fixed ? sm_count() * 5 : (int)std::max<int64_t>(1, std::min<int64_t>(n / 64 + nhalo / 4 + 1, sm_count() * 5)),
+                         32 * kSmallWarps, 0, s>>>((int32_t)ncap, q5_asbuilt, fpos, fperm, b);
+        GF_LAUNCH_CHECK();
+        int32_t nnode = -1;
+        if (!fixed) {
             GF_CUDA_TRY(cudaMemcpyAsync(hc, b.counter, sizeof(hc), cudaMemcpyDeviceToHost, s));
             GF_CUDA_TRY(cudaStreamSynchronize(s));
-            if (hc[1]) break;
-            levels.push_back(std::min<int32_t>(hc[0], (int32_t)ncap));
-            if (levels.size() > (size_t)kMaxLevels) {
+            if (hc[1] & 4) {
                 set_status(GF_EINVAL, "octree deeper than %d levels", kMaxLevels);
                 return GF_EINVAL;
             }
+            if (hc[1]) continue;  // node capacity exceeded: retry with more nodes
+            nnode = hc[0];
         }
-        if (hc[1]) continue;  // node capacity exceeded: retry with more nodes
-        if (fixed) {
-            check_build<<<1, 32, 0, s>>>(b, ctx->d_err);
-            GF_LAUNCH_CHECK();
-        }
-        const int32_t nnode = fixed ? -1 : levels.back();
-        for (int L = nlev - 1; L >= 0; L--) {
-            subtree_sizes<<<fixed ? fixed_grid : grid_exact(levels[L + 1] - levels[L], 256), 256, 0, s>>>(L, b);
-            GF_LAUNCH_CHECK();
-        }
-        if (nhalo > 0) {
-            root_preorder<<<1, 1024, 0, s>>>(nhalo, b);
-            GF_LAUNCH_CHECK();
-        }
-        for (int L = 0; L < nlev; L++) {
-            preorder<<<fixed ? fixed_grid : grid_exact(levels[L + 1] - levels[L], 256), 256, 0, s>>>(L, b);
-            GF_LAUNCH_CHECK();
-        }
+        const int node_grid = fixed ? fixed_grid : grid_exact(nnode, 256);
+        count_starts<<<node_grid, 256, 0, s>>>((int32_t)ncap, b, before);
+        GF_LAUNCH_CHECK();
+        scan_sums<<<(unsigned)nchunk, kScanThreads, 0, s>>>(nscan, before, sums);
+        GF_LAUNCH_CHECK();
+        scan_mid<<<1, 1024, 0, s>>>(nchunk, sums, nhalo, pstart_dev, empty);
+        GF_LAUNCH_CHECK();
+        scan_chunks<<<(unsigned)nchunk, kScanThreads, 0, s>>>(nscan, before, sums);
+        GF_LAUNCH_CHECK();
         if (shape) {
-            shape->levels = nlev;
+            shape->levels = std::max(hc[4], 1);
             shape->ncap = ncap;
             shape->nnode = nnode;
         }
@@ -751,8 +1037,7 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
         const int64_t nout = fixed ? ncap : std::max(nnode, 1);  // node slots written
         const size_t obytes = al((size_t)nout * sizeof(KnnNode)) + al((size_t)nout * sizeof(BhNode)) +
                               al((size_t)nout * sizeof(WalkNode)) +
-                              2 * al((size_t)std::max(nhalo, 1) * 4) +
-                              2 * al((size_t)std::max<int64_t>(n, 1) * 4);
+                              2 * al((size_t)std::max(nhalo, 1) * 4) + al((size_t)std::max<int64_t>(n, 1) * 4);
         GF_TRY(ctx->tree[2].reserve(obytes + 256));
         char *op = ctx->tree[2].as<char>();
         KnnNode *knn = carve<KnnNode>(op, (size_t)nout);
@@ -760,17 +1045,12 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
         WalkNode *walk = carve<WalkNode>(op, (size_t)nout);
         int32_t *root = carve<int32_t>(op, std::max(nhalo, 1));
         int32_t *rend = carve<int32_t>(op, std::max(nhalo, 1));
-        int32_t *phalo = carve<int32_t>(op, std::max<int64_t>(n, 1));
         int32_t *owner = carve<int32_t>(op, std::max<int64_t>(n, 1));
         if (fixed || nnode > 0) {
-            emit_nodes<<<fixed ? fixed_grid : grid_exact(nnode, 256), 256, 0, s>>>(nlev, theta2, b, knn, bh,
-                                                                                  walk, owner);
-            GF_LAUNCH_CHECK();
-            emit_roots<<<grid_exact(nhalo, 256), 256, 0, s>>>(nhalo, b, root, rend);
+            emit_nodes<<<node_grid, 256, 0, s>>>((int32_t)ncap, theta2, b, before, empty, nhalo, knn, bh, walk, owner,
+                                                 root, rend, fixed ? 1 : 0, ctx->d_err);
             GF_LAUNCH_CHECK();
         }
-        particle_halo<<<grid_n(n), kBlock, 0, s>>>(n, pstart_dev, nhalo, phalo);
-        GF_LAUNCH_CHECK();
         out->nhalo = nhalo;
         out->nnode = nnode;
         out->n = n;

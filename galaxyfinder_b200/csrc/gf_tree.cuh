@@ -24,8 +24,9 @@ __device__ __forceinline__ float w4(float dist, float h) {
 // theta2 fills BhNode::open_r2; q5_asbuilt reproduces ost.c:571 (m*y*x in
 // place of m*y*z).  Buffers live in ctx->tree[]; the view stays valid until
 // the next build on ctx.
-// Shape of a built octree: levels processed, node capacity and node count
-// (-1 for a build with a fixed shape, whose count stays on the device).
+// Shape of a built octree: depth (of a fixed shape: the levels that may hold
+// nodes of more than 256 particles), node capacity and node count (-1 for a
+// build with a fixed shape, whose count stays on the device).
 struct TreeShape {
     int32_t levels = 0;
     int64_t ncap = 0;
