@@ -396,6 +396,10 @@ int gf_ctx_destroy(gf_ctx *c) {
     for (auto &b : c->tmp) b.release();
     for (auto &b : c->tree) b.release();
     for (auto &b : c->pin) b.release();
+    for (auto &e : c->side_ev)
+        if (e) cudaEventDestroy(e);
+    for (auto &t : c->side)
+        if (t) cudaStreamDestroy(t);
     if (c->d_err) cudaFree(c->d_err);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -404,6 +408,7 @@ int gf_ctx_destroy(gf_ctx *c) {
 
 int gf_ctx_set_stream(gf_ctx *c, void *stream) {
     if (!c) return GF_EINVAL;
+    std::lock_guard<std::mutex> g(c->lock);  // a stage running on c switches c->stream to its side streams
     if (c->own_stream) cudaStreamDestroy(c->stream);
     c->stream = (cudaStream_t)stream;
     c->own_stream = false;

@@ -165,6 +165,10 @@ struct gf_ctx {
     gf::DevBuf tree[16];
     gf::HostPinned pin[4];
     gf::TreeView last_tree;  // the most recent build_tree() on this context
+    // the stage's side streams (stream's priority) and their fork and join events
+    cudaStream_t side[2] = {nullptr, nullptr};
+    int side_priority = 0;
+    cudaEvent_t side_ev[2] = {nullptr, nullptr};
     std::mutex lock;
 };
 

@@ -54,6 +54,68 @@ struct EventTimer {
     }
 };
 
+// The stage's independent parts on streams of their own: the mesh boxes and
+// their zeroing beside the octree build, then the rest of the mesh part and the
+// potential beside the neighbour search.  One after the other, each part of a
+// batch of up to some 1e5 particles ends with a tail of few busy SMs (a warp's
+// walk or search takes as long as the whole wave) and the mesh part is a chain
+// of launches of a few microseconds.  us for a stage in a row / with the mesh
+// part aside / with the potential aside too: 120 particles 245 / 229 / 216,
+// one halo of 131,072 1281 / 1190 / 1076, 256 halos (247 k) 1683 / 1490 /
+// 1370, replayed graph of 64 halos 608 / 508 / 441, 4096 halos (6 M) 25170 /
+// 24789 / 24989.  The mesh part is queued before the search: behind its blocks,
+// which stay for the whole search, 131,072 took 1099.
+// Work is put on a side stream by switching ctx->stream (the caller holds
+// ctx's lock), starts after what ctx's own stream held at the fork, and is
+// joined back into it, on errors too.
+class Lanes {
+  public:
+    Lanes(gf_ctx *c, bool on) : ctx_(c), own_(c->stream), on_(on) {}
+    ~Lanes() {
+        for (int i = 0; i < 2; i++) join(i);
+    }
+    int open() {
+        if (!on_) return GF_OK;
+        int prio = 0;
+        GF_CUDA_TRY(cudaStreamGetPriority(own_, &prio));
+        for (int i = 0; i < 2; i++) {
+            if (ctx_->side[i] && ctx_->side_priority != prio) {
+                GF_CUDA_TRY(cudaStreamDestroy(ctx_->side[i]));
+                ctx_->side[i] = nullptr;
+            }
+            if (!ctx_->side[i]) GF_CUDA_TRY(cudaStreamCreateWithPriority(&ctx_->side[i], cudaStreamNonBlocking, prio));
+            if (!ctx_->side_ev[i]) GF_CUDA_TRY(cudaEventCreateWithFlags(&ctx_->side_ev[i], cudaEventDisableTiming));
+        }
+        ctx_->side_priority = prio;
+        return GF_OK;
+    }
+    // Work put on lane i after this waits for what the context's stream holds now.
+    int fork(int i) {
+        if (!on_) return GF_OK;
+        GF_CUDA_TRY(cudaEventRecord(ctx_->side_ev[i], own_));
+        GF_CUDA_TRY(cudaStreamWaitEvent(ctx_->side[i], ctx_->side_ev[i], 0));
+        forked_[i] = true;
+        return GF_OK;
+    }
+    void use(int i) {
+        if (on_) ctx_->stream = ctx_->side[i];
+    }
+    void back() { ctx_->stream = own_; }
+    int join(int i) {
+        back();
+        if (!forked_[i]) return GF_OK;
+        forked_[i] = false;
+        GF_CUDA_TRY(cudaEventRecord(ctx_->side_ev[i], ctx_->side[i]));
+        GF_CUDA_TRY(cudaStreamWaitEvent(own_, ctx_->side_ev[i], 0));
+        return GF_OK;
+    }
+
+  private:
+    gf_ctx *ctx_;
+    cudaStream_t own_;
+    bool on_, forked_[2] = {false, false};
+};
+
 }  // namespace
 
 PotentialParams potential_params(float theta2, int ndirect, double potentfact, int add_bg) {
@@ -194,10 +256,63 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
     const double *frame_dev = ctx->mesh.as<double>();
     const gf_mesh_desc *mesh_dev =
         reinterpret_cast<const gf_mesh_desc *>(ctx->mesh.as<char>() + ((frame_bytes + 255) & ~size_t(255)));
+    // the mesh part's host plan (the FP64 stage has its own)
+    const bool do_mesh = cfg->do_mesh && !cfg->plain_fp64;
+    const double vf = tsc_volfact();
+    OnChipMeshes oc;
+    SmoothPlan sp;
+    char *dbuf = nullptr;
+    if (do_mesh) {
+        GF_TRY(ctx->tmp[3].reserve(sizeof(float) * (size_t)std::max<int64_t>(dev_cells, 1)));
+        GF_TRY(ctx->mesh_boxes.reserve(sizeof(int32_t) * kMeshBoxInts * (size_t)std::max(nh, 1)));
+        if (!onchip_halos.empty()) {
+            if (!o->dens_mesh || !volfact_folds(vf)) {
+                set_status(GF_EINVAL, "on-chip meshes need dens_mesh and a power-of-two volfact");
+                return GF_EINVAL;
+            }
+            oc.nmesh = (int32_t)onchip_halos.size();
+            oc.halos_host = onchip_halos.data();
+            oc.ptype = cfg->mesh.ptype;
+            oc.pstart = b->pstart;
+            oc.x = xr;
+            oc.y = yr;
+            oc.z = zr;
+            oc.mass = b->mass;
+            oc.type = b->type;
+            oc.volfold = (float)vf;
+            oc.densph = o->dens_mesh;
+        }
+        GF_TRY(smooth_plan(nh, mesh.data(), onchip_halos.empty() ? nullptr : &oc, &sp));
+        GF_TRY(smooth_upload(ctx, sp, &dbuf));
+    }
+    float *den = ctx->tmp[3].as<float>();
+    int32_t *boxes = ctx->mesh_boxes.as<int32_t>();
+    // only findDen reads the stage's meshes: with FFT axes and a folding
+    // volfact the passes run over the occupied boxes, and only the deposit
+    // boxes are zeroed (the rest of den is never read)
+    const bool box_mode = do_mesh && sp.box_ok && volfact_folds(vf) && !sp.blob.empty();
+    const bool need_tree = cfg->knn_k > 0 || cfg->do_potential;
     GF_TRY(recentre(ctx, b, hid, frame_dev, cfg->box, xr, yr, zr, pos));
     tm.mark();  // 1
+    // phases that are timed run one after the other
+    Lanes lanes(ctx, need_tree && do_mesh && !st);
+    GF_TRY(lanes.open());
+    auto mesh_prepare = [&]() -> int {
+        if (box_mode) {
+            GF_TRY(launch_mesh_boxes(ctx, n, xr, yr, zr, b->type, hid, nh, mesh_dev, boxes));
+            GF_TRY(smooth_box_prepare(ctx, sp, dbuf, mesh_dev, den, boxes));
+        } else {
+            GF_CUDA_TRY(cudaMemsetAsync(den, 0, sizeof(float) * dev_cells, ctx->stream));
+        }
+        return GF_OK;
+    };
+    if (do_mesh && !st) {
+        GF_TRY(lanes.fork(0));
+        lanes.use(0);
+        GF_TRY(mesh_prepare());
+        lanes.back();
+    }
     // ---- 2. octree
-    const bool need_tree = cfg->knn_k > 0 || cfg->do_potential;
     if (need_tree)
         GF_TRY(build_tree(ctx, nh, n, b->pstart, pos, cfg->theta2, cfg->q5_asbuilt, &ctx->last_tree, nullptr,
                           plan ? &plan->tree : nullptr));
@@ -232,62 +347,23 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
         }
         return status;
     }
+    if (cfg->knn_k > 0 && !o->nearindex) {
+        set_status(GF_EINVAL, "knn_k > 0 needs nearindex");
+        return GF_EINVAL;
+    }
     // ---- 3. kNN + SPH density
-    if (cfg->knn_k > 0) {
-        if (!o->nearindex) {
-            set_status(GF_EINVAL, "knn_k > 0 needs nearindex");
-            return GF_EINVAL;
-        }
+    auto knn = [&]() -> int {
+        if (cfg->knn_k <= 0) return GF_OK;
         unsigned long long *kc = nullptr;
         if (st && cfg->count_work) {
             GF_TRY(ctx->tmp[4].reserve(128));
             kc = ctx->tmp[4].as<unsigned long long>() + 4;
-            GF_CUDA_TRY(cudaMemsetAsync(kc, 0, 5 * sizeof(unsigned long long), s));
+            GF_CUDA_TRY(cudaMemsetAsync(kc, 0, 5 * sizeof(unsigned long long), ctx->stream));
         }
-        GF_TRY(launch_knn(ctx, ctx->last_tree, b->pstart, pos, cfg->knn_k, o->nearindex, o->dens_sph, kc));
-    }
-    tm.mark();  // 3
+        return launch_knn(ctx, ctx->last_tree, b->pstart, pos, cfg->knn_k, o->nearindex, o->dens_sph, kc);
+    };
     // ---- 4. TSC mesh -> smoothing -> findDen
-    bool used_box_mode = false;
-    if (cfg->do_mesh) {
-        GF_TRY(ctx->tmp[3].reserve(sizeof(float) * (size_t)std::max<int64_t>(dev_cells, 1)));
-        float *den = ctx->tmp[3].as<float>();
-        const double vf = tsc_volfact();
-        GF_TRY(ctx->mesh_boxes.reserve(sizeof(int32_t) * kMeshBoxInts * (size_t)std::max(nh, 1)));
-        int32_t *boxes = ctx->mesh_boxes.as<int32_t>();
-        OnChipMeshes oc;
-        if (!onchip_halos.empty()) {
-            if (!o->dens_mesh || !volfact_folds(vf)) {
-                set_status(GF_EINVAL, "on-chip meshes need dens_mesh and a power-of-two volfact");
-                return GF_EINVAL;
-            }
-            oc.nmesh = (int32_t)onchip_halos.size();
-            oc.halos_host = onchip_halos.data();
-            oc.ptype = cfg->mesh.ptype;
-            oc.pstart = b->pstart;
-            oc.x = xr;
-            oc.y = yr;
-            oc.z = zr;
-            oc.mass = b->mass;
-            oc.type = b->type;
-            oc.volfold = (float)vf;
-            oc.densph = o->dens_mesh;
-        }
-        SmoothPlan sp;
-        GF_TRY(smooth_plan(nh, mesh.data(), onchip_halos.empty() ? nullptr : &oc, &sp));
-        // only findDen reads the stage's meshes: with FFT axes and a folding
-        // volfact the passes run over the occupied boxes, and only the deposit
-        // boxes are zeroed (the rest of den is never read)
-        const bool box_mode = sp.box_ok && volfact_folds(vf) && !sp.blob.empty();
-        used_box_mode = box_mode;
-        char *dbuf = nullptr;
-        if (box_mode) {
-            GF_TRY(smooth_upload(ctx, sp, &dbuf));
-            GF_TRY(launch_mesh_boxes(ctx, n, xr, yr, zr, b->type, hid, nh, mesh_dev, boxes));
-            GF_TRY(smooth_box_prepare(ctx, sp, dbuf, mesh_dev, den, boxes));
-        } else {
-            GF_CUDA_TRY(cudaMemsetAsync(den, 0, sizeof(float) * dev_cells, s));
-        }
+    auto mesh_rest = [&]() -> int {
         // batch order: the deposit's float sums in octree order were faster
         // (2.73 -> 2.34 ms) but put the densest cells of the 5e7-particle
         // cluster 1.04e-5 from an FP64 deposit, past the 1e-5 target
@@ -301,33 +377,55 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
         tm.mark();  // 4
         if (box_mode) {
             GF_TRY(smooth_box_launch(ctx, sp, dbuf, mesh_dev, den, boxes, &oc));
-        } else {
+        } else if (!sp.blob.empty()) {
             MeshBoxes mb;
             mb.dev = boxes;
             mb.trim_last = true;  // den is read only by find_den below
-            GF_TRY(smooth_meshes(ctx, nh, mesh.data(), mesh_dev, den, &oc, &mb));
+            GF_TRY(smooth_launch(ctx, sp, dbuf, mesh_dev, den, &oc, &mb));
         }
         tm.mark();  // 5
         if (o->dens_mesh)
             GF_TRY(launch_find_den(ctx, n, xr, yr, zr, hid, mesh_dev, den, o->dens_mesh,
                                    need_tree ? ctx->last_tree.perm : nullptr));
         tm.mark();  // 6
-    } else {
-        tm.mark();
-        tm.mark();
-        tm.mark();
-    }
+        return GF_OK;
+    };
     // ---- 5. potential
     unsigned long long *counters = nullptr;
-    if (cfg->do_potential) {
+    auto potential = [&]() -> int {
+        if (!cfg->do_potential) return GF_OK;
         if (st && cfg->count_work) {
             GF_TRY(ctx->tmp[4].reserve(128));
             counters = ctx->tmp[4].as<unsigned long long>();
-            GF_CUDA_TRY(cudaMemsetAsync(counters, 0, 16, s));
+            GF_CUDA_TRY(cudaMemsetAsync(counters, 0, 16, ctx->stream));
         }
         const double pf = cfg->potentfact != 0.0 ? cfg->potentfact : physics().potentfact;
         PotentialParams pp = potential_params(cfg->theta2, cfg->ndirect, pf, cfg->add_bg);
-        GF_TRY(launch_self_potential(ctx, ctx->last_tree, b->pstart, pp, o->penergy, o->phi, counters));
+        return launch_self_potential(ctx, ctx->last_tree, b->pstart, pp, o->penergy, o->phi, counters);
+    };
+    if (st || !do_mesh || !need_tree) {
+        GF_TRY(knn());
+        tm.mark();  // 3
+        if (do_mesh) {
+            if (st) GF_TRY(mesh_prepare());
+            GF_TRY(mesh_rest());
+        } else {
+            tm.mark();
+            tm.mark();
+            tm.mark();
+        }
+        GF_TRY(potential());
+    } else {
+        GF_TRY(lanes.fork(0));
+        GF_TRY(lanes.fork(1));
+        lanes.use(0);
+        GF_TRY(mesh_rest());
+        lanes.back();
+        GF_TRY(knn());
+        lanes.use(1);
+        GF_TRY(potential());
+        GF_TRY(lanes.join(0));
+        GF_TRY(lanes.join(1));
     }
     tm.mark();  // 7
     int status = check_device_errors(ctx);
@@ -350,7 +448,7 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
                 if (m.ptype == kMeshOnChip) continue;
                 const int32_t *q = &bx[(size_t)kMeshBoxInts * h];
                 st->mesh_pass_cells += (int64_t)m.nx * len(q[2], q[3]) * len(q[4], q[5]);  // x pass
-                if (used_box_mode) {  // y pass over the evaluation box's x only
+                if (box_mode) {  // y pass over the evaluation box's x only
                     if (q[0] > q[1]) continue;  // nothing deposited: no pass
                     st->mesh_pass_cells += (int64_t)m.ny * len(q[6], q[7]) * len(q[4], q[5]);
                 } else {
@@ -472,31 +570,39 @@ int stage_pass_graph(StageGraph &g) {
     GF_TRY(launch_frames_plan(ctx, nh, cfg->box, cfg->mesh, cfg->do_mesh, g.planned.as<gf_mesh_desc>(), frame_dev,
                               mesh_dev));
     GF_TRY(recentre(ctx, b, hid, frame_dev, cfg->box, xr, yr, zr, pos));
-    if (g.plan.need_tree)
-        GF_TRY(build_tree(ctx, nh, n, b->pstart, pos, cfg->theta2, cfg->q5_asbuilt, &ctx->last_tree, &g.fixed));
-    if (cfg->knn_k > 0)
-        GF_TRY(launch_knn(ctx, ctx->last_tree, b->pstart, pos, cfg->knn_k, o->nearindex, o->dens_sph, nullptr));
+    const bool need_tree = g.plan.need_tree;
+    const double vf = tsc_volfact();
+    GF_TRY(ctx->tmp[3].reserve(sizeof(float) * (size_t)std::max<int64_t>(g.plan.dev_cells, 1)));
+    GF_TRY(ctx->mesh_boxes.reserve(sizeof(int32_t) * kMeshBoxInts * (size_t)std::max(nh, 1)));
+    float *den = ctx->tmp[3].as<float>();
+    int32_t *boxes = ctx->mesh_boxes.as<int32_t>();
+    // as the eager stage: passes over the occupied boxes, only the deposit
+    // boxes zeroed; the tile counts are recounted on the device each replay
+    const bool box_mode = cfg->do_mesh && g.smooth.box_ok && volfact_folds(vf) && !g.smooth.blob.empty();
+    Lanes lanes(ctx, need_tree && cfg->do_mesh);
+    GF_TRY(lanes.open());
     if (cfg->do_mesh) {
-        const int64_t dev_cells = g.plan.dev_cells;
-        GF_TRY(ctx->tmp[3].reserve(sizeof(float) * (size_t)std::max<int64_t>(dev_cells, 1)));
-        float *den = ctx->tmp[3].as<float>();
-        const double vf = tsc_volfact();
-        GF_TRY(ctx->mesh_boxes.reserve(sizeof(int32_t) * kMeshBoxInts * (size_t)std::max(nh, 1)));
-        int32_t *boxes = ctx->mesh_boxes.as<int32_t>();
-        // as the eager stage: passes over the occupied boxes, only the deposit
-        // boxes zeroed; the tile counts are recounted on the device each replay
-        const bool box_mode = g.smooth.box_ok && volfact_folds(vf) && !g.smooth.blob.empty();
+        GF_TRY(lanes.fork(0));
+        lanes.use(0);
         if (box_mode) {
             GF_TRY(launch_mesh_boxes(ctx, n, xr, yr, zr, b->type, hid, nh, mesh_dev, boxes));
             GF_TRY(smooth_box_prepare(ctx, g.smooth, g.smooth_blob.as<char>(), mesh_dev, den, boxes));
         } else {
-            GF_CUDA_TRY(cudaMemsetAsync(den, 0, sizeof(float) * dev_cells, s));
+            GF_CUDA_TRY(cudaMemsetAsync(den, 0, sizeof(float) * g.plan.dev_cells, ctx->stream));
         }
+        lanes.back();
+    }
+    if (need_tree)
+        GF_TRY(build_tree(ctx, nh, n, b->pstart, pos, cfg->theta2, cfg->q5_asbuilt, &ctx->last_tree, &g.fixed));
+    GF_TRY(lanes.fork(0));
+    GF_TRY(lanes.fork(1));
+    if (cfg->do_mesh) {
+        lanes.use(0);
         GF_TRY(launch_stage_deposit(ctx, n, xr, yr, zr, b->mass, b->type, hid, b->pstart,
-                                    g.plan.need_tree ? ctx->last_tree.perm : nullptr,
-                                    g.plan.need_tree ? ctx->last_tree.phalo : nullptr, nh, mesh_dev, den, vf,
+                                    need_tree ? ctx->last_tree.perm : nullptr,
+                                    need_tree ? ctx->last_tree.phalo : nullptr, nh, mesh_dev, den, vf,
                                     box_mode ? nullptr : boxes));
-        if (!volfact_folds(vf)) GF_TRY(launch_scale(ctx, den, dev_cells, vf));
+        if (!volfact_folds(vf)) GF_TRY(launch_scale(ctx, den, g.plan.dev_cells, vf));
         if (box_mode) {
             GF_TRY(smooth_box_launch(ctx, g.smooth, g.smooth_blob.as<char>(), mesh_dev, den, boxes));
         } else {
@@ -507,14 +613,19 @@ int stage_pass_graph(StageGraph &g) {
         }
         if (o->dens_mesh)
             GF_TRY(launch_find_den(ctx, n, xr, yr, zr, hid, mesh_dev, den, o->dens_mesh,
-                                   g.plan.need_tree ? ctx->last_tree.perm : nullptr));
+                                   need_tree ? ctx->last_tree.perm : nullptr));
+        lanes.back();
     }
+    if (cfg->knn_k > 0)
+        GF_TRY(launch_knn(ctx, ctx->last_tree, b->pstart, pos, cfg->knn_k, o->nearindex, o->dens_sph, nullptr));
     if (cfg->do_potential) {
         const double pf = cfg->potentfact != 0.0 ? cfg->potentfact : physics().potentfact;
         PotentialParams pp = potential_params(cfg->theta2, cfg->ndirect, pf, cfg->add_bg);
+        lanes.use(1);
         GF_TRY(launch_self_potential(ctx, ctx->last_tree, b->pstart, pp, o->penergy, o->phi, nullptr));
     }
-    return GF_OK;
+    GF_TRY(lanes.join(0));
+    return lanes.join(1);
 }
 
 void release_graph(StageGraph &g) {

@@ -69,7 +69,7 @@ struct Build {
 // few particles are left, and read every one of those from memory, so the
 // lower levels, most of a small batch's, go to shared memory: the stage on a
 // halo of 120 took 0.32 ms, now 0.24; on one of 131,072 1.59, now 1.40; a
-// replayed graph of 64 halos 0.70, now 0.59; four gradients of one million
+// replayed graph of 64 halos 0.75, now 0.66; four gradients of one million
 // particles, whose tree was their largest part, 1.35, now 1.16.  256 particles
 // (two buffers, 10 KB) leave 20 warps per SM; the pass is bound by the chain
 // of shuffles of a node (log2 32 steps for 17 values), 0.42 ms for 6 M

@@ -1,0 +1,122 @@
+"""The stage's parts on side streams of the context against the same parts one
+after the other (a run with phase times), on streams of several priorities and
+in stream order around a captured pass."""
+import ctypes
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+from galaxyfinder_b200 import _lib, batch, synth
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("nearindex", "dens_sph", "dens_mesh", "penergy", "phi")
+
+
+def _close(a, b):
+    """Searches are exact; mesh cells and node moments are float and double
+    sums in no fixed order (the bars of the captured pass's test)."""
+    for f in ("nearindex", "dens_sph"):
+        np.testing.assert_array_equal(a[f], b[f])
+    assert np.abs(a["dens_mesh"] - b["dens_mesh"]).max() <= 2e-6 * np.abs(b["dens_mesh"]).max()
+    assert (np.abs(a["phi"] - b["phi"]) / np.abs(b["phi"])).max() <= 1e-6
+
+
+def _get(out):
+    return {f: getattr(out, f).cpu().numpy() for f in FIELDS}
+
+
+def _case(cuda_device, nhalo=24, nmax=30000, seed=5):
+    hb = synth.catalogue(seed=seed, nhalo=nhalo, nmin=60, nmax=nmax, straddle_frac=0.2)
+    return hb, batch.DeviceBatch.from_halobatch(hb)
+
+
+@pytest.mark.parametrize("mesh", [dict(mode=_lib.MESH_POW2), dict(mode=_lib.MESH_FIXED, nfixed=48),
+                                  dict(mode=_lib.MESH_FIXED, nfixed=64)],
+                         ids=["pow2", "direct", "fixed64"])
+@pytest.mark.parametrize("onchip", [0, 1])
+def test_beside_equals_in_a_row(cuda_device, mesh, onchip):
+    hb, db = _case(cuda_device)
+    cfg = batch.stage_config(mesh=batch.mesh_rule(rg=2.0, rg_in_cells=True, **mesh), mesh_onchip=bool(onchip))
+    ctx = batch.Context(0)
+    try:
+        for n in (0, -1, 0):  # the context's side streams follow its stream's priority
+            s = torch.cuda.Stream(priority=n)
+            _lib.check(_lib.lib().gf_ctx_set_stream(ctx.handle, ctypes.c_void_p(s.cuda_stream)))
+            out = batch.StageBuffers(hb.n, 32, db.x.device, keep_phi=True)
+            torch.cuda.synchronize()
+            batch.stage_run(ctx, db, cfg, out)
+            got = _get(out)
+            for f in FIELDS:
+                getattr(out, f).zero_()
+            torch.cuda.synchronize()
+            batch.stage_run(ctx, db, cfg, out, stats=True)
+            _close(got, _get(out))
+    finally:
+        ctx.close()
+
+
+def test_replays_in_stream_order(cuda_device):
+    """Work queued on the context's stream after a replay sees all its
+    outputs, and the next replay leaves what was copied alone."""
+    hb, db = _case(cuda_device)
+    s = torch.cuda.Stream()
+    ctx = batch.Context(0, s)
+    out = batch.StageBuffers(hb.n, 32, db.x.device, keep_phi=True)
+    cfg = batch.stage_config()
+    g = batch.StageGraph(ctx, db, cfg, out)
+    ref = _get(out)
+    copies = []
+    with torch.cuda.stream(s):
+        for _ in range(4):
+            for f in FIELDS:
+                getattr(out, f).zero_()
+            g.launch()
+            copies.append({f: getattr(out, f).clone() for f in FIELDS})
+    g.sync()
+    for c in copies:
+        _close({f: t.cpu().numpy() for f, t in c.items()}, ref)
+    g.close()
+    ctx.close()
+
+
+def test_contexts_in_threads(cuda_device):
+    cases = [_case(cuda_device, nhalo=h, nmax=m, seed=h) for h, m in ((1, 200), (16, 20000), (40, 5000))]
+    cfg = batch.stage_config()
+    refs, got = [], [None] * len(cases)
+    for hb, db in cases:
+        ctx = batch.Context(0)
+        refs.append(_get(batch.stage_run(ctx, db, cfg, batch.StageBuffers(hb.n, 32, db.x.device, keep_phi=True),
+                                         stats=True)[0]))
+        ctx.close()
+
+    def work(i):
+        hb, db = cases[i]
+        ctx = batch.Context(0, torch.cuda.Stream(priority=-(i % 2)))
+        for _ in range(5):
+            got[i] = batch.stage_run(ctx, db, cfg, batch.StageBuffers(hb.n, 32, db.x.device, keep_phi=True))
+        ctx.close()
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(cases))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for ref, out in zip(refs, got):
+        _close(_get(out), ref)
+
+
+def test_a_refused_run_leaves_the_context_usable(cuda_device):
+    hb, db = _case(cuda_device, nhalo=4, nmax=2000)
+    ctx = batch.Context(0)
+    out = batch.StageBuffers(hb.n, 32, db.x.device, keep_phi=True)
+    cfg = batch.stage_config()
+    ref = _get(batch.stage_run(ctx, db, cfg, out, stats=True)[0])
+    bad = batch.stage_config(knn_k=33)  # refused after the mesh part was queued
+    with pytest.raises(_lib.GFError):
+        batch.stage_run(ctx, db, bad, out)
+    _close(_get(batch.stage_run(ctx, db, cfg, out)), ref)
+    ctx.close()
