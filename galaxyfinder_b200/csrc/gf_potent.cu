@@ -23,27 +23,35 @@
 //     Opening decisions are those of an FP64 walk of the same tree: FP32
 //     distances decide only outside a margin above their rounding error, and
 //     what falls inside it is decided by the reference's FP64 test;
-//   * accepted cells and the loose particles of opened nodes are gathered, one
-//     per lane, into shared-memory tiles of 32 with one array per field, each
-//     entry with its lane mask, and a full tile is evaluated: lane = target,
-//     two entries per instruction (packed FP32 pairs, whose 16-byte loads
-//     serve four entries), inactive lanes by a zero 1/r.
+//   * accepted cells and the loose particles of opened nodes are gathered in
+//     lists, each entry with its lane mask, and 32 entries are evaluated at
+//     once: lane = entry, its fields in registers, against all 32 targets,
+//     two per instruction (packed FP32 pairs; a 16-byte load of one coordinate
+//     serves four targets), inactive targets by a zero 1/r.  Every lane has
+//     32 partial sums; each kFlush tiles they go through shared memory to the
+//     targets' lanes, which add them up with Kahan compensation.
 // The terms are FP32 evaluated from position differences with two roundings
-// (the node centre is held as the sum of two floats) and summed with Kahan
-// compensation in two interleaved sums.
+// (the node centre is held as the sum of two floats).  Against an FP64 walk of
+// the same tree phi has 2.63e-8 to 2.81e-8 rms (1.4e5 to 1e6 particles), as
+// with one Kahan sum per target; without the Kahan step, or with eight tiles
+// between two additions, up to 2.9e-8.
 //
-// What bounds it: the FP32 pipe.  A cell costs 24 FP32 operations per lane
-// and a particle 10; a 131072-particle NFW halo at theta2 = 0.5 has, per
-// warp, 937 cells (23 of 32 lanes) and 1268 particles (12 of 32), about 35 k
-// of its cycles.  The lockstep walk that this replaces (every lane at its own
-// next node, the warp at the smallest) spent about 60 issue slots on a cell
-// and 17 on a particle, most of them on the walk and on FP64 differences.
-// Measured, lockstep -> tiled: 4096 halos (7.0 M particles) 13.3 -> 9.2 ms,
-// 300,007 particles at theta2 = 0.25 1.93 -> 1.26 ms, 131,072 at 0.5 0.46 ->
-// 0.30 ms, 64 small halos 0.31 -> 0.09 ms.  The FP32 pipe is then 46 % busy and
-// 61 % of the issue slots are used; the rest is the latency of the expansion
-// (its loads and shuffles).  A stack of 320 entries lets fewer nodes be popped
-// at once (9.4 ms), one of 768 costs resident warps (9.9 ms).
+// What bounds it: issue slots (62 % used, 27 k instructions per warp) and, at 5
+// blocks per SM (96 registers, of which 32 are sums and 26 a cell's fields),
+// the latency of the expansion's loads and shuffles; the FP32 pipe is 46 %
+// busy.  A 131072-particle NFW halo at theta2 = 0.5 has, per warp, 937 cells
+// (23 of 32 lanes) and 1268 particles (12 of 32).  With lane = target and the
+// entries in shared memory, 13 floats of every cell were loaded by all lanes:
+// 70 % of the shared-memory cycles, 35 k instructions.
+// Measured, a lockstep walk (every lane at its own next node, the warp at the
+// smallest) -> lane = target -> lane = entry: 4096 halos (6.1 M particles)
+// 13.3 -> 9.2 -> 8.7 ms, 300,007 particles at theta2 = 0.25 1.93 -> 1.27 ->
+// 1.07 ms, 256 halos (247 k) 0.60 -> 0.42 -> 0.39, 131,072 at 0.5 0.46 -> 0.30
+// -> 0.32 ms, 64 small halos 0.31 -> 0.085 -> 0.095 ms (the last tiles of a
+// warp are partly filled and cost as much as full ones).  4 blocks per SM: 9.3
+// ms, 6 (80 registers, spilled): 10.6; a stack of 320 entries lets fewer nodes
+// be popped at once: 9.0 ms; 64 threads per block: 8.7, but 64 small halos
+// 0.136 ms.
 #include <float.h>
 #include <limits.h>
 #include <math.h>
@@ -112,43 +120,28 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
     return r;
 }
 
-// Two Kahan sums side by side; nc is the negated compensation.  The terms
-// arrive as t * inv, folded into the first addition.
+// ---- per-warp shared memory of bh_kernel
+constexpr int kStack = 416;  // (node, lanes) still to visit
+constexpr int kDeal = 4;     // nodes per part before they are dealt out
+constexpr int kFlush = 4;    // tiles between two additions to the targets' sums
+struct __align__(16) BhWarp {
+    float target[3][32];  // positions of the warp's targets
+    uint2 cells[64];      // accepted (node, lanes) waiting for a tile
+    uint2 leaf[64];       // loose (particle, lanes) waiting for a tile
+    uint2 stack[kStack];
+    float sums[32][36];   // a lane's terms of every target, 16 bytes beside the banks of the next lane's
+};
+
+// Two Kahan sums side by side; nc is the negated compensation.
 struct Kahan2 {
     f2 s, nc;
-    __device__ __forceinline__ void add(f2 t, f2 inv, f2 minus1) {
-        const f2 y = f2_fma(t, inv, nc);
+    __device__ __forceinline__ void add(f2 t, f2 minus1) {
+        const f2 y = f2_add(t, nc);
         const f2 n = f2_add(s, y);
         nc = f2_add(y, f2_fma(n, minus1, s));  // y - (n - s)
         s = n;
     }
 };
-
-// ---- per-warp shared memory of bh_kernel
-constexpr int kCellFields = 13;  // -centre high and low parts, mass, six moments
-constexpr int kStack = 416;      // (node, lanes) still to visit
-constexpr int kDeal = 4;         // nodes per part before they are dealt out
-struct __align__(16) BhWarp {
-    float cell[kCellFields][32];
-    float leaf[4][64];   // -x, -y, -z, mass of a particle; a tile of 32 and what waits for the next
-    unsigned leaf_mask[64];
-    uint2 cells[64];     // accepted (node, lanes) waiting for a tile
-    uint2 stack[kStack];
-};
-
-// Bit l of row e (lane e's v) becomes bit e of row l: each lane receives, for
-// every tile entry, whether it takes part (five butterfly steps).
-__device__ __forceinline__ unsigned transpose_bits(unsigned v) {
-    const int lane = threadIdx.x & 31;
-    unsigned low = 0x0000ffffu;
-#pragma unroll
-    for (int j = 16; j; j >>= 1) {
-        const unsigned o = __shfl_xor_sync(0xffffffffu, v, j);
-        v = (lane & j) ? (v & ~low) | ((o & ~low) >> j) : (v & low) | ((o & low) << j);
-        low ^= low << (j >> 1);
-    }
-    return v;
-}
 
 // The walk one node at a time over the preorder nodes [i, end): every lane at
 // its own next node, the warp at the smallest of them (taking part: lanes
@@ -230,101 +223,101 @@ bh_kernel(int64_t ntarget, const float4 *__restrict__ tpos, const int32_t *__res
             h = thalo[t];
             P = tpos[t];
         }
-        const f2 px = f2_pack(P.x, P.x), py = f2_pack(P.y, P.y), pz = f2_pack(P.z, P.z);
-        Kahan2 acc{0ull, 0ull};
-        float aside = 0.f;  // subtrees walked one node at a time
+        W.target[0][lane] = P.x;
+        W.target[1][lane] = P.y;
+        W.target[2][lane] = P.z;
+        __syncwarp();
+        f2 acc[16];  // this lane's terms of the targets 2i, 2i + 1
+#pragma unroll
+        for (int i = 0; i < 16; i++) acc[i] = 0ull;
+        Kahan2 total{0ull, 0ull};  // of this lane's target
+        float aside = 0.f;   // subtrees walked one node at a time
         int cn = 0, ln = 0;  // waiting cells and particles (warp-uniform)
+        int tiles = 0;
+        auto flush = [&]() {
+#pragma unroll
+            for (int g = 0; g < 8; g++) {
+                *reinterpret_cast<ulonglong2 *>(&W.sums[lane][4 * g]) = make_ulonglong2(acc[2 * g], acc[2 * g + 1]);
+                acc[2 * g] = acc[2 * g + 1] = 0ull;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < 32; r += 2) total.add(f2_pack(W.sums[r][lane], W.sums[r + 1][lane]), minus1);
+            __syncwarp();
+            tiles = 0;
+        };
+        auto quad = [&](int a, int g) { return *reinterpret_cast<const ulonglong2 *>(&W.target[a][4 * g]); };
 
-        // a tile of up to 32 cells, taken from the end of the waiting list
+        // a tile of up to 32 cells, taken from the end of the waiting list: a lane each
         auto eval_cells = [&](int n) {
             cn -= n;
-            const bool have = lane < n;
-            const uint2 c = have ? W.cells[cn + lane] : make_uint2(0u, 0u);
+            const uint2 c = lane < n ? W.cells[cn + lane] : make_uint2(0u, 0u);
+            const unsigned on = c.y;
             float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a, m = a, q = a;
-            if (have) {
+            if (lane < n) {
                 const float4 *w = reinterpret_cast<const float4 *>(wnodes + c.x);
                 a = __ldg(w);
                 b = __ldg(w + 2);
                 m = __ldg(w + 3);
                 q = __ldg(w + 4);
             }
-            W.cell[0][lane] = -a.x;
-            W.cell[1][lane] = -a.y;
-            W.cell[2][lane] = -a.z;
-            W.cell[3][lane] = -b.x;
-            W.cell[4][lane] = -b.y;
-            W.cell[5][lane] = -b.z;
-            W.cell[6][lane] = b.w;
-            W.cell[7][lane] = m.x;
-            W.cell[8][lane] = m.y;
-            W.cell[9][lane] = m.z;
-            W.cell[10][lane] = m.w;
-            W.cell[11][lane] = q.x;
-            W.cell[12][lane] = q.y;
-            unsigned on = transpose_bits(c.y);
-            __syncwarp();
-#pragma unroll 1
-            for (int e = 0; e < n; e += 4, on >>= 4) {
-                ulonglong2 f[kCellFields];
+            auto dup = [](float v) { return f2_pack(v, v); };
+            const f2 hx = dup(-a.x), hy = dup(-a.y), hz = dup(-a.z), lx = dup(-b.x), ly = dup(-b.y), lz = dup(-b.z);
+            const f2 mass = dup(b.w), txx = dup(m.x), tyy = dup(m.y), tzz = dup(m.z), txy = dup(m.w);
+            const f2 txz = dup(q.x), tyz = dup(q.y);
 #pragma unroll
-                for (int i = 0; i < kCellFields; i++)
-                    f[i] = *reinterpret_cast<const ulonglong2 *>(&W.cell[i][e]);
+            for (int g = 0; g < 8; g++) {
+                const ulonglong2 X = quad(0, g), Y = quad(1, g), Z = quad(2, g);
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
-                    auto F = [&](int i) { return u ? f[i].y : f[i].x; };
-                    const f2 dx = f2_add(f2_add(px, F(0)), F(3));
-                    const f2 dy = f2_add(f2_add(py, F(1)), F(4));
-                    const f2 dz = f2_add(f2_add(pz, F(2)), F(5));
+                    const f2 dx = f2_add(f2_add(u ? X.y : X.x, hx), lx);
+                    const f2 dy = f2_add(f2_add(u ? Y.y : Y.x, hy), ly);
+                    const f2 dz = f2_add(f2_add(u ? Z.y : Z.x, hz), lz);
                     const f2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
                     float ra, rb;
                     f2_unpack(r2, ra, rb);
-                    ra = (on & (1u << (2 * u))) ? rsqrt_ftz(ra) : 0.f;
-                    rb = (on & (2u << (2 * u))) ? rsqrt_ftz(rb) : 0.f;
+                    ra = (on & (1u << (4 * g + 2 * u))) ? rsqrt_ftz(ra) : 0.f;
+                    rb = (on & (2u << (4 * g + 2 * u))) ? rsqrt_ftz(rb) : 0.f;
                     const f2 inv = f2_pack(ra, rb), inv2 = f2_mul(inv, inv), inv4 = f2_mul(inv2, inv2);
                     // d.Q.d over the upper triangle (off-diagonals doubled)
-                    const f2 q1 = f2_fma(F(7), dx, f2_fma(F(10), dy, f2_mul(F(11), dz)));
-                    const f2 q2 = f2_fma(F(8), dy, f2_mul(F(12), dz));
-                    const f2 qd = f2_fma(dx, q1, f2_fma(dy, q2, f2_mul(f2_mul(F(9), dz), dz)));
-                    acc.add(f2_fma(qd, inv4, F(6)), inv, minus1);
+                    const f2 q1 = f2_fma(txx, dx, f2_fma(txy, dy, f2_mul(txz, dz)));
+                    const f2 q2 = f2_fma(tyy, dy, f2_mul(tyz, dz));
+                    const f2 qd = f2_fma(dx, q1, f2_fma(dy, q2, f2_mul(f2_mul(tzz, dz), dz)));
+                    acc[2 * g + u] = f2_fma(f2_fma(qd, inv4, mass), inv, acc[2 * g + u]);
                 }
             }
-            __syncwarp();
+            __syncwarp();  // the list is read
+            if (++tiles == kFlush) flush();
         };
-        // the first n (up to 32) waiting particles
+        // up to 32 particles from the end of the waiting list
         auto eval_leaf = [&](int n) {
-            if (lane >= n && lane < ((n + 3) & ~3)) {  // pad to a multiple of four
-                W.leaf[3][lane] = 0.f;
-                W.leaf_mask[lane] = 0u;
-            }
-            unsigned on = transpose_bits(W.leaf_mask[lane]);
-            __syncwarp();
-#pragma unroll 2
-            for (int e = 0; e < n; e += 4, on >>= 4) {
-                const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(&W.leaf[0][e]);
-                const ulonglong2 Y = *reinterpret_cast<const ulonglong2 *>(&W.leaf[1][e]);
-                const ulonglong2 Z = *reinterpret_cast<const ulonglong2 *>(&W.leaf[2][e]);
-                const ulonglong2 M = *reinterpret_cast<const ulonglong2 *>(&W.leaf[3][e]);
+            ln -= n;
+            const uint2 c = lane < n ? W.leaf[ln + lane] : make_uint2(0u, 0u);
+            const unsigned on = c.y;
+            float4 S = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (lane < n) S = __ldg(spos + c.x);
+            const f2 sx = f2_pack(-S.x, -S.x), sy = f2_pack(-S.y, -S.y), sz = f2_pack(-S.z, -S.z);
+            const f2 mass = f2_pack(S.w, S.w);
+            const unsigned any = __reduce_or_sync(0xffffffffu, on);
+#pragma unroll
+            for (int g = 0; g < 8; g++) {
+                if (!(any & (15u << (4 * g)))) continue;  // four targets that opened none of these leaves
+                const ulonglong2 X = quad(0, g), Y = quad(1, g), Z = quad(2, g);
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
-                    const f2 dx = f2_add(px, u ? X.y : X.x), dy = f2_add(py, u ? Y.y : Y.x);
-                    const f2 dz = f2_add(pz, u ? Z.y : Z.x);
+                    const f2 dx = f2_add(u ? X.y : X.x, sx), dy = f2_add(u ? Y.y : Y.x, sy);
+                    const f2 dz = f2_add(u ? Z.y : Z.x, sz);
                     const f2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
                     float ra, rb;
                     f2_unpack(r2, ra, rb);
                     // ost.c:186-191: particle terms with r > 0
-                    ra = (on & (1u << (2 * u))) && ra > 0.f ? rsqrt_ftz(ra) : 0.f;
-                    rb = (on & (2u << (2 * u))) && rb > 0.f ? rsqrt_ftz(rb) : 0.f;
-                    acc.add(u ? M.y : M.x, f2_pack(ra, rb), minus1);
+                    ra = (on & (1u << (4 * g + 2 * u))) && ra > 0.f ? rsqrt_ftz(ra) : 0.f;
+                    rb = (on & (2u << (4 * g + 2 * u))) && rb > 0.f ? rsqrt_ftz(rb) : 0.f;
+                    acc[2 * g + u] = f2_fma(mass, f2_pack(ra, rb), acc[2 * g + u]);
                 }
             }
             __syncwarp();
-            ln -= n;
-            if (lane < ln) {  // the rest (at most 31) move to the front
-#pragma unroll
-                for (int i = 0; i < 4; i++) W.leaf[i][lane] = W.leaf[i][n + lane];
-                W.leaf_mask[lane] = W.leaf_mask[n + lane];
-            }
-            __syncwarp();
+            if (++tiles == kFlush) flush();
         };
 
         // ---- one halo of the warp's targets at a time (nearly always one)
@@ -467,35 +460,34 @@ bh_kernel(int64_t ntarget, const float4 *__restrict__ tpos, const int32_t *__res
                 if (am) W.cells[cn + __popc(ab & lt)] = make_uint2((unsigned)node, am);
                 cn += __popc(ab);
                 __syncwarp();
-                if (cn >= 32) eval_cells(32);
+                while (cn >= 32 || (top == 0 && cn > 0)) eval_cells(min(cn, 32));
                 // ---- loose particles of the opened nodes
-                for (unsigned lb = __ballot_sync(0xffffffffu, om != 0u && lk.w > 0); lb; lb &= lb - 1) {
+                int o = 0;
+                for (unsigned lb = __ballot_sync(0xffffffffu, om != 0u && lk.w > 0);;) {
+                    if (ln >= 32 || (!lb && top == 0 && ln > 0)) {
+                        eval_leaf(min(ln, 32));
+                        continue;
+                    }
+                    if (!lb) break;
                     const int src = __ffs(lb) - 1;
                     const int l0 = __shfl_sync(0xffffffffu, lk.z, src), lc = __shfl_sync(0xffffffffu, lk.w, src);
                     const unsigned lm = __shfl_sync(0xffffffffu, om, src);
-                    for (int o = 0; o < lc; o += 32) {
-                        const int k = min(32, lc - o);
-                        if (lane < k) {
-                            const float4 S = __ldg(spos + l0 + o + lane);
-                            W.leaf[0][ln + lane] = -S.x;
-                            W.leaf[1][ln + lane] = -S.y;
-                            W.leaf[2][ln + lane] = -S.z;
-                            W.leaf[3][ln + lane] = S.w;
-                            W.leaf_mask[ln + lane] = lm;
-                        }
-                        ln += k;
-                        __syncwarp();
-                        if (ln >= 32) eval_leaf(32);
+                    const int k = min(32, lc - o);
+                    if (lane < k) W.leaf[ln + lane] = make_uint2((unsigned)(l0 + o + lane), lm);
+                    ln += k;
+                    o += 32;
+                    if (o >= lc) {
+                        lb &= lb - 1;
+                        o = 0;
                     }
+                    __syncwarp();
                 }
             }
         }
-        if (cn > 0) eval_cells(cn);
-        if (ln > 0) eval_leaf(ln);
-        // the two sums and their compensations
-        float s0, s1, c0, c1;
-        f2_unpack(acc.s, s0, s1);
-        f2_unpack(acc.nc, c0, c1);
+        flush();
+        float s0, s1, c0, c1;  // the two sums and their compensations
+        f2_unpack(total.s, s0, s1);
+        f2_unpack(total.nc, c0, c1);
         double sum = (double)aside - (((double)s0 + (double)s1) + ((double)c0 + (double)c1));
         if (together) {
             double *red = reinterpret_cast<double *>(W.stack);  // 32 of each part, done with its stack
@@ -556,8 +548,8 @@ int launch_bh(gf_ctx *ctx, int64_t ntarget, const float4 *tpos, const int32_t *t
     // few targets: a block's warps divide the nodes of 32 targets among them
     // instead of leaving most of the SMs' warps without work.  Above half of
     // the resident warps the dealing costs more than it fills (more steps
-    // with less than 32 nodes each): 36,001 targets 165 -> 131 us, a batch of
-    // 64 small halos 150 -> 90, but 131,072 targets 305 -> 345.
+    // with less than 32 nodes each): 36,001 targets 139 -> 114 us, a batch of
+    // 64 small halos 257 -> 93, but 131,072 targets 313 -> 386.
     const bool together = 2 * groups <= wave * warps;
     int64_t grid = together ? groups : (groups + warps - 1) / warps;
     if (!together) {
