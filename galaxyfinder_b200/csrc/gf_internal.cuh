@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <string>
@@ -176,6 +177,18 @@ namespace gf {
 
 // The context used by the drop-in (reference-signature) entry points.
 gf_ctx *default_ctx();
+
+// Particles per warp, a multiple of 32, for kernels whose warps take runs of
+// consecutive particles (256 threads per block), and their grid: one step of 32
+// up to 1024 warps, then four (fewer updates of a large halo's words), then
+// what fills the SMs' warps once.
+inline int64_t warp_run(int64_t n) {
+    const int64_t steps = (n + 31) / 32, warps = (int64_t)sm_count() * 64;
+    return 32 * std::max<int64_t>(std::min<int64_t>(4, steps / 1024 + 1), (steps + warps - 1) / warps);
+}
+inline unsigned warp_run_grid(int64_t n, int64_t run) {
+    return (unsigned)std::max<int64_t>(1, ((n + run - 1) / run + 7) / 8);
+}
 
 // Reads and clears the device error word; maps set bits to a status.
 int check_device_errors(gf_ctx *ctx);

@@ -740,6 +740,7 @@ knn_bucket_kernel(int64_t n, int k, const float4 *__restrict__ pos, const int32_
 // Nodes of the walk staged per warp in shared memory (GF_KNNB_WIN at a time;
 // 0: every node is read from global memory through L1).  A smaller window
 // leaves room for more resident warps.
+#if GF_KNN_ALGO == 2
 constexpr int kWin = GF_KNNB_WIN;
 constexpr int kFBucketWarpBytes = 32 * 32 * 8 + kWin * (int)sizeof(KnnNode) + 32 * 16 + 32 * 4 +
                                   32 * GF_KNNB_QUEUE * 8;
@@ -1217,6 +1218,8 @@ knn_fbucket_kernel(int64_t n, int k, const float4 *__restrict__ pos, const int32
         }
     }
 }
+
+#endif  // GF_KNN_ALGO == 2
 
 // ------------------------------------------------- bucket kNN, sorted lists
 // As the float-key bucket kernel above (a warp walks the tree once for 32

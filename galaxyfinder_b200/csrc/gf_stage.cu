@@ -550,7 +550,6 @@ int stage_pass_graph(StageGraph &g) {
     gf_stage_out *o = &g.o;
     const int64_t n = b->nparticle;
     const int32_t nh = b->nhalo;
-    cudaStream_t s = ctx->stream;
     GF_TRY(ctx->hid.reserve(sizeof(int32_t) * std::max<int64_t>(n, 1)));
     int32_t *hid = ctx->hid.as<int32_t>();
     GF_TRY(compute_hid(ctx, nh, n, b->pstart, hid));

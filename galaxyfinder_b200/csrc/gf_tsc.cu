@@ -98,38 +98,91 @@ __global__ void tsc_deposit_kernel(int64_t n, const double *__restrict__ x,
 // deposited particles (deposit box) and of every particle (evaluation box) of
 // each device-memory mesh, with the same stencils as the deposit.  The
 // box-restricted mesh stage zeroes only the deposit boxes from them.
-__global__ void mesh_box_kernel(int64_t n, const double *__restrict__ x, const double *__restrict__ y,
+// As extent_kernel: a warp keeps the ranges of its current halo over a run of
+// consecutive particles.  Bound by the 28 bytes of a particle: with a warp
+// reduction and an update for every 32 particles, and a halo's descriptor and
+// the positions loaded one after the other, 6.1 M particles took 246 us, now
+// 130; 131,072 of one halo 35, now 16.
+constexpr int kBoxBatch = 4;
+
+__global__ void __launch_bounds__(256) mesh_box_kernel(int64_t n, const double *__restrict__ x, const double *__restrict__ y,
                                 const double *__restrict__ z, const int32_t *__restrict__ type,
                                 const int32_t *__restrict__ hid, const gf_mesh_desc *__restrict__ mesh,
-                                int32_t *__restrict__ boxes) {
-    // whole warps step together (the box update reduces over the warp)
-    for (int64_t t0 = blockIdx.x * (int64_t)blockDim.x; t0 < n; t0 += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t p = t0 + threadIdx.x;
-        int hb = -1;
-        bool dep = false;
-        int c[6] = {0, 0, 0, 0, 0, 0};
-        if (p < n) {
-            const int h = hid ? hid[p] : 0;
-            const gf_mesh_desc m = mesh[h];
-            if (m.ptype != kMeshOnChip) {
+                                int32_t *__restrict__ boxes, int64_t run) {
+    const int lane = threadIdx.x & 31;
+    const int64_t a0 = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * run;
+    const int64_t a1 = min(n, a0 + run);
+    int cur = -1;  // halo of the ranges, warp-uniform
+    gf_mesh_desc m{};
+    int r[12];  // minima at even places: deposited, then all
+    auto clear = [&]() {
+#pragma unroll
+        for (int i = 0; i < 12; i++) r[i] = i & 1 ? INT_MIN : INT_MAX;
+    };
+    auto flush = [&]() {
+        if (cur < 0) return;
+#pragma unroll
+        for (int i = 0; i < 12; i++)
+            r[i] = i & 1 ? __reduce_max_sync(0xffffffffu, r[i]) : __reduce_min_sync(0xffffffffu, r[i]);
+        if (lane == 0) {
+            int32_t *b = boxes + (int64_t)kMeshBoxInts * cur;
+#pragma unroll
+            for (int i = 0; i < 12; i += 2) {
+                // a plain read first: most warps of a large halo widen nothing
+                if (r[i] < __ldcg(b + i)) atomicMin(b + i, r[i]);
+                if (r[i + 1] > __ldcg(b + i + 1)) atomicMax(b + i + 1, r[i + 1]);
+            }
+        }
+        clear();
+    };
+    clear();
+    for (int64_t b = a0; b < a1; b += 32 * kBoxBatch) {
+        double c[kBoxBatch][3];
+        int h[kBoxBatch], ty[kBoxBatch];
+#pragma unroll
+        for (int u = 0; u < kBoxBatch; u++) {
+            const int64_t p = b + 32 * u + lane;
+            const bool valid = p < a1;
+            h[u] = valid ? (hid ? hid[p] : 0) : -1;
+            c[u][0] = valid ? x[p] : 0.0;
+            c[u][1] = valid ? y[p] : 0.0;
+            c[u][2] = valid ? z[p] : 0.0;
+            ty[u] = valid && type ? type[p] : GF_TYPE_DM;
+        }
+#pragma unroll
+        for (int u = 0; u < kBoxBatch; u++) {
+            for (unsigned todo = __ballot_sync(0xffffffffu, h[u] >= 0); todo;) {
+                const int hg = __shfl_sync(0xffffffffu, h[u], __ffs(todo) - 1);
+                todo &= ~__ballot_sync(0xffffffffu, h[u] == hg);
+                if (hg != cur) {
+                    flush();
+                    cur = hg;
+                    m = mesh[hg];
+                }
+                if (h[u] != hg || m.ptype == kMeshOnChip) continue;
                 TscStencil s;
                 float xd1, yd1, zd1;
-                tsc_cells(x[p], y[p], z[p], m, s, xd1, yd1, zd1);
-                if (tsc_in_mesh(s, m)) {  // particles outside are flagged by the deposit and findDen
-                    hb = h;
-                    dep = m.ptype == GF_TYPE_ALL || (type ? type[p] : GF_TYPE_DM) == m.ptype;
-                    c[0] = (int)s.i[0] - 1; c[1] = (int)s.i[0] + 1;
-                    c[2] = (int)s.j[0] - 1; c[3] = (int)s.j[0] + 1;
-                    c[4] = (int)s.k[0] - 1; c[5] = (int)s.k[0] + 1;
+                tsc_cells(c[u][0], c[u][1], c[u][2], m, s, xd1, yd1, zd1);
+                if (!tsc_in_mesh(s, m)) continue;  // particles outside are flagged by the deposit and findDen
+                const int q[3] = {(int)s.i[0], (int)s.j[0], (int)s.k[0]};
+                const bool dep = m.ptype == GF_TYPE_ALL || ty[u] == m.ptype;
+#pragma unroll
+                for (int a = 0; a < 3; a++) {
+                    if (dep) {
+                        r[2 * a] = min(r[2 * a], q[a] - 1);
+                        r[2 * a + 1] = max(r[2 * a + 1], q[a] + 1);
+                    }
+                    r[6 + 2 * a] = min(r[6 + 2 * a], q[a] - 1);
+                    r[7 + 2 * a] = max(r[7 + 2 * a], q[a] + 1);
                 }
             }
         }
-        box_update(boxes, hb, dep, c);
     }
+    flush();
 }
 
 // ---------------------------------------------------------------- tiled deposit
-// The deposit through shared-memory tiles.  A block takes kTileChunk
+// The deposit through shared-memory tiles.  A block takes up to kTileChunk
 // consecutive particles in octree order (spatial neighbours; the halos'
 // particle ranges are the batch's, so a chunk splits into halo segments at
 // pstart).  For each segment the block reduces the cell box its stencils
@@ -140,6 +193,11 @@ __global__ void mesh_box_kernel(int64_t n, const double *__restrict__ x, const d
 // global atomic, as in tsc_deposit_kernel.  The weights are the same; the
 // float sums run in two levels (tile, then mesh), in no fixed order.  The
 // occupied boxes are widened once per segment.
+// Bound by latency: the tile's float atomics are compare-and-swap loops, with
+// barriers between a segment's steps.  Chunks shrink to a particle per thread
+// where there are less than four full ones per SM: with 2048 throughout 131,072
+// particles ran on 64 SMs, 77 us, now 31; 247 k in 256 halos 72, now 40; 46 k
+// in 64 halos 65, now 20 (with at least 512: 38, 44 and 27).
 constexpr int kTileThreads = 256;
 constexpr int kTileChunk = 2048;
 
@@ -183,11 +241,11 @@ tsc_tile_deposit_kernel(int64_t n, const double *__restrict__ x, const double *_
                         const int32_t *__restrict__ type, const int64_t *__restrict__ pstart,
                         const int32_t *__restrict__ order, const int32_t *__restrict__ thalo,
                         const gf_mesh_desc *__restrict__ mesh, float *__restrict__ den, float volfold,
-                        int *err, int32_t *__restrict__ boxes) {
+                        int *err, int32_t *__restrict__ boxes, int64_t chunk) {
     __shared__ float tile[TILE];
     __shared__ int scratch[13 * (kTileThreads / 32)];
-    for (int64_t c0 = (int64_t)blockIdx.x * kTileChunk; c0 < n; c0 += (int64_t)gridDim.x * kTileChunk) {
-        const int64_t c1 = min(c0 + (int64_t)kTileChunk, n);
+    for (int64_t c0 = blockIdx.x * chunk; c0 < n; c0 += gridDim.x * chunk) {
+        const int64_t c1 = min(c0 + chunk, n);
         int64_t s0 = c0;
         while (s0 < c1) {
             const int h = thalo[s0];  // octree order keeps each halo's range [pstart[h], pstart[h+1])
@@ -406,7 +464,8 @@ int launch_mesh_boxes(gf_ctx *ctx, int64_t n, const double *x, const double *y, 
     box_init_kernel<<<grid_for(nint, 256), 256, 0, ctx->stream>>>(boxes, nint);
     GF_LAUNCH_CHECK();
     if (n <= 0) return GF_OK;
-    mesh_box_kernel<<<grid_for(n, 256), 256, 0, ctx->stream>>>(n, x, y, z, type, hid, mesh, boxes);
+    const int64_t run = warp_run(n);
+    mesh_box_kernel<<<warp_run_grid(n, run), 256, 0, ctx->stream>>>(n, x, y, z, type, hid, mesh, boxes, run);
     GF_LAUNCH_CHECK();
     return GF_OK;
 }
@@ -424,10 +483,12 @@ int launch_stage_deposit(gf_ctx *ctx, int64_t n, const double *x, const double *
     }
     if (n <= 0) return GF_OK;
     const float fold = is_pow2_double(volfact) ? (float)volfact : 1.f;
-    const int64_t chunks = (n + kTileChunk - 1) / kTileChunk;
+    const int64_t chunk =
+        std::max<int64_t>(kTileThreads, std::min<int64_t>(kTileChunk, n / (sm_count() * 4) / kTileThreads * kTileThreads));
+    const int64_t chunks = (n + chunk - 1) / chunk;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(chunks, (int64_t)sm_count() * 8));
     tsc_tile_deposit_kernel<(GF_TSC_TILE > 0 ? GF_TSC_TILE : 1024)><<<grid, kTileThreads, 0, ctx->stream>>>(
-        n, x, y, z, mass, type, pstart, order, thalo, mesh, den, fold, ctx->d_err, boxes);
+        n, x, y, z, mass, type, pstart, order, thalo, mesh, den, fold, ctx->d_err, boxes, chunk);
     GF_LAUNCH_CHECK();
     return GF_OK;
 }
