@@ -9,10 +9,10 @@
 //     particles of the node;
 //   * monopole, second moments and dist2 = max |x - com|^2 are per node.
 // Nodes of more than kSmall particles are built level by level, every active
-// particle of all halos at once: accumulate mass and first moments, finalise
-// the COM, accumulate extents/second moments/octant counts, allocate children,
-// and scatter the particles into [loose | child 0 | child 1 | ...] order.  A
-// node of at most kSmall particles is left to one warp, which builds its whole
+// particle of all halos at once: accumulate mass and first moments, accumulate
+// extents/second moments/octant counts about the centre of mass, allocate
+// children, and scatter the particles into [loose | child 0 | child 1 | ...]
+// order.  A node of at most kSmall particles is left to one warp, which builds its whole
 // subtree in shared memory (small_subtrees).  The nodes are then numbered in
 // depth-first preorder so the walks are stackless: opening node i continues at
 // i + 1, skipping it continues at skip[i].  A node's preorder number is the
@@ -65,7 +65,7 @@ struct Build {
 };
 
 // A node of at most kSmall particles is built with its subtree by one warp.  The
-// level passes cost five launches a level (and, eagerly, a host wait) however
+// level passes cost four launches a level (and, eagerly, a host wait) however
 // few particles are left, and read every one of those from memory, so the
 // lower levels, most of a small batch's, go to shared memory: the stage on a
 // halo of 120 took 0.32 ms, now 0.24; on one of 131,072 1.59, now 1.40; a
@@ -250,16 +250,16 @@ accum_mass(int L, int64_t n, const float4 *__restrict__ pos, const int32_t *__re
     }
 }
 
-__global__ void finalize_com(int L, Build b) {
-    if (b.nact[L] == 0) return;
-    FOR_LEVEL_NODES(node, L, b) {
-        if (b.count[node] <= kSmall) continue;
-        const double m = b.m[node];
-        if (m > 0) {  // ost.c:553-555
-            b.mx[node] /= m;
-            b.my[node] /= m;
-            b.mz[node] /= m;
-        }
+// ost.c:553-555: the centre of mass of a node whose sums are complete.
+__device__ __forceinline__ void centre_of(const Build &b, int node, double &x, double &y, double &z) {
+    const double m = b.m[node];
+    x = b.mx[node];
+    y = b.my[node];
+    z = b.mz[node];
+    if (m > 0) {
+        x /= m;
+        y /= m;
+        z /= m;
     }
 }
 
@@ -287,7 +287,8 @@ accum_moments(int L, int64_t n, const float4 *__restrict__ pos, const int32_t *_
         int key = 0;
         if (node >= 0) {
             const float4 P = pos[p];
-            const double cx = b.mx[node], cy = b.my[node], cz = b.mz[node];
+            double cx, cy, cz;  // (divided by every particle: cheaper than a launch per level for it)
+            centre_of(b, node, cx, cy, cz);
             // ost.c:561-571: float offsets, float moments
             const float tx = (float)((double)P.x - cx);
             const float ty = (float)((double)P.y - cy);
@@ -391,6 +392,13 @@ __global__ void split_nodes(int L, int32_t ncap, int last, Build b) {
     if (b.nact[L] == 0) return;
     FOR_LEVEL_NODES(node, L, b) {
     if (b.count[node] <= kSmall) continue;
+    {
+        double x, y, z;
+        centre_of(b, node, x, y, z);
+        b.mx[node] = x;
+        b.my[node] = y;
+        b.mz[node] = z;
+    }
     const float r2 = __uint_as_float(b.r2[node]);
     const double nodesize = sqrt((double)r2);           // ost.c:574
     const bool divide = nodesize > 0.5 * kMinWidth;     // divideThisNode, tree.h:36
@@ -988,8 +996,6 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
                 return GF_EINVAL;
             }
             accum_mass<<<grid_n(n), kBlock, 0, s>>>(L, n, pos[cur], pnode[cur], b);
-            GF_LAUNCH_CHECK();
-            finalize_com<<<level_grid, 256, 0, s>>>(L, b);
             GF_LAUNCH_CHECK();
             accum_moments<<<grid_n(n), kBlock, 0, s>>>(L, n, pos[cur], pnode[cur], pkey, q5_asbuilt, b);
             GF_LAUNCH_CHECK();
