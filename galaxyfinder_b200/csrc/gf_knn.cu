@@ -1842,7 +1842,7 @@ __global__ void __launch_bounds__(128) knn_redo_kernel(
 
 int launch_knn(gf_ctx *ctx, const TreeView &t, const int64_t *pstart, const float4 *pos_batch, int k,
                int32_t *nearindex, float *dens, unsigned long long *counters,
-               const int32_t *qlist, int64_t nq) {
+               const int32_t *qlist, int64_t nq, bool beside) {
     if (k < 1 || k > 32) {
         set_status(GF_EINVAL, "k = %d: the warp kNN supports 1 <= k <= 32", k);
         return GF_EINVAL;
@@ -1876,12 +1876,14 @@ int launch_knn(gf_ctx *ctx, const TreeView &t, const int64_t *pstart, const floa
         // time falls (a smaller part of the tree, shorter lists) while the
         // work of all of them grows.  us with 1 / 2 / 4 lanes: 120 particles
         // 30 / 21 / 16, 36,001 267 / 212 / 211, 131,072 425 / 395 / 489,
-        // 1,000,003 2300 / 2660 / 3440.
+        // 1,000,003 2300 / 2660 / 3440.  Beside other kernels, which fill idle
+        // warps, the added work counts earlier: a stage with 1 / 2 lanes takes
+        // 36,000 particles 640 / 617, 70,000 752 / 769, 131,072 956 / 1025.
         const int64_t warps = wave * (block / 32);
         if (t.n <= 8 * warps) {
             lanes = 4;
             kern = counters ? knn_net_kernel<4, true> : knn_net_kernel<4, false>;
-        } else if (2 * t.n <= 5 * 16 * warps) {
+        } else if ((beside ? 4 : 2) * t.n <= 5 * 16 * warps) {
             lanes = 2;
             kern = counters ? knn_net_kernel<2, true> : knn_net_kernel<2, false>;
         }

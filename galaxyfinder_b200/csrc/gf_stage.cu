@@ -97,6 +97,7 @@ class Lanes {
         forked_[i] = true;
         return GF_OK;
     }
+    bool on() const { return on_; }
     void use(int i) {
         if (on_) ctx_->stream = ctx_->side[i];
     }
@@ -360,7 +361,8 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
             kc = ctx->tmp[4].as<unsigned long long>() + 4;
             GF_CUDA_TRY(cudaMemsetAsync(kc, 0, 5 * sizeof(unsigned long long), ctx->stream));
         }
-        return launch_knn(ctx, ctx->last_tree, b->pstart, pos, cfg->knn_k, o->nearindex, o->dens_sph, kc);
+        return launch_knn(ctx, ctx->last_tree, b->pstart, pos, cfg->knn_k, o->nearindex, o->dens_sph, kc, nullptr, 0,
+                          lanes.on() && cfg->do_potential);
     };
     // ---- 4. TSC mesh -> smoothing -> findDen
     auto mesh_rest = [&]() -> int {
@@ -616,7 +618,8 @@ int stage_pass_graph(StageGraph &g) {
         lanes.back();
     }
     if (cfg->knn_k > 0)
-        GF_TRY(launch_knn(ctx, ctx->last_tree, b->pstart, pos, cfg->knn_k, o->nearindex, o->dens_sph, nullptr));
+        GF_TRY(launch_knn(ctx, ctx->last_tree, b->pstart, pos, cfg->knn_k, o->nearindex, o->dens_sph, nullptr, nullptr, 0,
+                          lanes.on() && cfg->do_potential));
     if (cfg->do_potential) {
         const double pf = cfg->potentfact != 0.0 ? cfg->potentfact : physics().potentfact;
         PotentialParams pp = potential_params(cfg->theta2, cfg->ndirect, pf, cfg->add_bg);

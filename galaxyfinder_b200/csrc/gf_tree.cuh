@@ -71,7 +71,7 @@ PotentialParams potential_params(float theta2, int ndirect, double potentfact, i
 // batch index).
 int launch_knn(gf_ctx *ctx, const TreeView &t, const int64_t *pstart, const float4 *pos_batch, int k,
                int32_t *nearindex, float *dens, unsigned long long *counters = nullptr,
-               const int32_t *qlist = nullptr, int64_t nq = 0);
+               const int32_t *qlist = nullptr, int64_t nq = 0, bool beside = false);
 int launch_self_potential(gf_ctx *ctx, const TreeView &t, const int64_t *pstart,
                           const PotentialParams &pp, float *penergy, float *raw,
                           unsigned long long *counters);

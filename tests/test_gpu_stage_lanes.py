@@ -28,8 +28,8 @@ def _get(out):
     return {f: getattr(out, f).cpu().numpy() for f in FIELDS}
 
 
-def _case(cuda_device, nhalo=24, nmax=30000, seed=5):
-    hb = synth.catalogue(seed=seed, nhalo=nhalo, nmin=60, nmax=nmax, straddle_frac=0.2)
+def _case(cuda_device, nhalo=24, nmax=30000, seed=5, nmin=60):
+    hb = synth.catalogue(seed=seed, nhalo=nhalo, nmin=nmin, nmax=nmax, straddle_frac=0.2)
     return hb, batch.DeviceBatch.from_halobatch(hb)
 
 
@@ -119,4 +119,20 @@ def test_a_refused_run_leaves_the_context_usable(cuda_device):
     with pytest.raises(_lib.GFError):
         batch.stage_run(ctx, db, bad, out)
     _close(_get(batch.stage_run(ctx, db, cfg, out)), ref)
+    ctx.close()
+
+
+def test_search_beside_the_potential(cuda_device):
+    """Sizes at which a search beside other kernels gives a query one lane and
+    a search alone two."""
+    hb, db = _case(cuda_device, nhalo=2, nmin=45000, nmax=65000, seed=8)
+    ctx = batch.Context(0)
+    out = batch.StageBuffers(hb.n, 32, db.x.device, keep_phi=True)
+    cfg = batch.stage_config()
+    batch.stage_run(ctx, db, cfg, out)
+    got = _get(out)
+    out.nearindex.zero_()
+    torch.cuda.synchronize()
+    batch.stage_run(ctx, db, cfg, out, stats=True)
+    _close(got, _get(out))
     ctx.close()
