@@ -611,6 +611,8 @@ __global__ void bg_eval_kernel(int32_t n, const double *__restrict__ mvir, Poten
     if (i < n) bg[i] = bg_potent_dev(mvir[i], pp);
 }
 
+}  // namespace
+
 // bg and direct flags of every halo of t (scratch in ctx->tmp[5]).
 int launch_halo_bg(gf_ctx *ctx, const TreeView &t, const int64_t *pstart, const PotentialParams &pp,
                    const int32_t *ntarget_halo, double **bg, int32_t **direct) {
@@ -628,8 +630,6 @@ int launch_halo_bg(gf_ctx *ctx, const TreeView &t, const int64_t *pstart, const 
     return GF_OK;
 }
 
-}  // namespace
-
 // The background term of n halo masses as the potential kernels evaluate it.
 int launch_bg_eval(gf_ctx *ctx, int32_t n, const double *mvir, const PotentialParams &pp, double *bg) {
     if (n <= 0) return GF_OK;
@@ -642,12 +642,10 @@ int launch_bg_eval(gf_ctx *ctx, int32_t n, const double *mvir, const PotentialPa
 // (self potential); outputs in batch order.
 int launch_self_potential(gf_ctx *ctx, const TreeView &t, const int64_t *pstart,
                           const PotentialParams &pp, float *penergy, float *raw,
-                          unsigned long long *counters) {
+                          unsigned long long *counters, double *bg, int32_t *direct) {
     if (t.n <= 0) return GF_OK;
     // tree-ordered positions carry the masses; halo h is still [pstart[h], pstart[h+1])
-    double *bg;
-    int32_t *direct;
-    GF_TRY(launch_halo_bg(ctx, t, pstart, pp, nullptr, &bg, &direct));
+    if (!bg) GF_TRY(launch_halo_bg(ctx, t, pstart, pp, nullptr, &bg, &direct));
     GF_TRY(launch_bh(ctx, t.n, t.pos, t.phalo, t.perm, t, direct, bg, pp, penergy, raw, counters));
     return GF_OK;
 }

@@ -307,16 +307,23 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
         }
         return GF_OK;
     };
+    // the boxes and their zeroing, queued while the host has the octree's first
+    // levels to wait for
+    auto mesh_first = [&]() -> int {
+        lanes.use(0);
+        const int r = mesh_prepare();
+        lanes.back();
+        return r;
+    };
     if (do_mesh && !st) {
         GF_TRY(lanes.fork(0));
-        lanes.use(0);
-        GF_TRY(mesh_prepare());
-        lanes.back();
+        if (!need_tree) GF_TRY(mesh_first());
     }
     // ---- 2. octree
     if (need_tree)
         GF_TRY(build_tree(ctx, nh, n, b->pstart, pos, cfg->theta2, cfg->q5_asbuilt, &ctx->last_tree, nullptr,
-                          plan ? &plan->tree : nullptr));
+                          plan ? &plan->tree : nullptr,
+                          do_mesh && !st ? std::function<int()>(mesh_first) : std::function<int()>()));
     if (plan) {
         plan->need_tree = need_tree;
         plan->mesh = mesh;
@@ -394,6 +401,10 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
     };
     // ---- 5. potential
     unsigned long long *counters = nullptr;
+    const double pf = cfg->potentfact != 0.0 ? cfg->potentfact : physics().potentfact;
+    const PotentialParams pp = potential_params(cfg->theta2, cfg->ndirect, pf, cfg->add_bg);
+    double *bg = nullptr;
+    int32_t *direct = nullptr;
     auto potential = [&]() -> int {
         if (!cfg->do_potential) return GF_OK;
         if (st && cfg->count_work) {
@@ -401,9 +412,7 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
             counters = ctx->tmp[4].as<unsigned long long>();
             GF_CUDA_TRY(cudaMemsetAsync(counters, 0, 16, ctx->stream));
         }
-        const double pf = cfg->potentfact != 0.0 ? cfg->potentfact : physics().potentfact;
-        PotentialParams pp = potential_params(cfg->theta2, cfg->ndirect, pf, cfg->add_bg);
-        return launch_self_potential(ctx, ctx->last_tree, b->pstart, pp, o->penergy, o->phi, counters);
+        return launch_self_potential(ctx, ctx->last_tree, b->pstart, pp, o->penergy, o->phi, counters, bg, direct);
     };
     if (st || !do_mesh || !need_tree) {
         GF_TRY(knn());
@@ -420,6 +429,10 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
     } else {
         GF_TRY(lanes.fork(0));
         GF_TRY(lanes.fork(1));
+        if (cfg->do_potential && n > 0) {  // small: not behind the search's blocks
+            lanes.use(1);
+            GF_TRY(launch_halo_bg(ctx, ctx->last_tree, b->pstart, pp, nullptr, &bg, &direct));
+        }
         lanes.use(0);
         GF_TRY(mesh_rest());
         lanes.back();
@@ -597,6 +610,15 @@ int stage_pass_graph(StageGraph &g) {
         GF_TRY(build_tree(ctx, nh, n, b->pstart, pos, cfg->theta2, cfg->q5_asbuilt, &ctx->last_tree, &g.fixed));
     GF_TRY(lanes.fork(0));
     GF_TRY(lanes.fork(1));
+    const double pf = cfg->potentfact != 0.0 ? cfg->potentfact : physics().potentfact;
+    const PotentialParams pp = potential_params(cfg->theta2, cfg->ndirect, pf, cfg->add_bg);
+    double *bg = nullptr;
+    int32_t *direct = nullptr;
+    if (cfg->do_potential && n > 0) {  // small: not behind the search's blocks
+        lanes.use(1);
+        GF_TRY(launch_halo_bg(ctx, ctx->last_tree, b->pstart, pp, nullptr, &bg, &direct));
+        lanes.back();
+    }
     if (cfg->do_mesh) {
         lanes.use(0);
         GF_TRY(launch_stage_deposit(ctx, n, xr, yr, zr, b->mass, b->type, hid, b->pstart,
@@ -621,10 +643,8 @@ int stage_pass_graph(StageGraph &g) {
         GF_TRY(launch_knn(ctx, ctx->last_tree, b->pstart, pos, cfg->knn_k, o->nearindex, o->dens_sph, nullptr, nullptr, 0,
                           lanes.on() && cfg->do_potential));
     if (cfg->do_potential) {
-        const double pf = cfg->potentfact != 0.0 ? cfg->potentfact : physics().potentfact;
-        PotentialParams pp = potential_params(cfg->theta2, cfg->ndirect, pf, cfg->add_bg);
         lanes.use(1);
-        GF_TRY(launch_self_potential(ctx, ctx->last_tree, b->pstart, pp, o->penergy, o->phi, nullptr));
+        GF_TRY(launch_self_potential(ctx, ctx->last_tree, b->pstart, pp, o->penergy, o->phi, nullptr, bg, direct));
     }
     GF_TRY(lanes.join(0));
     return lanes.join(1);

@@ -426,6 +426,7 @@ __global__ void split_nodes(int L, int32_t ncap, int last, Build b) {
         if (first < 0) nch = nbig = 0;  // out of node capacity: keep all particles loose
     }
     if (nbig > 0) atomicAdd(b.nact + L + 1, nbig);
+    int small_at = nch > nbig ? atomicAdd(b.counter + 3, nch - nbig) : 0;
     const int start = b.start[node], halo = b.halo[node];
     int off = start;
 #pragma unroll
@@ -455,7 +456,7 @@ __global__ void split_nodes(int L, int32_t ncap, int last, Build b) {
                 zero_node(b, id);
             } else {  // its particles go to the final arrays, as loose ones
                 b.first[id] = L + 1;
-                b.small[atomicAdd(b.counter + 3, 1)] = id;
+                b.small[small_at++] = id;
             }
             off += cnt[c];
         }
@@ -910,7 +911,8 @@ T *carve(char *&p, size_t count) {
 
 int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
                const float4 *pos_in, float theta2, int q5_asbuilt, TreeView *out,
-               const TreeShape *fixed, TreeShape *shape) {
+               const TreeShape *fixed, TreeShape *shape, const std::function<int()> &before_wait) {
+    bool waited = !before_wait;  // else the caller queues its own work before the host first waits
     if (n > 0x7fffffffLL) {
         set_status(GF_ENOTIMPL, "tree build over more than 2^31 particles in one batch");
         return GF_ENOTIMPL;
@@ -1007,6 +1009,8 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
             GF_LAUNCH_CHECK();
             cur ^= 1;
             if (fixed || L % 3 != 2) continue;
+            if (!waited) GF_TRY(before_wait());
+            waited = true;
             GF_CUDA_TRY(cudaMemcpyAsync(&act, b.nact + L + 1, sizeof(act), cudaMemcpyDeviceToHost, s));
             GF_CUDA_TRY(cudaStreamSynchronize(s));
             more = act > 0;
@@ -1016,6 +1020,8 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
         GF_LAUNCH_CHECK();
         int32_t nnode = -1;
         if (!fixed) {
+            if (!waited) GF_TRY(before_wait());
+            waited = true;
             GF_CUDA_TRY(cudaMemcpyAsync(hc, b.counter, sizeof(hc), cudaMemcpyDeviceToHost, s));
             GF_CUDA_TRY(cudaStreamSynchronize(s));
             if (hc[1] & 4) {

@@ -3,6 +3,8 @@
 
 #include "gf_internal.cuh"
 
+#include <functional>
+
 namespace gf {
 
 // W4 kernel, nnost.c:536-555 (float arguments, double constants); the
@@ -51,9 +53,12 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
 // With `fixed`, the build runs fixed->levels levels over fixed->ncap node
 // slots with no host round trip (capturable in a CUDA graph) and flags
 // GF_ERRBIT_PLAN when the batch needs more; `shape` receives the shape built.
+// `before_wait` is called once, before the host first waits for the device (not
+// with `fixed`).
 int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
                const float4 *pos, float theta2, int q5_asbuilt, TreeView *out,
-               const TreeShape *fixed = nullptr, TreeShape *shape = nullptr);
+               const TreeShape *fixed = nullptr, TreeShape *shape = nullptr,
+               const std::function<int()> &before_wait = {});
 
 // Potential walk parameters (see gf_potent.cu).
 struct PotentialParams {
@@ -74,7 +79,11 @@ int launch_knn(gf_ctx *ctx, const TreeView &t, const int64_t *pstart, const floa
                const int32_t *qlist = nullptr, int64_t nq = 0, bool beside = false);
 int launch_self_potential(gf_ctx *ctx, const TreeView &t, const int64_t *pstart,
                           const PotentialParams &pp, float *penergy, float *raw,
-                          unsigned long long *counters);
+                          unsigned long long *counters, double *bg = nullptr, int32_t *direct = nullptr);
+// The background terms and direct-sum flags of t's halos (scratch of ctx), for
+// a launch_self_potential that follows.
+int launch_halo_bg(gf_ctx *ctx, const TreeView &t, const int64_t *pstart, const PotentialParams &pp,
+                   const int32_t *ntarget_halo, double **bg, int32_t **direct);
 int launch_bg_eval(gf_ctx *ctx, int32_t n, const double *mvir, const PotentialParams &pp, double *bg);
 int launch_external_potential(gf_ctx *ctx, const TreeView &t, const int64_t *pstart_src,
                               int64_t ntarget, const float4 *tpos, const int32_t *thalo,
