@@ -33,6 +33,14 @@ constexpr int kMinCell = 10;          // MIN_CELL_PARTICLE_NUM, tree.h:20
 constexpr double kMinWidth = 1.E-6;   // MINCELLWIDTH, tree.h:18
 constexpr int kBlock = GF_TREE_BLOCK;
 
+// |x - com|^2 with its roundings spelled out: a node's extent decides what a walk
+// opens, so it may not depend on how a kernel's compilation pairs the products
+// (one unit in the last place flips an opening in some 1e8 and moves that
+// target's potential by 1e-5).
+__device__ __forceinline__ float offset2(float x, float y, float z) {
+    return __fmaf_rn(z, z, __fmaf_rn(x, x, __fmul_rn(y, y)));
+}
+
 // Order-preserving float <-> uint32 map for atomic min/max on any sign.
 __device__ __forceinline__ unsigned fkey(float v) {
     unsigned u = __float_as_uint(v);
@@ -294,7 +302,7 @@ accum_moments(int L, int64_t n, const float4 *__restrict__ pos, const int32_t *_
             const float ty = (float)((double)P.y - cy);
             const float tz = (float)((double)P.z - cz);
             const float m = P.w;
-            v[0] = tx * tx + ty * ty + tz * tz;
+            v[0] = offset2(tx, ty, tz);
             v[1] = m * tx * tx;
             v[2] = m * ty * ty;
             v[3] = m * tz * tz;
@@ -598,7 +606,7 @@ small_subtrees(int32_t ncap, int q5_asbuilt, float4 *__restrict__ fpos, int32_t 
                 const float ty = (float)((double)P.y - cy);
                 const float tz = (float)((double)P.z - cz);
                 const float m = P.w;
-                r2 = fmaxf(r2, tx * tx + ty * ty + tz * tz);
+                r2 = fmaxf(r2, offset2(tx, ty, tz));
                 q[0] += m * tx * tx;
                 q[1] += m * ty * ty;
                 q[2] += m * tz * tz;

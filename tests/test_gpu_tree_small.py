@@ -103,6 +103,23 @@ def test_chains(ctx, n):
     _check(ctx, [0.5 + np.abs(rng.standard_normal((n, 3))) * r[:, None], 0.5 - r[:, None] * np.ones(3)])
 
 
+@pytest.mark.parametrize("n", [200, 5000, 60000])
+def test_extent_rounding(ctx, n):
+    """max |x - com|^2 of every node to the bit, whichever kernel built it:
+    fma(z, z, fma(x, x, y y)) of float offsets (a sum of a float and an exact
+    product of two in doubles, rounded once more: equal but for ties within
+    2^-29 of a unit, which the seeds do not hit)."""
+    p = np.concatenate([_cloud(np.random.default_rng(n), n), np.ones((n, 1))], 1).astype(np.float32)
+    t = batch.tree_build_export(ctx, np.array([0, n], np.int64), p, theta2=0.5)
+    for k, b in zip(t["knn"], t["bh"]):
+        P = t["pos"][k["lstart"]:k["lstart"] + k["count"], :3].astype(np.float64)
+        d = (P - b["com"]).astype(np.float32)
+        x, y, z = (d[:, a].astype(np.float64) for a in range(3))
+        a = (x * x + (d[:, 1] * d[:, 1]).astype(np.float64)).astype(np.float32)
+        r2 = (z * z + a.astype(np.float64)).astype(np.float32)
+        assert b["open_r2"] == 2.0 * r2.max()
+
+
 @pytest.mark.parametrize("n", [100, 300])
 def test_endless_chain_is_refused(ctx, n):
     """One particle at infinity puts every centre of mass there: all particles
