@@ -105,35 +105,34 @@ constexpr int kMaxLevels = 4096;
     for (int node = (b).lev[L] + blockIdx.x * blockDim.x + threadIdx.x; node < (b).lev[(L) + 1]; \
          node += gridDim.x * blockDim.x)
 
-// The roots are nodes 0 .. nhalo-1 (counter and nact start zeroed).
-__global__ void init_roots(int32_t nhalo, const int64_t *__restrict__ pstart, Build b) {
-    int h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h == 0) {
-        b.counter[0] = nhalo;
-        b.lev[0] = 0;
-        b.lev[1] = nhalo;
-    }
-    if (h >= nhalo) return;
-    const int c = (int32_t)(pstart[h + 1] - pstart[h]);
-    b.start[h] = (int32_t)pstart[h];
-    b.count[h] = c;
-    b.halo[h] = h;
-    b.par[h] = -1;
-    if (c > kSmall) {
-        zero_node(b, h);
-        atomicAdd(b.nact, 1);
-    } else {
-        b.first[h] = 0;
-        b.small[atomicAdd(b.counter + 3, 1)] = h;
-    }
-}
-
-// Particles of small halos go straight to the final arrays, where
+// The roots, nodes 0 .. nhalo-1 (counter and nact start zeroed), and the
+// particles; those of small halos go straight to the final arrays, where
 // small_subtrees orders them.
-__global__ void init_particles(int64_t n, const int64_t *__restrict__ pstart, int32_t nhalo,
-                               const float4 *__restrict__ pos_in, float4 *__restrict__ pos,
-                               int32_t *__restrict__ perm, int32_t *__restrict__ pnode, float4 *__restrict__ fpos,
-                               int32_t *__restrict__ fperm, int32_t *__restrict__ phalo) {
+__global__ void init_build(int64_t n, const int64_t *__restrict__ pstart, int32_t nhalo,
+                           const float4 *__restrict__ pos_in, float4 *__restrict__ pos, int32_t *__restrict__ perm,
+                           int32_t *__restrict__ pnode, float4 *__restrict__ fpos, int32_t *__restrict__ fperm,
+                           int32_t *__restrict__ phalo, Build b) {
+    for (int64_t h = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; h < max(nhalo, 1);
+         h += (int64_t)gridDim.x * blockDim.x) {
+        if (h == 0) {
+            b.counter[0] = nhalo;
+            b.lev[0] = 0;
+            b.lev[1] = nhalo;
+        }
+        if (h >= nhalo) break;
+        const int c = (int32_t)(pstart[h + 1] - pstart[h]);
+        b.start[h] = (int32_t)pstart[h];
+        b.count[h] = c;
+        b.halo[h] = (int32_t)h;
+        b.par[h] = -1;
+        if (c > kSmall) {
+            zero_node(b, (int)h);
+            atomicAdd(b.nact, 1);
+        } else {
+            b.first[h] = 0;
+            b.small[atomicAdd(b.counter + 3, 1)] = (int32_t)h;
+        }
+    }
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
          p += (int64_t)gridDim.x * blockDim.x) {
         int lo = 0, hi = nhalo;
@@ -777,6 +776,50 @@ scan_sums(int64_t n, const int32_t *__restrict__ hist, int32_t *__restrict__ sum
     if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
+// Per halo, the halos before it without particles (their roots are nodes too).
+__device__ __forceinline__ void scan_empty(int32_t nhalo, const int64_t *__restrict__ pstart,
+                                           int32_t *__restrict__ empty, int *scratch) {
+    int run = 0, total;
+    for (int32_t c = 0; c < nhalo; c += 1024) {
+        const int h = c + threadIdx.x;
+        const int v = h < nhalo && pstart[h] == pstart[h + 1];
+        const int at = run + block_scan<1024>(v, total, scratch);
+        if (h < nhalo) empty[h] = at;
+        run += total;
+    }
+}
+
+// Small batches: all of the numbering's counts and scans in one block, in place
+// of a memset and four launches (the stage on 120 particles 185 us, now 172).
+constexpr int kNumberMax = 8192;
+__global__ void __launch_bounds__(1024)
+number_small(int32_t ncap, int32_t n, Build b, int32_t nhalo, const int64_t *__restrict__ pstart,
+             int32_t *__restrict__ before, int32_t *__restrict__ empty) {
+    constexpr int kItems = kNumberMax / 1024 + 1;  // of the n + 1 entries
+    __shared__ int hist[kItems * 1024];
+    __shared__ int scratch[32];
+    for (int p = threadIdx.x; p < kItems * 1024; p += 1024) hist[p] = 0;
+    __syncthreads();
+    const int nn = min(b.counter[0], ncap);
+    for (int node = threadIdx.x; node < nn; node += 1024)
+        if (b.count[node] > 0) atomicAdd(hist + b.start[node], 1);
+    __syncthreads();
+    int v[kItems], sum = 0, total;
+#pragma unroll
+    for (int i = 0; i < kItems; i++) {
+        v[i] = hist[threadIdx.x * kItems + i];
+        sum += v[i];
+    }
+    int at = block_scan<1024>(sum, total, scratch);
+#pragma unroll
+    for (int i = 0; i < kItems; i++) {
+        const int p = threadIdx.x * kItems + i;
+        if (p <= n) before[p] = at;
+        at += v[i];
+    }
+    scan_empty(nhalo, pstart, empty, scratch);
+}
+
 // The chunk sums (in place) and, per halo, the halos before it without
 // particles (their roots are nodes too), as exclusive prefixes: one block.
 __global__ void __launch_bounds__(1024)
@@ -790,14 +833,7 @@ scan_mid(int64_t nchunk, int32_t *__restrict__ sums, int32_t nhalo, const int64_
         if (c + threadIdx.x < nchunk) sums[c + threadIdx.x] = at;
         run += total;
     }
-    run = 0;
-    for (int32_t c = 0; c < nhalo; c += 1024) {
-        const int h = c + threadIdx.x;
-        const int v = h < nhalo && pstart[h] == pstart[h + 1];
-        const int at = run + block_scan<1024>(v, total, scratch);
-        if (h < nhalo) empty[h] = at;
-        run += total;
-    }
+    scan_empty(nhalo, pstart, empty, scratch);
 }
 
 __global__ void __launch_bounds__(kScanThreads)
@@ -983,11 +1019,9 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
         b.lev = carve<int32_t>(np_, kMaxLevels + 2);
         cudaStream_t s = ctx->stream;
         GF_CUDA_TRY(cudaMemsetAsync(b.counter, 0, zero_end - (char *)b.counter, s));
-        GF_CUDA_TRY(cudaMemsetAsync(before, 0, nscan * sizeof(int32_t), s));
-        init_roots<<<grid_exact(nhalo, 256), 256, 0, s>>>(nhalo, pstart_dev, b);
-        GF_LAUNCH_CHECK();
-        init_particles<<<grid_n(n), kBlock, 0, s>>>(n, pstart_dev, nhalo, pos_in, pos[0], perm[0], pnode[0], fpos,
-                                                    fperm, phalo);
+        if (n > kNumberMax) GF_CUDA_TRY(cudaMemsetAsync(before, 0, nscan * sizeof(int32_t), s));
+        init_build<<<grid_n(std::max<int64_t>(n, nhalo)), kBlock, 0, s>>>(n, pstart_dev, nhalo, pos_in, pos[0], perm[0],
+                                                                          pnode[0], fpos, fperm, phalo, b);
         GF_LAUNCH_CHECK();
         // Level by level.  Eagerly, the host looks after every third level
         // whether a level is left (levels past the last one return at once);
@@ -1040,14 +1074,19 @@ int build_tree(gf_ctx *ctx, int32_t nhalo, int64_t n, const int64_t *pstart_dev,
             nnode = hc[0];
         }
         const int node_grid = fixed ? fixed_grid : grid_exact(nnode, 256);
-        count_starts<<<node_grid, 256, 0, s>>>((int32_t)ncap, b, before);
-        GF_LAUNCH_CHECK();
-        scan_sums<<<(unsigned)nchunk, kScanThreads, 0, s>>>(nscan, before, sums);
-        GF_LAUNCH_CHECK();
-        scan_mid<<<1, 1024, 0, s>>>(nchunk, sums, nhalo, pstart_dev, empty);
-        GF_LAUNCH_CHECK();
-        scan_chunks<<<(unsigned)nchunk, kScanThreads, 0, s>>>(nscan, before, sums);
-        GF_LAUNCH_CHECK();
+        if (n <= kNumberMax) {
+            number_small<<<1, 1024, 0, s>>>((int32_t)ncap, (int32_t)n, b, nhalo, pstart_dev, before, empty);
+            GF_LAUNCH_CHECK();
+        } else {
+            count_starts<<<node_grid, 256, 0, s>>>((int32_t)ncap, b, before);
+            GF_LAUNCH_CHECK();
+            scan_sums<<<(unsigned)nchunk, kScanThreads, 0, s>>>(nscan, before, sums);
+            GF_LAUNCH_CHECK();
+            scan_mid<<<1, 1024, 0, s>>>(nchunk, sums, nhalo, pstart_dev, empty);
+            GF_LAUNCH_CHECK();
+            scan_chunks<<<(unsigned)nchunk, kScanThreads, 0, s>>>(nscan, before, sums);
+            GF_LAUNCH_CHECK();
+        }
         if (shape) {
             shape->levels = std::max(hc[4], 1);
             shape->ncap = ncap;

@@ -128,3 +128,11 @@ def test_endless_chain_is_refused(ctx, n):
     p[n // 2] = np.inf
     with pytest.raises(GFError, match="deeper than"):
         _check(ctx, [p])
+
+
+@pytest.mark.parametrize("n", [8191, 8192, 8193])
+def test_numbering_of_small_batches(ctx, n):
+    """Both sides of the batch size up to which one block numbers the nodes,
+    with halos without particles at the ends and between."""
+    rng = np.random.default_rng(n)
+    _check(ctx, [_cloud(rng, c) for c in (0, 3000, 0, 0, 12, 700, n - 3712, 0)])
