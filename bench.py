@@ -42,15 +42,14 @@ UNIT = "particles/s"
 K_NEIGH = 32
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per particle of
-# each phase's dominant kernel, from one ncu capture of the 1024-halo
-# catalogue (1,281,067 particles); the traffic scales with the particles
-# processed.
-TRAFFIC_PER_PARTICLE = {"knn": (59.67e6 + 115.437e6) / 1281067}
+# each phase's dominant kernel, from one ncu capture of a batch of 1024 halos
+# (1,206,438 particles); the traffic scales with the particles processed.
+TRAFFIC_PER_PARTICLE = {"knn": 149.5e6 / 1206438}
 # What bounds the kNN kernel instead of HBM, from the same capture: the tree
 # walk is latency- and issue-bound (its HBM traffic is the neighbour lists).
-KNN_LIMITER = ("latency/issue: 68.7% of issue slots active, 35.9% of warp slots occupied (6 blocks of 4 "
-               "warps per SM: 79 registers and 35.3 KB of heaps per block), dominant stall 'wait'; "
-               "DRAM 0.69% of peak")
+KNN_LIMITER = ("latency/issue: 61.3% of issue slots active, 35.5% of warp slots occupied (6 blocks of 4 "
+               "warps per SM: 80 registers and 34.3 KB of keys and slots per block), ALU pipe 51%; "
+               "DRAM 1.0% of peak")
 
 
 def parse():
@@ -863,7 +862,7 @@ def main():
         roofline = {"kernel": dom, "bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"],
                     "unit": "GB/s", "frac": achieved / pk["hbm_gbs"],
                     "traffic": None if traffic is None else traffic * n,
-                    "traffic_note": "bytes per launch, ncu capture of the 1024-halo catalogue scaled by particles",
+                    "traffic_note": "bytes per launch, ncu capture of a batch of 1024 halos scaled by particles",
                     "algorithmic_bytes": alg[dom], "peak_source": pk["source"]}
         if dom == "knn":
             roofline["limiter"] = KNN_LIMITER
@@ -879,7 +878,13 @@ def main():
 
     # the kNN kernel's own work counters, per query
     algo = _lib.tuning_value("GF_KNN_ALGO")
-    if algo in (1, 2):
+    if algo == 3:
+        names = ("node_tests_per_bucket", "particle_tests_per_bucket", "keys_appended",
+                 "warp_append_steps_per_bucket", "uncertified_fraction")
+        per = {"node_tests_per_bucket": 32, "particle_tests_per_bucket": 32, "warp_append_steps_per_bucket": 32}
+        kernel = ("knn_net_kernel (lane = query, sorting-network lists, exact FP64 certification; "
+                  "uncertified queries redone by knn_redo_kernel)")
+    elif algo in (1, 2):
         names = ("node_tests_per_bucket", "particle_tests_per_bucket", "heap_insertions",
                  "warp_insertion_steps_per_bucket",
                  "buckets_per_query" if algo == 1 else "uncertified_fraction")

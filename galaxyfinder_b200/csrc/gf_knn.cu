@@ -1251,7 +1251,7 @@ knn_fbucket_kernel(int64_t n, int k, const float4 *__restrict__ pos, const int32
 // queries of a clumpy halo: about 8 k append, 7 k test 1100 candidates, 6 k
 // merge 15 times, 5 k visit 160 nodes, 4 k write the lists) and, below a wave
 // of warps, the latency of one warp's chain of node visits and tiles.
-// Heaps (knn_fbucket_kernel) -> networks: 4096 halos (7.0 M particles) 14.5 ->
+// Heaps (knn_fbucket_kernel) -> networks: 4096 halos (6.1 M particles) 14.5 ->
 // 8.7 ms, 1,000,003 particles 3.71 -> 2.29 ms, 131,072 0.62 -> 0.39 ms, 120
 // 65 -> 16 us.  16 waiting keys, because 32 need 12.7 KB of shared memory per
 // warp instead of 8.6 (16 resident warps instead of 24) and sort twice the

@@ -36,9 +36,9 @@
 // with one Kahan sum per target; without the Kahan step, or with eight tiles
 // between two additions, up to 2.9e-8.
 //
-// What bounds it: issue slots (62 % used, 27 k instructions per warp) and, at 5
+// What bounds it: issue slots (62 % used, 29 k instructions per warp) and, at 5
 // blocks per SM (96 registers, of which 32 are sums and 26 a cell's fields),
-// the latency of the expansion's loads and shuffles; the FP32 pipe is 46 %
+// the latency of the expansion's loads and shuffles; the FP32 pipe is 44 %
 // busy.  A 131072-particle NFW halo at theta2 = 0.5 has, per warp, 937 cells
 // (23 of 32 lanes) and 1268 particles (12 of 32).  With lane = target and the
 // entries in shared memory, 13 floats of every cell were loaded by all lanes:

@@ -99,7 +99,7 @@ __device__ __forceinline__ float tsc_interp_add(float density, float v, const Ts
 // (or row padding) and gets +0.  Reductions per second at the L2 bound the
 // scattered deposits; scalar -> vector, 2e6 particles in 64 clumps into a
 // 256^3 mesh: deposit 435 -> 227 us, adjoint of the interpolation 582 -> 335;
-// the stage's tiled deposit (its segments too sparse for a tile) over 7.0 M
+// the stage's tiled deposit (its segments too sparse for a tile) over 6.1 M
 // particles 1061 -> 769.
 __device__ __forceinline__ void mesh_add3(float *p, float v0, float v1, float v2, bool wide) {
     const unsigned at = wide ? (unsigned)((uintptr_t)p >> 2) & 3u : 4u;

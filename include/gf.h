@@ -53,7 +53,7 @@ int gf_set_device(int device);
 uint64_t gf_kernel_launch_count(void);
 /* Compile-time launch parameter `name` of the loaded library (GF_KNN_ALGO,
  * GF_KNNB_BLOCK, GF_KNNB_ARITY, GF_KNNB_SEEDS, GF_KNNB_QUEUE, GF_KNNB_LANECERT,
- * GF_KNN_BLOCK, GF_KNN_MINB, GF_KNN_CHUNK, GF_BH_BLOCK, GF_BH_MINB, GF_BH_DYN, GF_BH_ACC, GF_KNNB_DYN,
+ * GF_KNN_BLOCK, GF_KNN_MINB, GF_KNN_CHUNK, GF_BH_BLOCK, GF_BH_MINB, GF_BH_DYN, GF_KNNB_DYN,
  * GF_FFT_PENCILS, GF_FFT_PENCILS_64, GF_FFT_PENCILS_128, GF_TSC_TILE,
  * GF_TREE_BLOCK) in *value.
  * Returns GF_EINVAL for an unknown name. */
@@ -472,7 +472,8 @@ typedef struct gf_stage_config {
     int32_t mesh_onchip;   /* 1: 64^3 meshes run their whole mesh stage (TSC, smoothing,
                               findDen) in one thread-block cluster's distributed shared
                               memory; 0: every mesh through device memory (faster on the
-                              benchmark catalogue: 18.2 vs 32.2 ms of smoothing) */
+                              benchmark catalogue: 3 ms of smoothing, against 24 ms for
+                              the on-chip meshes alone) */
     int32_t plain_fp64;    /* 1: the plain FP64 stage (every phase in FP64 by straightforward
                               kernels, meshes in device memory), the baseline the batched
                               FP32 stage is compared with */
@@ -505,7 +506,10 @@ typedef struct gf_stage_stats {
     int64_t mesh_pass_cells;
 } gf_stage_stats;
 
-/* stats may be NULL; when given, per-phase CUDA-event times are filled in. */
+/* stats may be NULL; when given, per-phase CUDA-event times are filled in and
+ * the phases run one after the other.  Without, the mesh part and the potential
+ * run on two streams of the context beside the octree build and the search;
+ * both are joined back into ctx's stream. */
 int gf_stage_run(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg, gf_stage_out *out,
                  gf_stage_stats *stats);
 
@@ -514,8 +518,9 @@ int gf_stage_run(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg, gf_
  * gf_stage_graph_create runs gf_stage_run once to plan (the meshes from the
  * halo extents, the octree's depth and node count; its outputs are this
  * batch's results), then captures a pass that computes the frames and meshes
- * on the device, builds the octree with a fixed depth (two levels above the
- * planned one) and node capacity (a quarter above), and runs every kernel of
+ * on the device, builds the octree with a fixed number of levels for nodes of
+ * more than 256 particles (two above the planned tree's depth) and node
+ * capacity (a quarter above), and runs every kernel of
  * the stage with no host round trip.  The batch, config and output structs
  * are copied: the device buffers they point to must stay allocated and are
  * read and written by every replay.
