@@ -524,7 +524,8 @@ int gf_stage_run(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg, gf_
 // the halo extents, the octree's depth and node count); the captured pass
 // then computes the frames and meshes on the device from the same extents,
 // builds the octree with a fixed number of levels of nodes above 256 particles
-// (two more than the planned tree is deep) and node capacity (a quarter more) and replays every kernel of the stage with
+// (two more than the planned tree is deep) and node capacity (a quarter more)
+// and replays every kernel of the stage with
 // no host round trip.  A replay is valid for any contents of the batch's
 // input buffers whose meshes keep the planned shapes and whose octree fits
 // the fixed shape; otherwise the pass flags GF_ERRBIT_PLAN and the replay
