@@ -429,23 +429,32 @@ __device__ __forceinline__ void dft(float2 (&a)[R]) {
     } else if (R == 4) {
         dft4<INV>(a[0], a[1], a[2], a[3]);
     } else if (R == 16) {  // 4 x 4: columns, W16 twiddles, rows
-        // cos and sin of pi/8, and of pi/4
-        const float c1 = 0.92387953251128676f, s1 = 0.38268343236508977f, h = 0.70710678118654752f;
+        // cos and sin of pi/8, and of pi/4.  The float cosine is off by nearly
+        // half a unit in the last place in every product it is in, which made a
+        // 256-cell axis 4 % less exact than its radix-8 passes were (rms of a
+        // mesh's cells against 64 bits); it is held as the sum of two floats.
+        constexpr double kCos = 0.92387953251128676;
+        constexpr float c1 = (float)kCos, c1lo = (float)(kCos - (double)c1);
+        const float s1 = 0.38268343236508977f, h = 0.70710678118654752f;
+        constexpr float sg = INV ? -1.f : 1.f;
         auto tw = [](float2 v, float c, float s) {  // v * (c - i s), conjugated for the inverse
-            return INV ? make_float2(v.x * c - v.y * s, v.y * c + v.x * s)
-                       : make_float2(v.x * c + v.y * s, v.y * c - v.x * s);
+            return make_float2(v.x * c + sg * v.y * s, v.y * c - sg * v.x * s);
         };
+        auto cadd1 = [=](float v, float t) { return fmaf(v, c1, fmaf(v, c1lo, t)); };  // v cos(pi/8) + t
+        auto tw1 = [=](float2 v) { return make_float2(cadd1(v.x, sg * v.y * s1), cadd1(v.y, -sg * v.x * s1)); };
+        auto tw3 = [=](float2 v) { return make_float2(cadd1(sg * v.y, v.x * s1), cadd1(-sg * v.x, v.y * s1)); };
 #pragma unroll
         for (int i = 0; i < 4; i++) dft4<INV>(a[i], a[4 + i], a[8 + i], a[12 + i]);
-        a[5] = tw(a[5], c1, s1);     // W16^1
+        a[5] = tw1(a[5]);            // W16^1
         a[9] = tw(a[9], h, h);       // W16^2
-        a[13] = tw(a[13], s1, c1);   // W16^3
+        a[13] = tw3(a[13]);          // W16^3
         a[6] = tw(a[6], h, h);       // W16^2
         a[10] = mul_mi<INV>(a[10]);  // W16^4
         a[14] = tw(a[14], -h, h);    // W16^6
-        a[7] = tw(a[7], s1, c1);     // W16^3
+        a[7] = tw3(a[7]);            // W16^3
         a[11] = tw(a[11], -h, h);    // W16^6
-        a[15] = tw(a[15], -c1, -s1); // W16^9
+        a[15] = tw1(a[15]);          // W16^9 = -W16^1
+        a[15] = make_float2(-a[15].x, -a[15].y);
 #pragma unroll
         for (int i = 0; i < 16; i += 4) dft4<INV>(a[i], a[i + 1], a[i + 2], a[i + 3]);
         // entry 4 k + j holds output k + 4 j
@@ -827,7 +836,11 @@ __device__ __forceinline__ void tile_sync() {
 }
 
 // Pair c of a tile (on: it holds a pencil), thread n0 of T: load(s) gives both
-// pencils' element s, store(s, v) takes the filtered one.
+// pencils' element s, store(s, v) takes the filtered one.  A pair is two
+// neighbouring pencils, 2c and 2c + 1: either half of a complex pencil carries
+// the rounding errors of the brighter one, and a neighbour is about as bright.
+// (Pencils half a tile apart: the cells beside a dense core took its noise 16
+// cells further; their median error was 2 to 17 times as large.)
 template <int AXIS, int LOGN, class Load, class Store>
 __device__ __forceinline__ void reg_fft_pair(float2 *sm, int c, int n0, bool on, const float2 *__restrict__ tw,
                                              const float *__restrict__ filt, Load load, Store store) {
@@ -893,8 +906,7 @@ smooth_reg_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh
     const int64_t mx = 2 * (m.nx / 2 + 1);
     const int c = AXIS == 0 ? threadIdx.x / F::T : threadIdx.x % F::PAIRS;
     const int n0 = AXIS == 0 ? threadIdx.x % F::T : threadIdx.x / F::PAIRS;
-    const int half = (t.npen + 1) >> 1;  // pair c: pencils c and c + half
-    const bool two = c + half < t.npen;
+    const bool on = 2 * c < t.npen, two = 2 * c + 1 < t.npen;
     // element (pencil p, position s) lives at base + p*pstride + s*sstride;
     // within one tile the offsets fit in 32 bits (axes <= 512, mx*ny < 2^21)
     int64_t base;
@@ -902,14 +914,26 @@ smooth_reg_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh
     if (AXIS == 0) { base = m.off + mx * t.base; pstride = (int)mx; sstride = 1; }
     else if (AXIS == 1) { base = m.off + t.base + mx * (int64_t)m.ny * t.other; pstride = 1; sstride = (int)mx; }
     else { base = m.off + t.base + mx * (int64_t)t.other; pstride = 1; sstride = (int)(mx * m.ny); }
-    float *p0 = den + base + c * pstride, *p1 = p0 + half * pstride;
+    float *p0 = den + base + 2 * c * pstride;
+    // mx and every tile's first pencil are even: pairs of cells are 8-byte
+    // aligned when the mesh is
+    const bool wide = AXIS != 0 && two && ((uintptr_t)(den + m.off) & 7) == 0;
     const float2 *tw = reinterpret_cast<const float2 *>(tables + at.tab_off);
     reg_fft_pair<AXIS, LOGN>(
-        smem, c, n0, c < half, tw, tables + at.tab_off + 2 * F::N,
-        [&](int s) { return make_float2(p0[s * sstride], two ? p1[s * sstride] : 0.f); },
+        smem, c, n0, on, tw, tables + at.tab_off + 2 * F::N,
+        [&](int s) {
+            const float *e = p0 + s * sstride;
+            if (wide) return *reinterpret_cast<const float2 *>(e);
+            return make_float2(e[0], two ? e[pstride] : 0.f);
+        },
         [&](int s, float2 v) {
-            p0[s * sstride] = v.x;
-            if (two) p1[s * sstride] = v.y;
+            float *e = p0 + s * sstride;
+            if (wide) {
+                *reinterpret_cast<float2 *>(e) = v;
+            } else {
+                e[0] = v.x;
+                if (two) e[pstride] = v.y;
+            }
         });
 }
 
@@ -1017,13 +1041,21 @@ smooth_fft_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh
 // (a CUDA graph replays them for new particle positions).
 struct BoxGeom {
     int u0, nu, v0, nv;                // pencil grid: u fastest
+    int a0, a1;                        // u of the pencils that are filtered
     int ustride, vstride, sstride;     // float offsets within the mesh
     int l0, l1, s0, s1;                // read and write ranges along the pencil
 };
 
 __device__ __forceinline__ int box_len(int lo, int hi) { return hi >= lo ? hi - lo + 1 : 0; }
 
-template <int AXIS>
+// Where the columns' pairs are moved as 8-byte words (the axes of the register
+// transform), the grid of their pencils starts and ends at a pair of cells.
+__device__ __forceinline__ int pair_lo(int lo, bool pairs) { return pairs ? lo & ~1 : lo; }
+__device__ __forceinline__ int pair_len(int lo, int hi, bool pairs) {
+    return hi < lo ? 0 : pairs ? (hi | 1) - (lo & ~1) + 1 : hi - lo + 1;
+}
+
+template <int AXIS, bool PAIRS>
 __device__ __forceinline__ BoxGeom box_geom(const gf_mesh_desc &m, const int32_t *__restrict__ bx) {
     const int mx = 2 * (m.nx / 2 + 1);
     BoxGeom g;
@@ -1032,24 +1064,26 @@ __device__ __forceinline__ BoxGeom box_geom(const gf_mesh_desc &m, const int32_t
         g.ustride = mx; g.vstride = mx * m.ny; g.sstride = 1;
         g.l0 = bx[0]; g.l1 = bx[1]; g.s0 = bx[6]; g.s1 = bx[7];
     } else if (AXIS == 1) {
-        g.u0 = bx[6]; g.nu = box_len(bx[6], bx[7]); g.v0 = bx[4]; g.nv = box_len(bx[4], bx[5]);
+        g.u0 = pair_lo(bx[6], PAIRS); g.nu = pair_len(bx[6], bx[7], PAIRS); g.v0 = bx[4]; g.nv = box_len(bx[4], bx[5]);
         g.ustride = 1; g.vstride = mx * m.ny; g.sstride = mx;
         g.l0 = bx[2]; g.l1 = bx[3]; g.s0 = bx[8]; g.s1 = bx[9];
     } else {
-        g.u0 = bx[6]; g.nu = box_len(bx[6], bx[7]); g.v0 = bx[8]; g.nv = box_len(bx[8], bx[9]);
+        g.u0 = pair_lo(bx[6], PAIRS); g.nu = pair_len(bx[6], bx[7], PAIRS); g.v0 = bx[8]; g.nv = box_len(bx[8], bx[9]);
         g.ustride = 1; g.vstride = mx; g.sstride = mx * m.ny;
         g.l0 = bx[4]; g.l1 = bx[5]; g.s0 = bx[10]; g.s1 = bx[11];
     }
+    g.a0 = AXIS == 0 ? bx[2] : bx[6];
+    g.a1 = AXIS == 0 ? bx[3] : bx[7];
     if (bx[0] > bx[1]) g.nu = g.nv = 0;  // nothing deposited: no pass
     return g;
 }
 
-__device__ __forceinline__ int64_t box_tiles(int axis, const int32_t *__restrict__ bx, int pmax) {
+__device__ __forceinline__ int64_t box_tiles(int axis, const int32_t *__restrict__ bx, int pmax, bool pairs) {
     if (bx[0] > bx[1]) return 0;
     int64_t pen;
     if (axis == 0) pen = (int64_t)box_len(bx[2], bx[3]) * box_len(bx[4], bx[5]);
-    else if (axis == 1) pen = (int64_t)box_len(bx[6], bx[7]) * box_len(bx[4], bx[5]);
-    else pen = (int64_t)box_len(bx[6], bx[7]) * box_len(bx[8], bx[9]);
+    else if (axis == 1) pen = (int64_t)pair_len(bx[6], bx[7], pairs) * box_len(bx[4], bx[5]);
+    else pen = (int64_t)pair_len(bx[6], bx[7], pairs) * box_len(bx[8], bx[9]);
     return (pen + pmax - 1) / pmax;
 }
 
@@ -1064,7 +1098,7 @@ constexpr int kBoxMaxGroups = 16;
 struct BoxPlanGroup {
     const int32_t *halos;
     int64_t *starts;  // ngroup + 1, written here
-    int32_t ngroup, axis, pmax;
+    int32_t ngroup, axis, pmax, pairs;
 };
 struct BoxPlanArgs {
     int32_t ngroups, nhalo;
@@ -1079,10 +1113,10 @@ struct BoxPlanArgs {
 __global__ void __launch_bounds__(1024) box_plan_kernel(BoxPlanArgs a) {
     __shared__ int64_t part[1024];
     const bool zero = (int)blockIdx.x == a.ngroups;
-    const BoxPlanGroup G = zero ? BoxPlanGroup{nullptr, a.zstart, a.nhalo, 0, 1} : a.g[blockIdx.x];
+    const BoxPlanGroup G = zero ? BoxPlanGroup{nullptr, a.zstart, a.nhalo, 0, 1, 0} : a.g[blockIdx.x];
     auto count = [&](int i) -> int64_t {
         if (zero) return box_zero_rows(a.mesh[i], a.boxes + (int64_t)kMeshBoxInts * i);
-        return box_tiles(G.axis, a.boxes + (int64_t)kMeshBoxInts * G.halos[i], G.pmax);
+        return box_tiles(G.axis, a.boxes + (int64_t)kMeshBoxInts * G.halos[i], G.pmax, G.pairs);
     };
     const int cnt = G.ngroup, per = (cnt + 1023) / 1024;
     const int i0 = min(cnt, (int)threadIdx.x * per), i1 = min(cnt, i0 + per);
@@ -1189,7 +1223,7 @@ smooth_box_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh
                                                            : gi;
         const int h = g.halos[gi];
         const gf_mesh_desc m = mesh[h];
-        const BoxGeom q = box_geom<AXIS>(m, boxes + (int64_t)kMeshBoxInts * h);
+        const BoxGeom q = box_geom<AXIS, false>(m, boxes + (int64_t)kMeshBoxInts * h);
         const int64_t f0 = (tb - g.tile_start[gi]) * P;
         const int npen = (int)min((int64_t)P, (int64_t)q.nu * q.nv - f0);
         if (threadIdx.x < P) {
@@ -1271,29 +1305,49 @@ smooth_reg_box_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ 
                                                            : gi;
         const int h = g.halos[gi];
         const gf_mesh_desc m = mesh[h];
-        const BoxGeom q = box_geom<AXIS>(m, boxes + (int64_t)kMeshBoxInts * h);
+        const BoxGeom q = box_geom<AXIS, true>(m, boxes + (int64_t)kMeshBoxInts * h);
         const int64_t f0 = (tb - g.tile_start[gi]) * F::P;
         const int npen = (int)min((int64_t)F::P, (int64_t)q.nu * q.nv - f0);
-        const int half = (npen + 1) >> 1;  // pair c: pencils f0 + c and f0 + c + half
-        const bool two = c + half < npen;
+        const bool on = 2 * c < npen;
+        bool one = on, two = 2 * c + 1 < npen;  // the pair's pencils that are filtered
+        int u;
         auto pencil = [&](int64_t f) {
-            const int v = (int)((unsigned)f / (unsigned)q.nu), u = (int)f - v * q.nu;  // nu nv < 2^31
+            const int v = (int)((unsigned)f / (unsigned)q.nu);  // nu nv < 2^31
+            u = (int)f - v * q.nu;
             return den + m.off + (int64_t)((q.u0 + u) * q.ustride + (q.v0 + v) * q.vstride);
         };
-        float *p0 = pencil(f0 + (c < half ? c : 0));
-        float *p1 = pencil(f0 + (two ? c + half : 0));
+        float *p0 = pencil(f0 + (on ? 2 * c : 0));
+        float *p1 = nullptr;
+        if (AXIS == 0) {
+            p1 = pencil(f0 + (two ? 2 * c + 1 : 0));
+        } else {  // a pair of cells, 8-byte aligned (the meshes start on 256 bytes, their rows are even)
+            one = one && q.u0 + u >= q.a0;
+            two = two && q.u0 + u + 1 <= q.a1;
+        }
         const AxisTable at = axes[3 * h + AXIS];
         const float2 *tw = reinterpret_cast<const float2 *>(tables + at.tab_off);
         reg_fft_pair<AXIS, LOGN>(
-            smem, c, n0, c < half, tw, tables + at.tab_off + 2 * F::N,
+            smem, c, n0, on, tw, tables + at.tab_off + 2 * F::N,
             [&](int s) {
                 const bool in = s >= q.l0 && s <= q.l1;
-                return make_float2(in ? p0[s * q.sstride] : 0.f, in && two ? p1[s * q.sstride] : 0.f);
+                if (AXIS == 0) return make_float2(in ? p0[s] : 0.f, in && two ? p1[s] : 0.f);
+                const float2 v = in ? *reinterpret_cast<const float2 *>(p0 + s * q.sstride) : make_float2(0.f, 0.f);
+                return make_float2(one ? v.x : 0.f, two ? v.y : 0.f);
             },
             [&](int s, float2 v) {
                 if (s < q.s0 || s > q.s1) return;
-                p0[s * q.sstride] = v.x;
-                if (two) p1[s * q.sstride] = v.y;
+                if (AXIS == 0) {
+                    p0[s] = v.x;
+                    if (two) p1[s] = v.y;
+                    return;
+                }
+                float *e = p0 + s * q.sstride;
+                if (one && two) {
+                    *reinterpret_cast<float2 *>(e) = v;
+                } else {
+                    if (one) e[0] = v.x;
+                    if (two) e[1] = v.y;
+                }
             });
         tile_sync<AXIS>();  // the tile is reused by the next one
     }
@@ -1717,6 +1771,7 @@ int smooth_box_prepare(gf_ctx *ctx, const SmoothPlan &plan, char *dbuf, const gf
         a.g[i].ngroup = sg.ngroup;
         a.g[i].axis = sg.axis;
         a.g[i].pmax = sg.pmax;
+        a.g[i].pairs = sg.n <= 256;  // smooth_reg_box_kernel's axes
     }
     a.boxes = boxes;
     a.mesh = mesh_dev;
