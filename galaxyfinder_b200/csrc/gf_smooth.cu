@@ -907,8 +907,9 @@ smooth_reg_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh
     const int c = AXIS == 0 ? threadIdx.x / F::T : threadIdx.x % F::PAIRS;
     const int n0 = AXIS == 0 ? threadIdx.x % F::T : threadIdx.x / F::PAIRS;
     const bool on = 2 * c < t.npen, two = 2 * c + 1 < t.npen;
-    // element (pencil p, position s) lives at base + p*pstride + s*sstride;
-    // within one tile the offsets fit in 32 bits (axes <= 512, mx*ny < 2^21)
+    // element (pencil p, position s) lives at base + p*pstride + s*sstride; the
+    // strides fit in 32 bits (the other axes have at most 12,800 cells, what a
+    // pencil tile in shared memory holds), s*sstride does not
     int64_t base;
     int pstride, sstride;
     if (AXIS == 0) { base = m.off + mx * t.base; pstride = (int)mx; sstride = 1; }
@@ -922,12 +923,12 @@ smooth_reg_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh
     reg_fft_pair<AXIS, LOGN>(
         smem, c, n0, on, tw, tables + at.tab_off + 2 * F::N,
         [&](int s) {
-            const float *e = p0 + s * sstride;
+            const float *e = p0 + (int64_t)s * sstride;
             if (wide) return *reinterpret_cast<const float2 *>(e);
             return make_float2(e[0], two ? e[pstride] : 0.f);
         },
         [&](int s, float2 v) {
-            float *e = p0 + s * sstride;
+            float *e = p0 + (int64_t)s * sstride;
             if (wide) {
                 *reinterpret_cast<float2 *>(e) = v;
             } else {
@@ -960,8 +961,9 @@ smooth_fft_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh
     float2 *b0 = smem;
     float2 *b1 = smem + (P / 2) * L::SN;
     float *fa = reinterpret_cast<float *>(b0);
-    // element (pencil p, position s) lives at base + p*pstride + s*sstride;
-    // within one tile the offsets fit in 32 bits (axes <= 512, mx*ny < 2^21)
+    // element (pencil p, position s) lives at base + p*pstride + s*sstride; the
+    // strides fit in 32 bits (the other axes have at most 12,800 cells, what a
+    // pencil tile in shared memory holds), s*sstride does not
     int64_t base;
     int pstride, sstride;
     if (AXIS == 0) { base = m.off + mx * t.base; pstride = (int)mx; sstride = 1; }
@@ -996,7 +998,7 @@ smooth_fft_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh
         if (p < npen2) {
             float v[PER];
 #pragma unroll
-            for (int r = 0; r < PER; r++) v[r] = p < t.npen ? gsrc[p + (w + r * NG) * sstride] : 0.f;
+            for (int r = 0; r < PER; r++) v[r] = p < t.npen ? gsrc[p + (int64_t)(w + r * NG) * sstride] : 0.f;
 #pragma unroll
             for (int r = 0; r < PER; r++) fa[2 * L::at(p >> 1, w + r * NG) + (p & 1)] = v[r];
         }
@@ -1018,7 +1020,7 @@ smooth_fft_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh
         const int p = threadIdx.x % P;
         if (p < t.npen) {
             for (int s = threadIdx.x / P; s < N; s += NG)
-                gdst[p + s * sstride] = fs[2 * L::at(p >> 1, s) + (p & 1)];
+                gdst[p + (int64_t)s * sstride] = fs[2 * L::at(p >> 1, s) + (p & 1)];
         }
     }
 }
