@@ -67,7 +67,7 @@ struct Build {
     int32_t *par;                   // id of the parent, -1 for roots
     int32_t *small;                 // nodes left to small_subtrees (their level stands in first until then)
     int32_t *counter;               // [0] nodes allocated, [1] overflow flags, [2] blocks done, [3] small nodes,
-                                    // [4] depth of the trees (small_subtrees)
+                                    // [4] depth of the trees, in levels
     int32_t *lev;                   // level L holds the nodes [lev[L], lev[L+1]) (while the levels run)
     int32_t *nact;                  // nodes of level L that the level passes process
 };
@@ -397,6 +397,7 @@ __device__ __forceinline__ int take_nodes(const Build &b, int nch, int32_t ncap)
 // the build (counter[1]).
 __global__ void split_nodes(int L, int32_t ncap, int last, Build b) {
     if (b.nact[L] == 0) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicMax(b.counter + 4, L + 1);
     FOR_LEVEL_NODES(node, L, b) {
     if (b.count[node] <= kSmall) continue;
     {
