@@ -169,6 +169,7 @@ struct gf_ctx {
     // the stage's side streams (stream's priority) and their fork and join events
     cudaStream_t side[2] = {nullptr, nullptr};
     int side_priority = 0;
+    int lanes_priority = 1;  // of the stream of the last stage that could use them (1: none yet)
     cudaEvent_t side_ev[2] = {nullptr, nullptr};
     std::mutex lock;
 };

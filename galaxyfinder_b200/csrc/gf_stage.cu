@@ -68,16 +68,35 @@ struct EventTimer {
 // Work is put on a side stream by switching ctx->stream (the caller holds
 // ctx's lock), starts after what ctx's own stream held at the fork, and is
 // joined back into it, on errors too.
+// Two streams and two events cost a context about 100 us to make (milliseconds
+// on a busy host) and as much to destroy.  A program that makes a context per
+// group never gets that back on small groups, so they are made in a context's
+// second stage, unless the first is of kLanesAtOnce particles.  us for the
+// first stage of a new context with / without them: 120 particles 700 / 630,
+// 2000 845 / 785, 16,000 1650 / 1650, 39,358 in 64 halos 2040 / 2090, 50,000
+// 2600 / 2660, 131,072 3290 / 3410; a later stage of 120 particles 200 / 230.
+constexpr int64_t kLanesAtOnce = 32768;
+
 class Lanes {
   public:
     Lanes(gf_ctx *c, bool on) : ctx_(c), own_(c->stream), on_(on) {}
     ~Lanes() {
         for (int i = 0; i < 2; i++) join(i);
     }
-    int open() {
+    // Off unless ctx has streams of its own stream's priority or makes them
+    // here: after an earlier stage at this priority (a context that is switched
+    // between streams of two priorities would remake them for each call), or
+    // its first ones if `at_once`.
+    int open(bool at_once) {
         if (!on_) return GF_OK;
         int prio = 0;
         GF_CUDA_TRY(cudaStreamGetPriority(own_, &prio));
+        const bool again = ctx_->lanes_priority == prio, have = ctx_->side[0] || ctx_->side[1];
+        ctx_->lanes_priority = prio;
+        if (!(have && ctx_->side_priority == prio) && !again && (have || !at_once)) {
+            on_ = false;
+            return GF_OK;
+        }
         for (int i = 0; i < 2; i++) {
             if (ctx_->side[i] && ctx_->side_priority != prio) {
                 GF_CUDA_TRY(cudaStreamDestroy(ctx_->side[i]));
@@ -297,7 +316,7 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
     tm.mark();  // 1
     // phases that are timed run one after the other
     Lanes lanes(ctx, need_tree && do_mesh && !st);
-    GF_TRY(lanes.open());
+    GF_TRY(lanes.open(n >= kLanesAtOnce));
     auto mesh_prepare = [&]() -> int {
         if (box_mode) {
             GF_TRY(launch_mesh_boxes(ctx, n, xr, yr, zr, b->type, hid, nh, mesh_dev, boxes));
@@ -595,7 +614,7 @@ int stage_pass_graph(StageGraph &g) {
     // boxes zeroed; the tile counts are recounted on the device each replay
     const bool box_mode = cfg->do_mesh && g.smooth.box_ok && volfact_folds(vf) && !g.smooth.blob.empty();
     Lanes lanes(ctx, need_tree && cfg->do_mesh);
-    GF_TRY(lanes.open());
+    GF_TRY(lanes.open(true));
     if (cfg->do_mesh) {
         GF_TRY(lanes.fork(0));
         lanes.use(0);
