@@ -282,9 +282,14 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
     OnChipMeshes oc;
     SmoothPlan sp;
     char *dbuf = nullptr;
-    if (do_mesh) {
+    float *den = nullptr;
+    int32_t *boxes = nullptr;
+    bool box_mode = false;
+    auto mesh_plan = [&]() -> int {
         GF_TRY(ctx->tmp[3].reserve(sizeof(float) * (size_t)std::max<int64_t>(dev_cells, 1)));
         GF_TRY(ctx->mesh_boxes.reserve(sizeof(int32_t) * kMeshBoxInts * (size_t)std::max(nh, 1)));
+        den = ctx->tmp[3].as<float>();
+        boxes = ctx->mesh_boxes.as<int32_t>();
         if (!onchip_halos.empty()) {
             if (!o->dens_mesh || !volfact_folds(vf)) {
                 set_status(GF_EINVAL, "on-chip meshes need dens_mesh and a power-of-two volfact");
@@ -303,18 +308,18 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
             oc.densph = o->dens_mesh;
         }
         GF_TRY(smooth_plan(nh, mesh.data(), onchip_halos.empty() ? nullptr : &oc, &sp));
-        GF_TRY(smooth_upload(ctx, sp, &dbuf));
-    }
-    float *den = ctx->tmp[3].as<float>();
-    int32_t *boxes = ctx->mesh_boxes.as<int32_t>();
-    // only findDen reads the stage's meshes: with FFT axes and a folding
-    // volfact the passes run over the occupied boxes, and only the deposit
-    // boxes are zeroed (the rest of den is never read)
-    const bool box_mode = do_mesh && sp.box_ok && volfact_folds(vf) && !sp.blob.empty();
+        // only findDen reads the stage's meshes: with FFT axes and a folding
+        // volfact the passes run over the occupied boxes, and only the deposit
+        // boxes are zeroed (the rest of den is never read)
+        box_mode = sp.box_ok && volfact_folds(vf) && !sp.blob.empty();
+        if (st && !box_mode) return GF_OK;  // timed: uploaded as part of the smoothing
+        return smooth_upload(ctx, sp, &dbuf);
+    };
+    // phases that are timed run one after the other, this one before the deposit
+    if (do_mesh && !st) GF_TRY(mesh_plan());
     const bool need_tree = cfg->knn_k > 0 || cfg->do_potential;
     GF_TRY(recentre(ctx, b, hid, frame_dev, cfg->box, xr, yr, zr, pos));
     tm.mark();  // 1
-    // phases that are timed run one after the other
     Lanes lanes(ctx, need_tree && do_mesh && !st);
     GF_TRY(lanes.open(n >= kLanesAtOnce));
     auto mesh_prepare = [&]() -> int {
@@ -409,6 +414,7 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
             MeshBoxes mb;
             mb.dev = boxes;
             mb.trim_last = true;  // den is read only by find_den below
+            if (!dbuf) GF_TRY(smooth_upload(ctx, sp, &dbuf));
             GF_TRY(smooth_launch(ctx, sp, dbuf, mesh_dev, den, &oc, &mb));
         }
         tm.mark();  // 5
@@ -437,7 +443,10 @@ int stage_run_locked(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg,
         GF_TRY(knn());
         tm.mark();  // 3
         if (do_mesh) {
-            if (st) GF_TRY(mesh_prepare());
+            if (st) {
+                GF_TRY(mesh_plan());
+                GF_TRY(mesh_prepare());
+            }
             GF_TRY(mesh_rest());
         } else {
             tm.mark();
