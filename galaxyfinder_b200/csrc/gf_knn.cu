@@ -1879,13 +1879,15 @@ int launch_knn(gf_ctx *ctx, const TreeView &t, const int64_t *pstart, const floa
         // 1,000,003 2300 / 2660 / 3440.  Beside other kernels, which fill idle
         // warps, the added work counts earlier: a stage with 1 / 2 lanes takes
         // 36,000 particles 640 / 617, 70,000 752 / 769, 131,072 956 / 1025.
+        // A counted search gives a query one lane at every size: its counters
+        // are those of 32 queries per warp.
         const int64_t warps = wave * (block / 32);
-        if (t.n <= 8 * warps) {
+        if (!counters && t.n <= 8 * warps) {
             lanes = 4;
-            kern = counters ? knn_net_kernel<4, true> : knn_net_kernel<4, false>;
-        } else if ((beside ? 4 : 2) * t.n <= 5 * 16 * warps) {
+            kern = knn_net_kernel<4, false>;
+        } else if (!counters && (beside ? 4 : 2) * t.n <= 5 * 16 * warps) {
             lanes = 2;
-            kern = counters ? knn_net_kernel<2, true> : knn_net_kernel<2, false>;
+            kern = knn_net_kernel<2, false>;
         }
         if (lanes > 1) GF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem));
 #endif

@@ -495,8 +495,11 @@ typedef struct gf_stage_stats {
     int32_t nhalo, reserved;
     uint64_t pp_interactions, pc_interactions;
     float ms_recentre, ms_tree, ms_knn, ms_tsc, ms_smooth, ms_findden, ms_potential, ms_pad;
-    /* kNN work: nodes tested, 32-wide leaf batches, candidates passing the
-     * float filter, candidates inserted one by one, bitonic batch merges */
+    /* kNN work of a counted run, whose warps search for 32 queries each: nodes
+     * tested and particles tested per warp, keys appended per query, warp-wide
+     * append steps, queries left to the exact search.  (GF_KNN_ALGO 0: nodes
+     * tested, 32-wide leaf batches, candidates passing the float filter,
+     * candidates inserted one by one, bitonic batch merges.) */
     uint64_t knn_nodes, knn_batches, knn_candidates, knn_single_inserts, knn_bitonic_merges;
     /* meshes: floats laid out in device memory (mesh_cells counts every
      * planned mesh), and the meshes and particles of the on-chip path */
