@@ -14,10 +14,10 @@
 #define GF_KNN_CHUNK 32
 #endif
 #ifndef GF_KNN_ALGO    // 1: bucket kNN (a warp walks once for 32 tree-order queries,
-#define GF_KNN_ALGO 1  //    lane = query); 2: the same with float heap keys and an
+#define GF_KNN_ALGO 3  //    lane = query); 2: the same with float heap keys and an
 #endif                 //    exact certification; 3: sorting networks instead of
                        //    heaps; 0: one warp per query
-#ifndef GF_KNNB_BLOCK  // threads per block of knn_bucket_kernel (14.5 KB shared memory per warp)
+#ifndef GF_KNNB_BLOCK  // threads per block of the bucket searches (knn_bucket_kernel: 14.5 KB shared memory per warp)
 #define GF_KNNB_BLOCK 32
 #endif
 #ifndef GF_KNNB_MINB

@@ -5,18 +5,22 @@
 For each group of parameters it builds variants of the one translation unit
 that uses them (the other objects are reused), times the stage phase that the
 group drives on a seeded catalogue (gf_stage_run's own per-phase CUDA-event
-times, best of --steps after warm-up), and keeps the fastest; groups are
+times, best of --steps after warm-up), and keeps the fastest, the parameters
+that it began with unless another set is over 1 % faster; groups are
 tuned one after another, each with the best values of the ones before.  The
 result goes to galaxyfinder_b200/tuned.json (parameters, every measurement,
 the GPU and the workload), which build.py turns into -D flags.
 
   group   parameters                                   phase
-  knn     GF_KNN_ALGO x GF_KNNB_BLOCK (x GF_KNNB_ARITY), then GF_KNNB_SEEDS,
+  knn     GF_KNN_ALGO x GF_KNNB_BLOCK (x GF_KNNB_ARITY); for the sorting
+          networks then GF_KNNB_DYN and GF_KNNB_MINB (resident blocks); for
+          the float-key heaps GF_KNNB_SEEDS,
           GF_KNNB_LANECERT, GF_KNNB_DYN, GF_KNNB_WIN x GF_KNNB_MINB
           (node window against resident blocks), GF_KNNB_QUEUE and
-          GF_KNNB_FILT x GF_KNNB_HEAPF (tile filter, heap order) for the
-          float-key kernel; for the warp-per-query
-          kernel GF_KNN_CHUNK, then GF_KNN_BLOCK x register cap   knn
+          GF_KNNB_FILT x GF_KNNB_HEAPF (tile filter, heap order); for the
+          warp-per-query kernel GF_KNN_CHUNK, then GF_KNN_BLOCK x register
+          cap; from an algorithm other than the networks, only the others
+          are tried                                    knn
   bh      GF_BH_DYN, GF_BH_BLOCK, then the register cap   potential
   fft     GF_FFT_PENCILS                               smooth
   tsc     GF_TSC_TILE (0: direct global atomics)       tsc
@@ -40,9 +44,10 @@ from pathlib import Path
 from . import build as B
 
 TUNE_DIR = B.PKG / "_tune"
-DEFAULTS = {"GF_KNN_ALGO": 2, "GF_KNNB_BLOCK": 64, "GF_KNNB_ARITY": 2, "GF_KNNB_SEEDS": 64, "GF_KNNB_QUEUE": 0, "GF_KNNB_LANECERT": 0,
+# (GF_BH_TMA and GF_BH_LEAF4 named variants of an earlier walk; no source reads them)
+DEFAULTS = {"GF_KNN_ALGO": 3, "GF_KNNB_BLOCK": 64, "GF_KNNB_ARITY": 2, "GF_KNNB_SEEDS": 64, "GF_KNNB_QUEUE": 0, "GF_KNNB_LANECERT": 0,
             "GF_KNN_BLOCK": 256, "GF_KNN_MINB": 1, "GF_KNN_CHUNK": 32,
-            "GF_BH_BLOCK": 128, "GF_BH_DYN": 0, "GF_BH_ACC": 0, "GF_BH_TMA": 0, "GF_BH_LEAF4": 0, "GF_KNNB_FILT": 0, "GF_KNNB_HEAPF": 0, "GF_KNNB_DYN": 0, "GF_KNNB_WIN": 32, "GF_KNNB_MINB": 1,
+            "GF_BH_BLOCK": 128, "GF_BH_DYN": 0, "GF_BH_TMA": 0, "GF_BH_LEAF4": 0, "GF_KNNB_FILT": 0, "GF_KNNB_HEAPF": 0, "GF_KNNB_DYN": 0, "GF_KNNB_WIN": 32, "GF_KNNB_MINB": 1,
             "GF_BH_MINB": 1, "GF_FFT_PENCILS": 32, "GF_FFT_PENCILS_64": 32, "GF_FFT_PENCILS_128": 32, "GF_TSC_TILE": 0, "GF_TREE_BLOCK": 256}
 REGCAPS = (255, 64, 48)
 
@@ -51,17 +56,26 @@ def minb(block: int, regs: int) -> int:
     return max(1, 65536 // (block * regs)) if regs < 255 else 1
 
 
+def no_cap(base: dict) -> dict:
+    """From the networks' resident blocks, which the heaps' shared memory does not fit."""
+    return {"GF_KNNB_MINB": 1} if base["GF_KNN_ALGO"] == 3 else {}
+
+
 # group -> stages; each stage maps the current best parameters to a list of
 # overrides (an empty list skips the stage)
 def stages(group: str):
     if group == "knn":
-        return [lambda base: [{"GF_KNN_ALGO": a, "GF_KNNB_BLOCK": b, "GF_KNNB_ARITY": 2}
-                              for a in (1, 2) for b in (32, 64, 128)] +
-                [{"GF_KNN_ALGO": 1, "GF_KNNB_BLOCK": 32, "GF_KNNB_ARITY": 4}, {"GF_KNN_ALGO": 0}],
+        # sorting networks: 24 warps per SM fill its shared memory and registers
+        return [lambda base: ([{"GF_KNN_ALGO": 3, "GF_KNNB_BLOCK": b, "GF_KNNB_MINB": 768 // b} for b in (64, 128, 256)]
+                              if base["GF_KNN_ALGO"] == 3 else []) +
+                [{"GF_KNN_ALGO": a, "GF_KNNB_BLOCK": b, "GF_KNNB_ARITY": 2, **no_cap(base)}
+                 for a in (1, 2) for b in (32, 64, 128)] +
+                [{"GF_KNN_ALGO": 1, "GF_KNNB_BLOCK": 32, "GF_KNNB_ARITY": 4, **no_cap(base)}, {"GF_KNN_ALGO": 0}],
                 lambda base: [] if base["GF_KNN_ALGO"] != 2 else [{"GF_KNNB_SEEDS": n} for n in (32, 48, 64, 80, 96)],
                 lambda base: [] if base["GF_KNN_ALGO"] != 2 else [{"GF_KNNB_LANECERT": c} for c in (0, 1)],
-                lambda base: [] if base["GF_KNN_ALGO"] != 2 else [{"GF_KNNB_DYN": d} for d in (0, 1)],
-                lambda base: [] if base["GF_KNN_ALGO"] != 2 else
+                lambda base: [] if base["GF_KNN_ALGO"] not in (2, 3) else [{"GF_KNNB_DYN": d} for d in (0, 1)],
+                lambda base: [{"GF_KNNB_MINB": w * 32 // base["GF_KNNB_BLOCK"]} for w in (16, 24)]
+                if base["GF_KNN_ALGO"] == 3 else [] if base["GF_KNN_ALGO"] != 2 else
                 [{"GF_KNNB_WIN": w, "GF_KNNB_MINB": mb} for w, mb in ((32, 1), (8, 6), (0, 6), (0, 1))],
                 lambda base: [] if base["GF_KNN_ALGO"] != 2 else [{"GF_KNNB_QUEUE": q} for q in (0, 2, 4, 8)],
                 lambda base: [] if base["GF_KNN_ALGO"] != 2 else
@@ -154,6 +168,8 @@ def tune(nhalo: int, steps: int, groups=("knn", "bh", "fft", "tsc", "tree")) -> 
             if not stage:
                 continue
             cands = [dict(base, **ov) for ov in stage]
+            if base not in cands:
+                cands.append(base)
             with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as ex:
                 libs = list(ex.map(lambda p: build_variant(src, p), cands))
             keys = sorted(set().union(*(ov.keys() for ov in stage)))
@@ -164,9 +180,9 @@ def tune(nhalo: int, steps: int, groups=("knn", "bh", "fft", "tsc", "tree")) -> 
                 shown = {k: p[k] for k in keys}
                 log[g].append({"params": shown, "ms": ms})
                 print(f"{g}: {variant_name(shown)}: {phase} {ms:.3f} ms", flush=True)
-            ref_ms = next(ms for ms, p in timed if p == base) if base in [p for _, p in timed] else None
+            ref_ms = next(ms for ms, p in timed if p == base)
             ms, p = min(timed, key=lambda t: t[0])
-            if ref_ms is None or ms < 0.99 * ref_ms:  # keep the incumbent unless >1% faster
+            if ms < 0.99 * ref_ms:  # keep the incumbent unless >1% faster
                 base = p
     import torch
     if B.TUNED.exists():  # keep the measurements of the groups not re-run
