@@ -1238,7 +1238,7 @@ knn_fbucket_kernel(int64_t n, int k, const float4 *__restrict__ pos, const int32
 //     that whatever the filter or a node's box rejects lies clear of the list;
 //   * the least key ever dropped by a merge is kept, and the list is certified
 //     as above against min(that key's lower end, the bound, the distance to
-//     the outside of the processed box); a query that fails goes to knn_kernel;
+//     the outside of the processed box); a query that fails goes to knn_redo_kernel;
 //   * the certified list is ordered by its exact distances.
 // Lists shorter than 32 (k < 32, small halos) start with 32 - k keys below
 // every distance, so that the bound is always the last key.

@@ -44,7 +44,8 @@ from pathlib import Path
 from . import build as B
 
 TUNE_DIR = B.PKG / "_tune"
-# (GF_BH_TMA and GF_BH_LEAF4 named variants of an earlier walk; no source reads them)
+# variants of an earlier walk, which no source reads: not written to tuned.json
+GONE = ("GF_BH_TMA", "GF_BH_LEAF4")
 DEFAULTS = {"GF_KNN_ALGO": 3, "GF_KNNB_BLOCK": 64, "GF_KNNB_ARITY": 2, "GF_KNNB_SEEDS": 64, "GF_KNNB_QUEUE": 0, "GF_KNNB_LANECERT": 0,
             "GF_KNN_BLOCK": 256, "GF_KNN_MINB": 1, "GF_KNN_CHUNK": 32,
             "GF_BH_BLOCK": 128, "GF_BH_DYN": 0, "GF_BH_TMA": 0, "GF_BH_LEAF4": 0, "GF_KNNB_FILT": 0, "GF_KNNB_HEAPF": 0, "GF_KNNB_DYN": 0, "GF_KNNB_WIN": 32, "GF_KNNB_MINB": 1,
@@ -189,7 +190,7 @@ def tune(nhalo: int, steps: int, groups=("knn", "bh", "fft", "tsc", "tree")) -> 
         prev = json.loads(B.TUNED.read_text())
         log = {**prev.get("measured", {}), **log}
         groups = tuple(dict.fromkeys(list(prev.get("phase_of_group", {})) + list(groups)))
-    res = {"params": base, "measured": log, "phase_of_group": {g: GROUPS[g][1] for g in groups},
+    res = {"params": {k: v for k, v in base.items() if k not in GONE}, "measured": log, "phase_of_group": {g: GROUPS[g][1] for g in groups},
            "workload": f"seeded catalogue, {nhalo} halos (N_p ~ N^-1.9 on [100, 2e6]), best of {steps} steps",
            "gpu": torch.cuda.get_device_name(0), "date": datetime.date.today().isoformat()}
     B.TUNED.write_text(json.dumps(res, indent=1) + "\n")

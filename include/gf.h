@@ -512,7 +512,8 @@ typedef struct gf_stage_stats {
 /* stats may be NULL; when given, per-phase CUDA-event times are filled in and
  * the phases run one after the other.  Without, the mesh part and the potential
  * run on two streams of the context beside the octree build and the search;
- * both are joined back into ctx's stream. */
+ * both are joined back into ctx's stream.  (A context makes the two streams in
+ * its second stage, or in a first one of at least 32768 particles.) */
 int gf_stage_run(gf_ctx *ctx, const gf_batch *b, const gf_stage_config *cfg, gf_stage_out *out,
                  gf_stage_stats *stats);
 
