@@ -902,7 +902,13 @@ __global__ void emit_nodes(int32_t ncap, float theta2, Build b, const int32_t *_
     h.com[1] = b.my[node];
     h.com[2] = b.mz[node];
     // ost.c:573,80: dist2 = (double)distmax (a float); ratio = dist2/theta2
-    h.open_r2 = (double)__uint_as_float(b.r2[node]) / (double)theta2;
+    // Where that is 0 the node's particles all lie at its centre, to within
+    // offsets whose squares underflow a float: opened by a target there, which
+    // gets the particles' terms (none) instead of a cell's at distance zero.
+    // Whether such a centre rounds to the particles' very position depends on
+    // the order of its sums, so their potential was finite or not by chance.
+    const float far2 = __uint_as_float(b.r2[node]);
+    h.open_r2 = far2 > 0.f ? (double)far2 / (double)theta2 : 4e-45;  // 3 * 2^-150 < 4e-45
     h.mass = (float)b.m[node];
     float q[6];
     for (int a = 0; a < 6; a++) q[a] = b.q[6 * (int64_t)node + a];
