@@ -367,7 +367,12 @@ smooth_direct_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ m
 // The taps of the direct path: h_m = (1/n) sum_i G_i cos(2 pi (i m mod n) / n) in
 // FP64, rounded once; a block per 128 taps of a table.  On the host these
 // O(n^2) sums were most of a call on the reference's own meshes (48 meshes,
-// 144 tables: 0.8 of 1.41 ms; 5 us here).
+// 144 tables: 0.8 of 1.41 ms; 5 us here).  Up to kHostTaps terms in all they
+// stay on the host, where they take less than the launch.  us for the smoothing
+// of one mesh with the tables on the host / on the device: 64 x 1 x 1 cells 38
+// / 42, 10 x 11 x 12 39.8 / 41.6, 20^3 39.5 / 42.7, 36^3 54.2 / 54.3, 24 x 25
+// x 26 45.9 / 45.1, 30 x 31 x 33 59.5 / 52.3.
+constexpr int64_t kHostTaps = 1024;
 struct TableJob {
     int32_t n, pad;
     int64_t tab_off;  // float offset of the table
@@ -1542,6 +1547,16 @@ int smooth_plan(int32_t nhalo, const gf_mesh_desc *mesh_host, const OnChipMeshes
             }
             axes[3 * (size_t)h + a] = it->second;
         }
+    }
+    // a launch for a few short tables costs more than their sums on the host
+    int64_t terms = 0;
+    for (const TableJob &j : jobs) terms += (int64_t)j.n * j.n;
+    if (terms <= kHostTaps) {
+        for (const TableJob &j : jobs) {
+            std::vector<double> work(2 * (size_t)j.n);
+            write_axis_tables(j.n, j.rg_cells, tables.data() + j.tab_off, work.data(), work.data() + j.n);
+        }
+        jobs.clear();
     }
     // groups: (axis, n) for the FFT path; per axis, one group for the blocked
     // direct path and one for the rest
