@@ -807,12 +807,13 @@ static_assert(FftTile<9>::NT <= 1024, "FFT tile threads");
 // columns (y, z) have neighbouring pairs in neighbouring lanes, for the
 // mesh accesses and for conflict-free rows of the tile.
 // What bounds it: the latency of the mesh loads (16 to 32 in flight per thread;
-// whole 256^3 passes move 134 MB in 38 us, 54 % of the measured copy rate).
-// Stockham tiles -> register passes: the box passes of 4096 halos 4.93 -> 2.50
-// ms (64 cells 1.59 -> 0.87, 128 1.30 -> 0.62, 256 2.02 -> 1.02), nine whole
-// passes of a 256^3 mesh 661 -> 350 us.  Resident threads per SM (registers
-// against warps), 512 / 768 / 1024: box passes of 64 cells 942 / 921 / 866 us,
-// of 128 625 / 670 / 730, of 256 1022 / 1062 / 1106; whole passes 374 / 350 / 386.
+// whole 256^3 passes move 134 MB in 35 us, 58 % of the measured copy rate).
+// Stockham tiles -> register passes: the box passes of 4096 halos 4.93 -> 2.46
+// ms (64 cells 1.60 -> 0.85, 128 1.30 -> 0.62, 256 2.03 -> 1.00), nine whole
+// passes of a 256^3 mesh 651 -> 318 us (344 with 4-byte columns).  Resident
+// threads per SM (registers against warps), 512 / 768 / 1024, with 4-byte
+// columns: box passes of 64 cells 942 / 921 / 866 us, of 128 625 / 670 / 730, of
+// 256 1022 / 1062 / 1106; whole passes 374 / 350 / 386.
 template <int LOGN>
 struct RegFft {
     static constexpr int N = 1 << LOGN;
