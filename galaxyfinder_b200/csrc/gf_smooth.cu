@@ -433,45 +433,6 @@ __device__ __forceinline__ void dft(float2 (&a)[R]) {
         a[1] = csub(t, a[1]);
     } else if (R == 4) {
         dft4<INV>(a[0], a[1], a[2], a[3]);
-    } else if (R == 16) {  // 4 x 4: columns, W16 twiddles, rows
-        // cos and sin of pi/8, and of pi/4.  The float cosine is off by nearly
-        // half a unit in the last place in every product it is in, which made a
-        // 256-cell axis 4 % less exact than its radix-8 passes were (rms of a
-        // mesh's cells against 64 bits); it is held as the sum of two floats.
-        constexpr double kCos = 0.92387953251128676;
-        constexpr float c1 = (float)kCos, c1lo = (float)(kCos - (double)c1);
-        const float s1 = 0.38268343236508977f, h = 0.70710678118654752f;
-        constexpr float sg = INV ? -1.f : 1.f;
-        auto tw = [](float2 v, float c, float s) {  // v * (c - i s), conjugated for the inverse
-            return make_float2(v.x * c + sg * v.y * s, v.y * c - sg * v.x * s);
-        };
-        auto cadd1 = [=](float v, float t) { return fmaf(v, c1, fmaf(v, c1lo, t)); };  // v cos(pi/8) + t
-        auto tw1 = [=](float2 v) { return make_float2(cadd1(v.x, sg * v.y * s1), cadd1(v.y, -sg * v.x * s1)); };
-        auto tw3 = [=](float2 v) { return make_float2(cadd1(sg * v.y, v.x * s1), cadd1(-sg * v.x, v.y * s1)); };
-#pragma unroll
-        for (int i = 0; i < 4; i++) dft4<INV>(a[i], a[4 + i], a[8 + i], a[12 + i]);
-        a[5] = tw1(a[5]);            // W16^1
-        a[9] = tw(a[9], h, h);       // W16^2
-        a[13] = tw3(a[13]);          // W16^3
-        a[6] = tw(a[6], h, h);       // W16^2
-        a[10] = mul_mi<INV>(a[10]);  // W16^4
-        a[14] = tw(a[14], -h, h);    // W16^6
-        a[7] = tw3(a[7]);            // W16^3
-        a[11] = tw(a[11], -h, h);    // W16^6
-        a[15] = tw1(a[15]);          // W16^9 = -W16^1
-        a[15] = make_float2(-a[15].x, -a[15].y);
-#pragma unroll
-        for (int i = 0; i < 16; i += 4) dft4<INV>(a[i], a[i + 1], a[i + 2], a[i + 3]);
-        // entry 4 k + j holds output k + 4 j
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-#pragma unroll
-            for (int j = k + 1; j < 4; j++) {
-                const float2 t = a[4 * k + j];
-                a[4 * k + j] = a[4 * j + k];
-                a[4 * j + k] = t;
-            }
-        }
     } else {  // R == 8: two 4-point DFTs (even, odd) and the W8 butterflies
         float2 e0 = a[0], e1 = a[2], e2 = a[4], e3 = a[6];
         float2 o0 = a[1], o1 = a[3], o2 = a[5], o3 = a[7];
@@ -793,52 +754,143 @@ struct FftTile {
 };
 static_assert(FftTile<9>::NT <= 1024, "FFT tile threads");
 
-// ---- axes of 64, 128 and 256 cells: the transform of a pencil pair in two
-// register passes, N = R1 x R2 (8 x 8, 16 x 8, 16 x 16), T = R2 threads per pair.
-// A thread loads the R1 elements n0 + r T of its pair from the mesh straight
-// into registers, transforms them, applies w^(n0 j) and leaves output j at
-// place j T + n0 of the shared tile; block j (R2 consecutive places) is then a
-// transform of its own, whose outputs are the frequencies j + R1 k: one thread
-// reads it, multiplies by the filter and transforms it back in place; the
-// mirrored first pass ends in registers again and stores to the mesh.  Two
-// exchanges through shared memory and three barriers per tile, where separate
-// load, Stockham passes and store took five (64) or seven.
+// ---- axes of 64, 128 and 256 cells: the transform of a pencil pair in
+// registers, radix 8, 8 and A = N / 64, by T = 8 threads with N / 8 elements
+// each.  Thread n0 holds the elements n0 + 8 m.  The first radix-8 butterflies
+// (elements p + r N/8, p = n0 + 8 a) and their twiddles stay within a thread; one
+// exchange through shared memory then brings output j = n0 of all N/8
+// butterflies together, which the second radix 8 and the radix A need, again
+// within a thread.  Their outputs are the frequencies n0 + 8 m: the filter, and
+// the same two steps back, which end at the elements n0 + 8 m.  Two exchanges
+// and three barriers per tile, where load, Stockham passes in shared memory and
+// store took five (64) or seven.
+// Butterflies, twiddles (table values) and roundings are those of
+// stockham_pass, written with explicit roundings where a compiler may contract
+// differently: the passes give the same bits as the Stockham passes did.
 // Rows (x) keep a pair's threads in one warp, so they need no block barrier;
 // columns (y, z) have neighbouring pairs in neighbouring lanes, for the
 // mesh accesses and for conflict-free rows of the tile.
-// What bounds it: the latency of the mesh loads (16 to 32 in flight per thread;
-// whole 256^3 passes move 134 MB in 35 us, 58 % of the measured copy rate).
-// Stockham tiles -> register passes: the box passes of 4096 halos 4.93 -> 2.46
-// ms (64 cells 1.60 -> 0.85, 128 1.30 -> 0.62, 256 2.03 -> 1.00), nine whole
-// passes of a 256^3 mesh 651 -> 318 us (344 with 4-byte columns).  Resident
-// threads per SM (registers against warps), 512 / 768 / 1024, with 4-byte
-// columns: box passes of 64 cells 942 / 921 / 866 us, of 128 625 / 670 / 730, of
-// 256 1022 / 1062 / 1106; whole passes 374 / 350 / 386.
+// What bounds it: the latency of the mesh loads (8 to 32 in flight per thread;
+// whole 256^3 passes move 134 MB in 37 us, 55 % of the measured copy rate).
+// Stockham tiles -> register passes: the box passes of 4096 halos 4.93 -> 2.52
+// ms (64 cells 1.60 -> 0.87, 128 1.30 -> 0.59, 256 2.03 -> 1.07), the three
+// passes of a whole 64^3 mesh 14.8 -> 10.2 us, 128^3 37.9 -> 21.6, 256^3 217 ->
+// 111.  In two passes of 8 x 8, 16 x 8 and 16 x 16, whose roundings differ from
+// the Stockham passes', the same took 0.85, 0.61 and 1.00 ms; 10.2, 22.9 and
+// 106 us.  Resident threads per SM (registers against warps), 384 / 512 / 640 /
+// 768: box passes of 64 cells 959 / 956 / 902 / 880 (1024: 868) us, of 128 657 /
+// 592 / 585 / 636, of 256 1068 / 1156 / 1347 / 1752; whole 256^3 118 / 111 / 112 /
+// 136 us.
 template <int LOGN>
 struct RegFft {
     static constexpr int N = 1 << LOGN;
-    static constexpr int R1 = LOGN == 6 ? 8 : 16;
-    static constexpr int R2 = N / R1;
-    static constexpr int T = R2;       // threads per pair
-    static constexpr int B = R1 / T;   // blocks per thread in the second pass
+    static constexpr int T = 8;        // threads per pair
+    static constexpr int M = N / 8;    // elements per thread, radix-8 butterflies per pass
+    static constexpr int A = N / 64;   // last radix
     static constexpr int P = LOGN == 6 ? GF_FFT_PENCILS_64 : LOGN == 7 ? GF_FFT_PENCILS_128 : 32;  // real pencils per tile
     static constexpr int PAIRS = P / 2;
     static constexpr int NT = PAIRS * T;
-    // float2 stride of a pair of rows: a padding slot per block, and pairs of
-    // one half-warp in different banks
-    static constexpr int SN = N + R1 + (LOGN == 7 ? 8 : 0);
+    // resident threads per SM of the whole-mesh and the box passes
+    static constexpr int WHOLE = LOGN == 6 ? 768 : LOGN == 7 ? 640 : 512;
+    static constexpr int BOX = LOGN == 6 ? 1024 : LOGN == 7 ? 640 : 384;
+    // float2 stride of a pair of rows: a padding slot per output j, and the
+    // pairs of a half-warp in different banks (8 (M + 1) = 8 mod 16)
+    static constexpr int SN = 8 * (M + 1);
     static_assert(LOGN >= 6 && LOGN <= 8 && NT <= 1024, "register FFT lengths 64..256");
     template <int AXIS>
     static constexpr size_t smem() { return (size_t)(AXIS == 0 ? PAIRS * SN : N * PAIRS) * sizeof(float2); }
+    // output j of butterfly p of pair c.  (The inverse keeps output j of thread
+    // n0's butterfly a at place (8 a + j, n0): those that this thread has read
+    // last, so that no barrier is needed before.)
     template <int AXIS>
-    __device__ static __forceinline__ int at(int c, int pos) {
-        return AXIS == 0 ? c * SN + pos + pos / R2 : pos * PAIRS + c;
+    __device__ static __forceinline__ int at(int c, int p, int j) {
+        return AXIS == 0 ? c * SN + j * (M + 1) + p : (p * 8 + j) * PAIRS + c;
     }
 };
+
+// a * w (w conjugated for the inverse): which of two products is rounded before
+// the sum is stockham_pass's choice
+template <bool INV>
+__device__ __forceinline__ float2 twiddle_rn(float2 a, float2 w) {
+    if (INV) return make_float2(__fmaf_rn(a.x, w.x, __fmul_rn(a.y, w.y)), __fmaf_rn(a.y, w.x, -__fmul_rn(a.x, w.y)));
+    return make_float2(__fmaf_rn(a.x, w.x, -__fmul_rn(a.y, w.y)), __fmaf_rn(a.x, w.y, __fmul_rn(a.y, w.x)));
+}
+// e +- sqrt(1/2) t, one rounding
+__device__ __forceinline__ void add_half(float2 e, float2 t, float2 &sum, float2 &diff) {
+    constexpr float h = 0.70710678118654752f;
+    sum = make_float2(__fmaf_rn(h, t.x, e.x), __fmaf_rn(h, t.y, e.y));
+    diff = make_float2(__fmaf_rn(-h, t.x, e.x), __fmaf_rn(-h, t.y, e.y));
+}
+// dft<8> with its roundings spelled out
+template <bool INV>
+__device__ __forceinline__ void dft8_rn(float2 (&a)[8]) {
+    float2 e0 = a[0], e1 = a[2], e2 = a[4], e3 = a[6];
+    float2 o0 = a[1], o1 = a[3], o2 = a[5], o3 = a[7];
+    dft4<INV>(e0, e1, e2, e3);
+    dft4<INV>(o0, o1, o2, o3);
+    a[0] = cadd(e0, o0);
+    a[4] = csub(e0, o0);
+    add_half(e1, INV ? make_float2(o1.x - o1.y, o1.x + o1.y) : make_float2(o1.x + o1.y, o1.y - o1.x), a[1], a[5]);
+    o2 = mul_mi<INV>(o2);
+    a[2] = cadd(e2, o2);
+    a[6] = csub(e2, o2);
+    const float s3 = o3.x + o3.y;
+    add_half(e3, INV ? make_float2(-s3, o3.x - o3.y) : make_float2(o3.y - o3.x, -s3), a[3], a[7]);
+}
 
 template <int AXIS>
 __device__ __forceinline__ void tile_sync() {
     if (AXIS == 0) __syncwarp(); else __syncthreads();
+}
+
+// v[m] holds the elements (frequencies) n0 + 8 m of pair c before and after.
+template <int AXIS, int LOGN, bool INV>
+__device__ __forceinline__ void reg_fft(float2 *sm, int c, int n0, bool on, const float2 *__restrict__ tw,
+                                        float2 (&v)[RegFft<LOGN>::M]) {
+    using F = RegFft<LOGN>;
+    auto twiddle = [&](float2 x, int k) { return twiddle_rn<INV>(x, __ldg(tw + k)); };
+    if (on) {
+#pragma unroll
+        for (int a = 0; a < F::A; a++) {
+            const int p = n0 + 8 * a;
+            float2 b[8];
+#pragma unroll
+            for (int r = 0; r < 8; r++) b[r] = v[a + F::A * r];
+            dft8_rn<INV>(b);
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                sm[INV ? F::template at<AXIS>(c, 8 * a + j, n0) : F::template at<AXIS>(c, p, j)] =
+                    j ? twiddle(b[j], p * j) : b[j];
+        }
+    }
+    tile_sync<AXIS>();
+    if (on) {
+#pragma unroll
+        for (int p = 0; p < F::M; p++)  // output n0 of butterfly p
+            v[p] = sm[INV ? F::template at<AXIS>(c, (p & ~7) + n0, p & 7) : F::template at<AXIS>(c, p, n0)];
+#pragma unroll
+        for (int a = 0; a < F::A; a++) {
+            float2 b[8];
+#pragma unroll
+            for (int r = 0; r < 8; r++) b[r] = v[a + F::A * r];
+            dft8_rn<INV>(b);
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[a + F::A * j] = a && j ? twiddle(b[j], 8 * a * j) : b[j];
+        }
+        // radix A over a: output j + 8 k
+        float2 y[F::M];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            float2 b[F::A];
+#pragma unroll
+            for (int a = 0; a < F::A; a++) b[a] = v[a + F::A * j];
+            if constexpr (F::A > 1) dft<F::A, INV>(b);
+#pragma unroll
+            for (int k = 0; k < F::A; k++) y[j + 8 * k] = b[k];
+        }
+#pragma unroll
+        for (int m = 0; m < F::M; m++) v[m] = y[m];
+    }
 }
 
 // Pair c of a tile (on: it holds a pencil), thread n0 of T: load(s) gives both
@@ -846,59 +898,33 @@ __device__ __forceinline__ void tile_sync() {
 // neighbouring pencils, 2c and 2c + 1: either half of a complex pencil carries
 // the rounding errors of the brighter one, and a neighbour is about as bright.
 // (Pencils half a tile apart: the cells beside a dense core took its noise 16
-// cells further; their median error was 2 to 17 times as large.)
+// cells further; their median error was 4 to 6 times as large.)
 template <int AXIS, int LOGN, class Load, class Store>
 __device__ __forceinline__ void reg_fft_pair(float2 *sm, int c, int n0, bool on, const float2 *__restrict__ tw,
                                              const float *__restrict__ filt, Load load, Store store) {
     using F = RegFft<LOGN>;
-    float2 a[F::R1];
+    float2 v[F::M];
     if (on) {
 #pragma unroll
-        for (int r = 0; r < F::R1; r++) a[r] = load(n0 + r * F::T);
-        dft<F::R1, false>(a);
-#pragma unroll
-        for (int j = 1; j < F::R1; j++) a[j] = cmul(a[j], __ldg(tw + n0 * j));
-#pragma unroll
-        for (int j = 0; j < F::R1; j++) sm[F::template at<AXIS>(c, j * F::T + n0)] = a[j];
+        for (int m = 0; m < F::M; m++) v[m] = load(n0 + 8 * m);
     }
-    tile_sync<AXIS>();
+    reg_fft<AXIS, LOGN, false>(sm, c, n0, on, tw, v);
     if (on) {
 #pragma unroll
-        for (int b = 0; b < F::B; b++) {
-            const int u = n0 + b * F::T;
-            float2 d[F::R2];
-#pragma unroll
-            for (int i = 0; i < F::R2; i++) d[i] = sm[F::template at<AXIS>(c, u * F::R2 + i)];
-            dft<F::R2, false>(d);
-#pragma unroll
-            for (int i = 0; i < F::R2; i++) {
-                const float g = __ldg(filt + u + F::R1 * i);
-                d[i].x *= g;
-                d[i].y *= g;
-            }
-            dft<F::R2, true>(d);
-#pragma unroll
-            for (int i = 0; i < F::R2; i++) sm[F::template at<AXIS>(c, u * F::R2 + i)] = d[i];
+        for (int m = 0; m < F::M; m++) {
+            const float g = __ldg(filt + n0 + 8 * m);
+            v[m] = make_float2(__fmul_rn(v[m].x, g), __fmul_rn(v[m].y, g));
         }
     }
-    tile_sync<AXIS>();
+    reg_fft<AXIS, LOGN, true>(sm, c, n0, on, tw, v);
     if (on) {
 #pragma unroll
-        for (int j = 0; j < F::R1; j++) a[j] = sm[F::template at<AXIS>(c, j * F::T + n0)];
-#pragma unroll
-        for (int j = 1; j < F::R1; j++) {
-            float2 w = __ldg(tw + n0 * j);
-            w.y = -w.y;
-            a[j] = cmul(a[j], w);
-        }
-        dft<F::R1, true>(a);
-#pragma unroll
-        for (int r = 0; r < F::R1; r++) store(n0 + r * F::T, a[r]);
+        for (int m = 0; m < F::M; m++) store(n0 + 8 * m, v[m]);
     }
 }
 
 template <int AXIS, int LOGN>
-__global__ void __launch_bounds__(RegFft<LOGN>::NT, 768 / RegFft<LOGN>::NT)
+__global__ void __launch_bounds__(RegFft<LOGN>::NT, RegFft<LOGN>::WHOLE / RegFft<LOGN>::NT)
 smooth_reg_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh, GroupLaunch g,
                   const AxisTable *__restrict__ axes, const float *__restrict__ tables,
                   const int32_t *__restrict__ boxes, int trim) {
@@ -1297,7 +1323,7 @@ smooth_box_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh
 
 // The same passes of the axes that the register transform serves.
 template <int AXIS, int LOGN>
-__global__ void __launch_bounds__(RegFft<LOGN>::NT, (LOGN == 6 ? 1024 : 512) / RegFft<LOGN>::NT)
+__global__ void __launch_bounds__(RegFft<LOGN>::NT, RegFft<LOGN>::BOX / RegFft<LOGN>::NT)
 smooth_reg_box_kernel(float *__restrict__ den, const gf_mesh_desc *__restrict__ mesh, GroupLaunch g,
                       const AxisTable *__restrict__ axes, const float *__restrict__ tables,
                       const int32_t *__restrict__ boxes) {
