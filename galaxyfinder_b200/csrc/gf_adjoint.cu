@@ -18,7 +18,6 @@
 #include <vector>
 
 #include "gf_tree.cuh"
-#include "gf_tsc_weights.cuh"
 
 namespace gf {
 
@@ -101,7 +100,6 @@ __global__ void find_den_adjoint_kernel(int64_t n, const double *__restrict__ x,
             continue;
         }
         const int64_t mx = 2 * (m.nx / 2 + 1);
-        const bool wide = gS && mesh_wide(gS + m.off);
         double sx = 0, sy = 0, sz = 0;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
@@ -111,11 +109,11 @@ __global__ void find_den_adjoint_kernel(int64_t n, const double *__restrict__ x,
                 const double wyz = ay.w[b] * az.w[c];
                 const double dyz = ay.dw[b] * az.w[c];
                 const double ydz = ay.w[b] * az.dw[c];
-                if (gS)
-                    mesh_add3(gS + row, (float)(gp * ax.w[0] * wyz), (float)(gp * ax.w[1] * wyz),
-                              (float)(gp * ax.w[2] * wyz), wide);
 #pragma unroll
                 for (int a = 0; a < 3; a++) {
+                    // one reduction per cell, as in tsc_deposit_kernel (vector
+                    // reductions: 582 -> 335 us for 2e6 particles, in another order)
+                    if (gS) atomicAdd(gS + row + a, (float)(gp * ax.w[a] * wyz));
                     if (S) {
                         const double v = __ldg(S + row + a);
                         sx += v * ax.dw[a] * wyz;

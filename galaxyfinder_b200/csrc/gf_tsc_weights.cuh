@@ -96,11 +96,10 @@ __device__ __forceinline__ float tsc_interp_add(float density, float v, const Ts
 // share an aligned 16- or 8-byte word go in one vector reduction (float4 /
 // float2 atomics add each element separately), half as many as cells on
 // average; the fourth element of a 16-byte word is a cell of the same mesh
-// (or row padding) and gets +0.  Reductions per second at the L2 bound the
-// scattered deposits; scalar -> vector, 2e6 particles in 64 clumps into a
-// 256^3 mesh: deposit 435 -> 227 us, adjoint of the interpolation 582 -> 335;
-// the stage's tiled deposit (its segments too sparse for a tile) over 6.1 M
-// particles 1061 -> 769.
+// (or row padding) and gets +0.  For the stage's tiled deposit, whose sums have
+// two levels anyhow (segments too sparse for a tile): reductions per second at
+// the L2 bound it, 6.1 M particles 1061 -> 769 us.  A whole mesh is deposited
+// with one reduction per cell (see tsc_deposit_kernel).
 __device__ __forceinline__ void mesh_add3(float *p, float v0, float v1, float v2, bool wide) {
     const unsigned at = wide ? (unsigned)((uintptr_t)p >> 2) & 3u : 4u;
     if (at == 0u) {
