@@ -45,6 +45,8 @@ def test_streams_of_the_first_stages(cuda_device, tmp_path, npart, want):
         np.testing.assert_array_equal(o["dens_sph"], outs[0]["dens_sph"])
         assert np.abs(o["dens_mesh"] - outs[0]["dens_mesh"]).max() <= 2e-6 * outs[0]["dens_mesh"].max()
         np.testing.assert_allclose(o["phi"], outs[0]["phi"], rtol=1e-6)
+        # phi * potentfact + the background term, rounded once; of opposite signs
+        assert np.abs(o["penergy"] - outs[0]["penergy"]).max() <= 2e-6 * np.abs(outs[0]["penergy"]).max()
 
 
 def test_streams_of_two_priorities(cuda_device, tmp_path):
